@@ -2280,7 +2280,11 @@ void importance_probabilities(int device, uha_metric metric, const float* host_r
     DeviceBuffer<float> copied(host_rows != nullptr ? row_count * dimension : 0);
     DeviceBuffer<double> inverse(row_count * row_count);
     DeviceBuffer<double> gram_matrix(gram ? row_count * row_count : 0);
-    DeviceBuffer<unsigned long long> maxima(dimension);
+    // the columns' maxima (8 bytes each), then the filter's largest products
+    // (4 bytes each) and its out-of-range flag
+    DeviceBuffer<unsigned long long> maxima(dimension + (dimension + 1) / 2 + 1);
+    unsigned int* top_bits = reinterpret_cast<unsigned int*>(maxima.get() + dimension);
+    int* odd = reinterpret_cast<int*>(maxima.get() + dimension + (dimension + 1) / 2);
     DeviceBuffer<int> flag(1);
     const float* rows = host_rows != nullptr ? copied.get() : device_rows;
     check_cuda(cudaEventRecord(ev[0], stream), "event");
@@ -2306,20 +2310,17 @@ void importance_probabilities(int device, uha_metric metric, const float* host_r
     const int m = metric == UHA_L2 ? 0 : 1;
     if (gram) {
         uha::launch_gram_inverse_distances(rows, row_count, dimension, gram_matrix.get(),
-                                           inverse.get(), stream);
+                                           inverse.get(), odd, stream);
     } else {
-        uha::launch_pair_distances(m, rows, row_count, dimension, inverse.get(), stream);
+        uha::launch_pair_distances(m, rows, row_count, dimension, inverse.get(), odd, stream);
     }
     check_cuda(cudaEventRecord(ev[2], stream), "event");
-    for (uint64_t c = 0; c < rep.pair_chunks; ++c) {
-        const uint64_t begin = rep.pair_count * c / rep.pair_chunks;
-        const uint64_t end = rep.pair_count * (c + 1) / rep.pair_chunks;
-        uha::launch_coordinate_maxima(m, rows, row_count, dimension, inverse.get(),
-                                      maxima.get(), begin, end, stream, single);
-    }
+    uha::launch_coordinate_maxima(m, rows, row_count, dimension, inverse.get(), top_bits, odd,
+                                  maxima.get(), rep.pair_chunks, stream, single);
     check_cuda(cudaEventRecord(ev[3], stream), "event");
     std::vector<unsigned long long> bits(dimension);
-    check_cuda(cudaMemcpyAsync(bits.data(), maxima.get(), maxima.bytes(),
+    check_cuda(cudaMemcpyAsync(bits.data(), maxima.get(),
+                               dimension * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, stream),
                "cannot copy probabilities from the CUDA device");
     check_cuda(cudaEventRecord(ev[4], stream), "event");

@@ -423,23 +423,25 @@ void launch_row_norms(const float* rows, uint64_t row_count,
                       uint64_t padded_dim, float* norms, cudaStream_t stream);
 
 // ---- importance probabilities (binary64 pair distances and normalisation)
+// inverse_distances: r x r, receives 1 / distance of every pair a < b (0 for
+// zero distance) and, in the mirror slots, the column filter's weights; *odd
+// (0 before) becomes nonzero when a weight is out of the filter's range.
 void launch_pair_distances(int metric, const float* rows, uint64_t row_count,
-                           uint64_t dim, double* inverse_distances,
+                           uint64_t dim, double* inverse_distances, int* odd,
                            cudaStream_t stream);
 // L2 pair distances through the binary64 Gram identity with direct
 // recomputation of cancellation-prone pairs; `gram` holds r x r doubles.
 void launch_gram_inverse_distances(const float* rows, uint64_t row_count,
                                    uint64_t dim, double* gram,
-                                   double* inverse_distances,
+                                   double* inverse_distances, int* odd,
                                    cudaStream_t stream);
-// Folds the pairs [pair_begin, pair_end) of the row-major order of pairs
-// a < b into the per-column maxima (one launch per chunk of pairs); `single`:
-// the contributions in binary32 (within 3e-7 relative).
-void launch_coordinate_maxima(int metric, const float* rows,
-                              uint64_t row_count, uint64_t dim,
-                              const double* inverse_distances,
-                              unsigned long long* maxima_bits,
-                              uint64_t pair_begin, uint64_t pair_end,
+// The per-column maxima over all pairs, in at most pair_chunks launches per
+// run; top_bits: dim words, maxima_bits: dim words, both zero before.
+// `single`: the contributions in binary32 (within 3e-7 relative).
+void launch_coordinate_maxima(int metric, const float* rows, uint64_t row_count,
+                              uint64_t dim, const double* inverse_distances,
+                              unsigned int* top_bits, const int* odd,
+                              unsigned long long* maxima_bits, uint64_t pair_chunks,
                               cudaStream_t stream, bool single = false);
 // flag |= 1 when any of the `count` values is not finite
 void launch_finite_check(const float* values, uint64_t count, int* flag,
