@@ -200,6 +200,63 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
         rep.kernel = 2;
         rep.tile_queries = static_cast<uint32_t>(best.lowp_plan.bn);
         rep.splits = best.lowp_plan.splits;
+    } else if (const uha::SplitRows* sp = !ws->split_disabled && split_shape(index, strategy, batch)
+                                              ? split_rows(index, stream)
+                                              : nullptr;
+               sp != nullptr) {
+        // the certified split scan: its tile widths and column splits
+        std::vector<uha::SplitPlan> cands =
+            uha::split_candidates(index->rows, sp->pitch, batch, index->sm_count);
+        if (uha::split_filter_applies(cands[0], index->rows)) {
+            // the filtered form has one shape
+            if (report != nullptr) {
+                *report = rep;
+            }
+            return;
+        }
+        // the scores of every candidate go to a slab here
+        uint64_t most = 0;
+        bool room = true;
+        for (const uha::SplitPlan& p : cands) {
+            most = std::max<uint64_t>(most, p.splits);
+            room = room && ensure_split_workspace(ws, index, sp->pitch, batch, p);
+        }
+        const uint64_t slab = checked_mul(checked_mul(most, batch, "partials"), index->rows,
+                                          "partials");
+        if (room && ws->split_partials.size() < slab) {
+            check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
+            room = ws->split_partials.try_allocate(slab);
+        }
+        if (!room) {
+            ws->split_disabled = true;
+            autotune(index, ws, batch, strategy, report);
+            return;
+        }
+        check_cuda(cudaMemsetAsync(ws->split_queries.get(), 0, ws->split_queries.bytes(),
+                                   stream),
+                   "cannot clear the query buffer");
+        int* flag = reinterpret_cast<int*>(ws->counters.get() + 1);
+        for (size_t i = 0; i < cands.size(); ++i) {
+            const uha::SplitPlan& p = cands[i];
+            const double ms = time_launches(stream, reps, [&] {
+                uha::launch_split_scores(p, sp->data.get(), index->rows,
+                                         ws->split_queries.get(), batch, sp->pitch,
+                                         ws->split_partials.get(), flag, index->sm_count,
+                                         stream);
+            });
+            if (i == 0) {
+                rep.default_ms = ms;
+            }
+            if (best.ms < 0 || ms < best.ms) {
+                best.ms = ms;
+                best.split = true;
+                best.split_plan = p;
+            }
+        }
+        best.candidates = static_cast<int>(cands.size());
+        rep.kernel = 2;
+        rep.tile_queries = static_cast<uint32_t>(best.split_plan.bn);
+        rep.splits = best.split_plan.splits;
     } else {
         const bool hierarchical = index->kind == IndexKind::hierarchical;
         const float* queries = hierarchical ? ws->projected.get() : ws->prepared.get();
@@ -464,6 +521,8 @@ uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_c
             check_cuda(cudaEventCreateWithFlags(&p.join, cudaEventDisableTiming),
                        "cannot create CUDA event");
             uha_workspace* ws = p.ws;
+            // the persistent kernels' units are the binary32 scan's
+            ws->split_disabled = persistent;
             ws->call_results.allocate(p.count);
             ws->call_exact.allocate(p.count);
             ws->host_results.allocate(p.count);
@@ -628,18 +687,24 @@ extern "C" uha_status uha_batch_run(uha_batch* batch, const float* const* querie
                 continue;
             }
             if ((p.ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u) {
-                // a filtered candidate list overflowed: this pair again,
-                // eagerly, with the slab selection (its queries are still in
-                // the workspace)
-                p.ws->filter_disabled = true;
-                try {
-                    enqueue_pair(p);
-                    check_cuda(cudaStreamSynchronize(p.ws->stream), "CUDA batch failed");
-                } catch (...) {
-                    p.ws->filter_disabled = false;
-                    throw;
+                // a candidate list overflowed: this pair again, without the
+                // list, in a workspace of its own (the graph reads and writes
+                // the pair's buffers, which such a run would replace)
+                uha_workspace* again = nullptr;
+                uha_status status = uha_workspace_create(p.index, p.count, &again);
+                if (status == UHA_OK) {
+                    again->filter_disabled = true;
+                    again->candidates_per_query = p.ws->candidates_per_query;
+                    status = uha_query(p.index, again, p.ws->raw_queries.get(), p.count, 1,
+                                       p.strategy, idx, dist);
+                    st.replayed_queries += again->last.replayed_queries;
                 }
-                p.ws->filter_disabled = false;
+                const std::string message = status != UHA_OK ? uha_last_error() : "";
+                uha_workspace_destroy(again);
+                if (status != UHA_OK) {
+                    fail(status, message);
+                }
+                continue;
             }
             finish_call(p.index, p.ws, p.count, p.ws->host_results.get(),
                         p.ws->host_exact.get(), idx, dist);

@@ -26,6 +26,7 @@
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 namespace uha {
@@ -669,7 +670,8 @@ __device__ void resolve_without_fp64(const ReplayInputs& in, const float* qrow,
 // binary64 squared distance in the projected space (j order); the block keeps
 // the lexicographic minimum of (distance, row).
 __global__ void __launch_bounds__(kFinalizeThreads)
-    rescore_projected_kernel(const uint32_t* __restrict__ candidates, uint32_t k,
+    rescore_projected_kernel(const uint32_t* __restrict__ candidates, uint32_t stride,
+                             const uint32_t* __restrict__ counts,
                              const double* __restrict__ rows64,
                              const double* __restrict__ y64, uint32_t p, Result* results,
                              double* exact_distances)
@@ -679,10 +681,11 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const double* y = y64 + static_cast<uint64_t>(q) * p;
+    const uint32_t k = counts != nullptr ? min(counts[q], stride) : stride;
     double best = __longlong_as_double(0x7ff0000000000000ll);
     uint32_t best_row = 0xffffffffu;
     for (uint32_t i = warp; i < k; i += warps) {
-        const uint32_t row = candidates[static_cast<uint64_t>(q) * k + i];
+        const uint32_t row = candidates[static_cast<uint64_t>(q) * stride + i];
         if (row == 0xffffffffu) {
             continue;
         }
@@ -1889,6 +1892,87 @@ __device__ __forceinline__ Interval64 interval64(double s, const Bound64& b)
     return {lo > 0.0 ? lo : 0.0, hi};
 }
 
+// Block-wide: the answer of one query among k candidates with binary64
+// distances dist[i] (both arrays in shared memory, synchronised): one candidate
+// whose interval can hold the reference minimum is the answer; otherwise the
+// candidates that can are replayed in the reference CPU's order (one warp each)
+// and the lexicographic minimum of (distance, row) wins. *exact_distance is
+// the binary64 distance of the answer.
+__device__ void settle64(const Bound64& bound, const ReplayInputs& in, const float* qrow,
+                         const uint32_t* cand, const double* dist, uint32_t k,
+                         uint32_t row_count, Result* result, double* exact_distance,
+                         uint32_t* replay_count)
+{
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    __shared__ bool certified;
+    __shared__ double min_upper;
+    if (threadIdx.x == 0) {
+        double first = inf, second = inf, upper = inf;
+        uint32_t first_i = 0xffffffffu;
+        for (uint32_t i = 0; i < k; ++i) {
+            if (cand[i] >= row_count) {
+                continue;
+            }
+            const Interval64 b = interval64(dist[i], bound);
+            upper = fmin(upper, b.upper);
+            if (first_i == 0xffffffffu || b.lower < first ||
+                (b.lower == first && cand[i] < cand[first_i])) {
+                second = first;
+                first = b.lower;
+                first_i = i;
+            } else if (b.lower < second) {
+                second = b.lower;
+            }
+        }
+        certified = first_i != 0xffffffffu && second > upper;
+        min_upper = upper;
+        if (certified) {
+            *result = Result{cand[first_i], static_cast<float>(dist[first_i])};
+            *exact_distance = dist[first_i];
+        } else {
+            atomicAdd(replay_count, 1u);
+        }
+    }
+    __syncthreads();
+    if (certified) {
+        return;
+    }
+    constexpr int warps = kFinalizeThreads / 32;
+    const int warp = threadIdx.x / 32;
+    const int lane = threadIdx.x % 32;
+    double best = inf;
+    uint32_t best_row = 0xffffffffu;
+    for (uint32_t i = warp; i < k; i += warps) {
+        const uint32_t r = cand[i];
+        if (r >= row_count || interval64(dist[i], bound).lower > min_upper) {
+            continue;
+        }
+        const double v = replay_row(in, qrow, in.rows + static_cast<uint64_t>(r) * in.padded_dim,
+                                    lane);
+        if (lex_less(v, r, best, best_row)) {
+            best = v;
+            best_row = r;
+        }
+    }
+    __shared__ double warp_best[warps];
+    __shared__ uint32_t warp_best_row[warps];
+    if (lane == 0) {
+        warp_best[warp] = best;
+        warp_best_row[warp] = best_row;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 0; w < warps; ++w) {
+            if (lex_less(warp_best[w], warp_best_row[w], best, best_row)) {
+                best = warp_best[w];
+                best_row = warp_best_row[w];
+            }
+        }
+        *result = Result{best_row, static_cast<float>(best)};
+        *exact_distance = best;
+    }
+}
+
 // Certified argmin of each query over its candidate rows (the precision
 // form). grid = (k, batch): CTA (c, q) computes the binary64 distance of
 // candidate c; the last CTA of the query to finish decides. One candidate
@@ -1931,74 +2015,11 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         cand[i] = candidates[static_cast<uint64_t>(q) * k + i];
     }
     __syncthreads();
-    __shared__ bool certified;
-    __shared__ double min_upper;
     if (threadIdx.x == 0) {
         done[q] = 0;
-        double first = inf, second = inf, upper = inf;
-        uint32_t first_i = 0xffffffffu;
-        for (uint32_t i = 0; i < k; ++i) {
-            if (cand[i] >= row_count) {
-                continue;
-            }
-            const Interval64 b = interval64(dist[i], bound);
-            upper = fmin(upper, b.upper);
-            if (first_i == 0xffffffffu || b.lower < first ||
-                (b.lower == first && cand[i] < cand[first_i])) {
-                second = first;
-                first = b.lower;
-                first_i = i;
-            } else if (b.lower < second) {
-                second = b.lower;
-            }
-        }
-        certified = first_i != 0xffffffffu && second > upper;
-        min_upper = upper;
-        if (certified) {
-            results[q] = Result{cand[first_i], static_cast<float>(dist[first_i])};
-            exact_distances[q] = dist[first_i];
-        } else {
-            atomicAdd(replay_count, 1u);
-        }
     }
-    __syncthreads();
-    if (certified) {
-        return;
-    }
-    constexpr int warps = kFinalizeThreads / 32;
-    const int warp = threadIdx.x / 32;
-    const int lane = threadIdx.x % 32;
-    double best = inf;
-    uint32_t best_row = 0xffffffffu;
-    for (uint32_t i = warp; i < k; i += warps) {
-        const uint32_t r = cand[i];
-        if (r >= row_count || interval64(dist[i], bound).lower > min_upper) {
-            continue;
-        }
-        const double v = replay_row(in, qrow, in.rows + static_cast<uint64_t>(r) * in.padded_dim,
-                                    lane);
-        if (lex_less(v, r, best, best_row)) {
-            best = v;
-            best_row = r;
-        }
-    }
-    __shared__ double warp_best[warps];
-    __shared__ uint32_t warp_best_row[warps];
-    if (lane == 0) {
-        warp_best[warp] = best;
-        warp_best_row[warp] = best_row;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 0; w < warps; ++w) {
-            if (lex_less(warp_best[w], warp_best_row[w], best, best_row)) {
-                best = warp_best[w];
-                best_row = warp_best_row[w];
-            }
-        }
-        results[q] = Result{best_row, static_cast<float>(best)};
-        exact_distances[q] = best;
-    }
+    settle64(bound, in, qrow, cand, dist, k, row_count, results + q, exact_distances + q,
+             replay_count);
 }
 
 // Binary32 squared distance of one row summed by the whole block with the
@@ -2060,6 +2081,60 @@ __device__ float block_l2_32(const float* q, const float* r, uint64_t padded_dim
                                __fadd_rn(scratch[6], scratch[7])));
 }
 
+// The same with binary32 distances and without FP64 instructions: candidates
+// the bounds do not separate are settled by resolve_without_fp64.
+__device__ void settle32(const Bound& bound, const ReplayInputs& in, const float* qrow,
+                         const uint32_t* cand, const float* dist, uint32_t k,
+                         uint32_t row_count, uint32_t q, Result* result,
+                         double* exact_distance, uint32_t* replay_count)
+{
+    const float inf = __int_as_float(0x7f800000);
+    __shared__ bool certified;
+    __shared__ float min_upper;
+    if (threadIdx.x == 0) {
+        float first = inf, second = inf, upper = inf;
+        uint32_t first_i = 0xffffffffu;
+        for (uint32_t i = 0; i < k; ++i) {
+            if (cand[i] >= row_count) {
+                continue;
+            }
+            const Bounds2 b = bound_of(dist[i], bound, cand[i], q);
+            upper = fminf(upper, b.upper);
+            if (first_i == 0xffffffffu || b.lower < first ||
+                (b.lower == first && cand[i] < cand[first_i])) {
+                second = first;
+                first = b.lower;
+                first_i = i;
+            } else if (b.lower < second) {
+                second = b.lower;
+            }
+        }
+        certified = first_i != 0xffffffffu && second > upper;
+        min_upper = upper;
+        if (certified) {
+            *result = Result{cand[first_i], dist[first_i]};
+            *exact_distance = __longlong_as_double(
+                static_cast<long long>(x64::from_float(dist[first_i])));
+        } else {
+            atomicAdd(replay_count, 1u);
+        }
+    }
+    __syncthreads();
+    if (certified) {
+        return;
+    }
+    __shared__ ResolveSmem rs;
+    resolve_begin(rs);
+    for (uint32_t i = threadIdx.x; i < k; i += kFinalizeThreads) {
+        if (cand[i] < row_count && bound_of(dist[i], bound, cand[i], q).lower <= min_upper) {
+            resolve_push(rs, cand[i]);
+        }
+    }
+    // k <= kMaxCandidates < kResolveCap: the list never overflows
+    resolve_without_fp64(in, qrow, rs, row_count, [](uint32_t) { return false; },
+                         result, exact_distance);
+}
+
 // The FP32 re-score of the precision strategies, without FP64 instructions.
 // grid = (k, batch): CTA (c, q) computes candidate c's binary32 distance from
 // the original rows; the last CTA of the query certifies: one candidate whose
@@ -2101,51 +2176,93 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         cand[i] = candidates[static_cast<uint64_t>(q) * k + i];
     }
     __syncthreads();
-    __shared__ bool certified;
-    __shared__ float min_upper;
     if (threadIdx.x == 0) {
         done[q] = 0;
-        float first = inf, second = inf, upper = inf;
-        uint32_t first_i = 0xffffffffu;
-        for (uint32_t i = 0; i < k; ++i) {
-            if (cand[i] >= row_count) {
-                continue;
-            }
-            const Bounds2 b = bound_of(dist[i], bound, cand[i], q);
-            upper = fminf(upper, b.upper);
-            if (first_i == 0xffffffffu || b.lower < first ||
-                (b.lower == first && cand[i] < cand[first_i])) {
-                second = first;
-                first = b.lower;
-                first_i = i;
-            } else if (b.lower < second) {
-                second = b.lower;
-            }
-        }
-        certified = first_i != 0xffffffffu && second > upper;
-        min_upper = upper;
-        if (certified) {
-            results[q] = Result{cand[first_i], dist[first_i]};
-            exact_distances[q] = __longlong_as_double(
-                static_cast<long long>(x64::from_float(dist[first_i])));
-        } else {
-            atomicAdd(replay_count, 1u);
-        }
     }
-    __syncthreads();
-    if (certified) {
+    settle32(bound, in, qrow, cand, dist, k, row_count, q, results + q, exact_distances + q,
+             replay_count);
+}
+
+// The candidate lists of the split scan (split_scan.cu). grid = (parts, batch):
+// each block sums its part of the columns for every candidate of the query
+// (usually one or two), from the original binary32 rows; the query's last block
+// adds the parts in order and settles the query, in binary64 or, with
+// kEmulated, without FP64 instructions. Bound: memory (a candidate's row and
+// the query); the parts spread a small batch over the chip (64 queries x
+// 60,660 columns: 58 us with one block per query, 19 us with 16). A query
+// without candidates (its list overflowed, so the call is answered again) gets
+// row 0.
+template <bool kEmulated>
+__global__ void __launch_bounds__(kFinalizeThreads)
+    settle_kernel(Bound64 bound64, Bound bound32, ReplayInputs in,
+                  const uint32_t* __restrict__ candidates,
+                  const uint32_t* __restrict__ counts, uint32_t row_count, double* sums,
+                  uint32_t* done, Result* results, double* exact_distances,
+                  uint32_t* replay_count)
+{
+    using T = std::conditional_t<kEmulated, float, double>;
+    static_assert(kSplitCandidates <= kMaxCandidates, "candidate lists fit the settlement");
+    __shared__ T scratch[kFinalizeThreads / 32];
+    __shared__ T dist[kSplitCandidates];
+    __shared__ uint32_t cand[kSplitCandidates];
+    __shared__ bool is_last;
+    const uint32_t q = blockIdx.y;
+    const uint32_t parts = gridDim.x;
+    const uint32_t k = min(counts[q], kSplitCandidates);
+    if (k == 0) {
+        if (threadIdx.x == 0 && blockIdx.x == 0) {
+            results[q] = Result{0, 0.f};
+            exact_distances[q] = __longlong_as_double(0x7ff8000000000000ll);
+        }
         return;
     }
-    __shared__ ResolveSmem rs;
-    resolve_begin(rs);
-    for (uint32_t i = threadIdx.x; i < k; i += kFinalizeThreads) {
-        if (cand[i] < row_count && bound_of(dist[i], bound, cand[i], q).lower <= min_upper) {
-            resolve_push(rs, cand[i]);
+    const float* qrow = in.queries + static_cast<uint64_t>(q) * in.padded_dim;
+    const uint64_t width = (in.padded_dim / 4 + parts - 1) / parts * 4;
+    const uint64_t begin = min(in.padded_dim, blockIdx.x * width);
+    const uint64_t end = min(in.padded_dim, begin + width);
+    // parts[q][candidate][part]; the emulated form keeps binary32 sums there
+    T* mine = reinterpret_cast<T*>(sums) +
+              static_cast<uint64_t>(q) * kSplitCandidates * parts;
+    for (uint32_t i = 0; i < k; ++i) {
+        const uint32_t row = candidates[static_cast<uint64_t>(q) * kSplitCandidates + i];
+        const float* rrow = in.rows + static_cast<uint64_t>(row) * in.padded_dim;
+        T d;
+        if constexpr (kEmulated) {
+            d = block_l2_32(qrow + begin, rrow + begin, end - begin, scratch);
+        } else {
+            d = block_l2_64(qrow + begin, rrow + begin, end - begin, scratch);
+        }
+        __syncthreads();  // scratch is free again
+        if (threadIdx.x == 0) {
+            mine[i * parts + blockIdx.x] = d;
         }
     }
-    // k <= kMaxCandidates < kResolveCap: the list never overflows
-    resolve_without_fp64(in, qrow, rs, row_count, [](uint32_t) { return false; },
-                         results + q, exact_distances + q);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        is_last = atomicAdd(done + q, 1u) == parts - 1;
+    }
+    __syncthreads();
+    if (!is_last) {
+        return;
+    }
+    __threadfence();
+    for (uint32_t i = threadIdx.x; i < k; i += kFinalizeThreads) {
+        T d = static_cast<volatile T*>(mine)[i * parts];
+        for (uint32_t p = 1; p < parts; ++p) {
+            d = kEmulated ? __fadd_rn(d, static_cast<volatile T*>(mine)[i * parts + p])
+                          : d + static_cast<volatile T*>(mine)[i * parts + p];
+        }
+        dist[i] = d;
+        cand[i] = candidates[static_cast<uint64_t>(q) * kSplitCandidates + i];
+    }
+    __syncthreads();
+    if constexpr (kEmulated) {
+        settle32(bound32, in, qrow, cand, dist, k, row_count, q, results + q,
+                 exact_distances + q, replay_count);
+    } else {
+        settle64(bound64, in, qrow, cand, dist, k, row_count, results + q,
+                 exact_distances + q, replay_count);
+    }
 }
 
 // ------------------------------------------ the persistent multi-index batch
@@ -2565,10 +2682,10 @@ void launch_argmin(PartialView view, Bound bound, ReplayInputs in,
 void launch_rescore_projected(const uint32_t* candidates, uint32_t k, uint32_t batch,
                               const double* rows64, const double* y64, uint32_t p,
                               Result* results, double* exact_distances,
-                              cudaStream_t stream)
+                              cudaStream_t stream, const uint32_t* counts)
 {
     rescore_projected_kernel<<<batch, kFinalizeThreads, 0, stream>>>(
-        candidates, k, rows64, y64, p, results, exact_distances);
+        candidates, k, counts, rows64, y64, p, results, exact_distances);
     check_cuda(cudaGetLastError(), "cannot launch projected re-score kernel");
 }
 
@@ -2609,6 +2726,49 @@ void launch_rescore32(Bound bound, ReplayInputs in, const uint32_t* candidates,
         bound, in, candidates, k, rows, cand_dist, done, results, exact_distances,
         replay_count);
     check_cuda(cudaGetLastError(), "cannot launch FP32 re-score kernel");
+}
+
+namespace {
+
+// Blocks per query: eight per SM in all, at most 16 (about 4,000 columns of a
+// 60,660-column row each).
+constexpr uint32_t kSettleBlocks = 8 * 148;
+constexpr uint32_t kSettleParts = 16;
+
+uint32_t settle_parts(uint64_t batch)
+{
+    return static_cast<uint32_t>(
+        std::max<uint64_t>(1, std::min<uint64_t>(kSettleParts, kSettleBlocks / batch)));
+}
+
+}  // namespace
+
+uint32_t settle_depth(uint64_t padded_dim)
+{
+    return rescore_depth(padded_dim) + kSettleParts;
+}
+
+uint64_t settle_sums(uint64_t batch)
+{
+    // batch x parts is at most this for every smaller batch
+    return kSplitCandidates * std::max<uint64_t>(kSettleBlocks, batch);
+}
+
+void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32_t* candidates,
+                   const uint32_t* counts, uint32_t batch, uint32_t rows, double* sums,
+                   uint32_t* done, Result* results, double* exact_distances,
+                   uint32_t* replay_count, cudaStream_t stream)
+{
+    if (batch == 0) {
+        return;
+    }
+    // short rows are one part
+    const uint32_t parts = in.padded_dim >= 8192 ? settle_parts(batch) : 1;
+    const auto kernel = in.emulated ? settle_kernel<true> : settle_kernel<false>;
+    kernel<<<dim3(parts, batch), kFinalizeThreads, 0, stream>>>(
+        bound64, bound32, in, candidates, counts, rows, sums, done, results, exact_distances,
+        replay_count);
+    check_cuda(cudaGetLastError(), "cannot launch the settlement kernel");
 }
 
 void emulated_replay_bound(uint64_t dim, float* rel, float* abs)

@@ -96,6 +96,22 @@ public:
         ptr_ = static_cast<T*>(p);
         count_ = count;
     }
+    // allocate(), but false (and empty) when the device has no room.
+    bool try_allocate(uint64_t count)
+    {
+        release();
+        void* p = nullptr;
+        const cudaError_t e =
+            cudaMalloc(&p, checked_mul(count, sizeof(T), "device buffer"));
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return false;
+        }
+        check_cuda(e, "cannot allocate device memory");
+        ptr_ = static_cast<T*>(p);
+        count_ = count;
+        return true;
+    }
     void release() noexcept
     {
         if (ptr_ != nullptr) {

@@ -1073,6 +1073,49 @@ const uha::LowpRows& lowp_rows(const uha_index* index, uha::LowpType type,
     return lp;
 }
 
+bool split_shape(const uha_index* index, uha_strategy strategy, uint64_t n)
+{
+    return strategy == UHA_DIRECT && index->metric == UHA_L2 && n > 8 && n <= 65535 &&
+           index->rows >= 2 && !small_path_applies(index, strategy);
+}
+
+bool ensure_split_workspace(uha_workspace* ws, const uha_index* index, uint64_t pitch,
+                            uint64_t n, const uha::SplitPlan& plan)
+{
+    cudaStream_t stream = ws->stream;
+    // grows a buffer that earlier work on the stream may still use
+    auto grow = [&](auto& buffer, uint64_t count) {
+        if (buffer.size() >= count) {
+            return true;
+        }
+        check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
+        return buffer.try_allocate(count);
+    };
+    const uint64_t b = ws->max_batch;
+    const uint64_t bytes = checked_mul(
+        checked_mul(uha::lowp_padded_count(b), pitch, "query buffer"), 4, "query buffer");
+    if (ws->split_queries.size() < bytes) {
+        if (!grow(ws->split_queries, bytes)) {
+            return false;
+        }
+        // vectors past a batch are read by the score kernel (and not stored)
+        check_cuda(cudaMemsetAsync(ws->split_queries.get(), 0, bytes, stream),
+                   "cannot clear the query buffer");
+    }
+    const bool filter = uha::split_filter_applies(plan, index->rows);
+    const uint64_t partials =
+        filter ? 0
+               : checked_mul(checked_mul(plan.splits, n, "partials"), index->rows, "partials");
+    const bool hierarchical = index->kind == IndexKind::hierarchical;
+    return grow(ws->split_squares, b * uha::kSplitSlices) && grow(ws->split_words, 3 * b) &&
+           grow(ws->split_candidates, b * uha::kSplitCandidates) &&
+           grow(ws->split_partials, partials) &&
+           (!filter || grow(ws->split_keys, checked_mul(b, uha::kSplitListKeys, "keys"))) &&
+           (hierarchical
+                ? grow(ws->projected64, checked_mul(b, index->projection_dimension, "queries"))
+                : grow(ws->split_sums, uha::settle_sums(b)));
+}
+
 // Workspace buffers of the precision strategies for batches up to max_batch.
 void ensure_lowp_workspace(uha_workspace* ws, const uha_index* index,
                            cudaStream_t stream)
@@ -1155,6 +1198,9 @@ void enqueue_hierarchical_projection(const uha_index* index, uha_workspace* ws,
                    "cannot clear the query buffer");
         ws->gathered_scales.allocate(uha::lowp_padded_count(ws->max_batch));
         ws->gathered_amax.allocate(uha::lowp_padded_count(ws->max_batch));
+    }
+    if (ws->projected64.size() < ws->max_batch * p) {
+        check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
         ws->projected64.allocate(checked_mul(ws->max_batch, p, "projected queries"));
     }
     uha::launch_lowp_queries(type, ws->prepared.get(), n, index->padded_sample,
@@ -1317,6 +1363,93 @@ uint64_t enqueue_lowp_candidates(const BatchContext& c, uint64_t n, const uha::L
     return 6;
 }
 
+// The split form of the index's rows (split_scan.cu), built on first use on
+// `stream` and synchronised before it is published; null when the index keeps
+// the binary32 scan.
+const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
+{
+    std::lock_guard<std::mutex> lock(index->lowp_mutex);
+    uha::SplitRows& sp = index->split;
+    if (sp.ready) {
+        return sp.usable ? &sp : nullptr;
+    }
+    const bool hierarchical = index->kind == IndexKind::hierarchical;
+    sp.pitch = uha::split_pitch(index->scan_dim);
+    const uint64_t bytes = checked_mul(
+        checked_mul(uha::lowp_padded_count(index->rows), sp.pitch, "split rows"), 4,
+        "split rows");
+    if (!sp.data.try_allocate(bytes) || !sp.norms.try_allocate(index->rows) ||
+        !sp.roots.try_allocate(index->rows + 1) || !sp.centre.try_allocate(sp.pitch)) {
+        sp = uha::SplitRows{};
+        sp.ready = true;
+        return nullptr;
+    }
+    // the word past the roots receives the largest of them
+    unsigned int* largest = reinterpret_cast<unsigned int*>(sp.roots.get() + index->rows);
+    check_cuda(cudaMemsetAsync(sp.data.get(), 0, bytes, stream), "cannot clear split rows");
+    auto split = [&] {
+        if (hierarchical) {
+            uha::launch_split_rows(index->rows64.get(), index->rows, index->scan_dim,
+                                   index->scan_dim, sp.data.get(), sp.pitch, sp.scale,
+                                   sp.centre.get(), sp.norms.get(), sp.roots.get(), largest,
+                                   stream);
+        } else {
+            uha::launch_split_rows(index->scan_rows.get(), index->rows, index->padded_dim,
+                                   index->scan_dim, sp.data.get(), sp.pitch, sp.scale,
+                                   sp.centre.get(), sp.norms.get(), sp.roots.get(), largest,
+                                   stream);
+        }
+        float root = 0.f;
+        check_cuda(cudaMemcpyAsync(&root, largest, sizeof(root), cudaMemcpyDeviceToHost, stream),
+                   "cannot copy the largest norm from the CUDA device");
+        check_cuda(cudaStreamSynchronize(stream), "cannot build split rows");
+        return root;
+    };
+    float root = split();
+    if (std::isfinite(root) && root > 0.f && (root < 0x1p-8f || root > 0x1p24f)) {
+        sp.scale = std::ldexp(1.f, -std::clamp(std::ilogb(root), -126, 126));
+        root = split();
+    }
+    sp.ready = true;
+    sp.usable = root <= uha::split_largest_norm();
+    if (!sp.usable) {
+        sp.data.release();
+    }
+    return sp.usable ? &sp : nullptr;
+}
+
+// The split scan of this batch, or false when it takes the binary32 scan: the
+// direct strategy on L2 indexes, batches past the streaming scan's, whose
+// caller answers a call again when a candidate list overflows. Everything the
+// batch needs is allocated here.
+bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** rows,
+                   uha::SplitPlan* plan)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+        !split_shape(index, c.strategy, n)) {
+        return false;
+    }
+    const uha::SplitRows* sp = split_rows(index, ws->stream);
+    if (sp == nullptr) {
+        return false;
+    }
+    const TunedPlan* tuned = ws->find_tuned(n, static_cast<int>(c.strategy));
+    if (tuned != nullptr && !tuned->split) {
+        return false;
+    }
+    *plan = tuned != nullptr
+                ? tuned->split_plan
+                : uha::plan_split(index->rows, sp->pitch, n, index->sm_count);
+    *rows = sp;
+    if (!ensure_split_workspace(ws, index, sp->pitch, n, *plan)) {
+        ws->split_disabled = true;
+        return false;
+    }
+    return true;
+}
+
 // One query batch's kernels on the workspace stream: gather / copy with
 // validation, (projection), scan, certified argmin with in-kernel replay (or
 // the norm identity), (the replayed distance of each selected row of a
@@ -1400,7 +1533,7 @@ bool persistent_pair(const uha_index* index, uha_workspace* ws, uint64_t n,
     const TunedPlan* tuned = ws->find_tuned(n, static_cast<int>(UHA_DIRECT));
     uha::ScanPlan plan = uha::plan_scan(index->rows, index->padded_dim, n, index->sm_count);
     if (!median && tuned != nullptr && !tuned->lowp && !tuned->median &&
-        tuned->scan.kernel == 1) {
+        !tuned->split && tuned->scan.kernel == 1) {
         plan = tuned->scan;
     }
     if (median) {
@@ -1492,6 +1625,104 @@ void ensure_flat_scratch(const uha_index* index, uha_workspace* ws)
                "cannot clear flat query scratch");
 }
 
+// One batch by the split scan: gather / copy with validation (and, for a
+// hierarchy, the reference's binary64 projection), the split queries, the
+// tensor-core estimates, every row that can be the minimum, and their
+// settlement from the original values.
+uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
+                             const uha::SplitPlan& plan, const float* source, uint64_t n,
+                             uha::Result* results, double* exact, bool time_scan,
+                             cudaEvent_t scan_start, cudaEvent_t scan_stop)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    cudaStream_t stream = ws->stream;
+    int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
+    const bool hierarchical = index->kind == IndexKind::hierarchical;
+    const uint32_t b = static_cast<uint32_t>(n);
+    uint32_t* words = ws->split_words.get();
+    uha::SplitVectors v{};
+    v.source = source;
+    v.source_pitch = index->dimension;
+    v.dim = index->scan_dim;
+    v.columns = index->columns.get();
+    v.scales = index->scales.get();
+    v.centre = rows.centre.get();
+    v.scale = rows.scale;
+    v.out = ws->split_queries.get();
+    v.pitch = rows.pitch;
+    v.prepared = ws->prepared.get();
+    v.prepared_pitch = index->padded_dim;
+    v.squares = ws->split_squares.get();
+    v.counts = words;
+    v.upper = words + ws->max_batch;
+    v.done = words + 2 * ws->max_batch;
+    v.error_flag = error_flag;
+    uint64_t launches = 1;
+    if (hierarchical) {
+        const uint64_t p = index->projection_dimension;
+        uha::launch_prepare_sampled(source, n, index->dimension, index->columns.get(), nullptr,
+                                    index->sample_size, ws->prepared.get(),
+                                    index->padded_sample, error_flag, stream);
+        uha::launch_project_queries64(ws->prepared.get(), n, index->padded_sample,
+                                      index->sample_size, index->projection64_t.get(), p,
+                                      ws->projected64.get(), error_flag, stream);
+        v.source = ws->projected64.get();
+        v.source_pitch = p;
+        launches += 2;
+    }
+    uha::launch_split_queries(v, n, hierarchical, stream);
+    const uha::SplitQuery sq{rows.norms.get(),
+                             rows.roots.get(),
+                             v.squares,
+                             uha::split_slices(rows.pitch, n),
+                             uha::split_error_rel(plan, index->rows),
+                             v.upper,
+                             v.counts};
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_start, stream), "event");
+    }
+    if (uha::split_filter_applies(plan, index->rows)) {
+        uha::launch_split_filter_scan(plan, rows.data.get(), index->rows,
+                                      ws->split_queries.get(), n, rows.pitch, sq,
+                                      ws->split_keys.get(), ws->split_candidates.get(),
+                                      error_flag, index->sm_count, stream);
+        launches += 3;
+    } else {
+        uha::launch_split_scan(plan, rows.data.get(), index->rows, ws->split_queries.get(), n,
+                               rows.pitch, ws->split_partials.get(), sq,
+                               ws->split_candidates.get(), error_flag, index->sm_count, stream);
+        launches += 3;
+    }
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_stop, stream), "event");
+    }
+    if (hierarchical) {
+        // the reference's binary64 distance of every listed row, in the
+        // projected space; the smallest (lowest row on ties) is the answer
+        uha::launch_rescore_projected(
+            ws->split_candidates.get(), uha::kSplitCandidates, b, index->rows64.get(),
+            ws->projected64.get(), static_cast<uint32_t>(index->projection_dimension), results,
+            exact, stream, v.counts);
+        return launches + 1;
+    }
+    uha::ReplayInputs in{};
+    in.op = uha::ReplayOp::l2_sequential;
+    in.rows = index->scan_rows.get();
+    in.queries = ws->prepared.get();
+    in.dim = index->scan_dim;
+    in.padded_dim = index->padded_dim;
+    if (ws->emulated_replay) {
+        set_emulated(in, index);
+    }
+    const uint32_t depth = uha::settle_depth(index->padded_dim);
+    uha::launch_settle(uha::make_bound64(depth, index->scan_dim),
+                       make_bound(depth, index->scan_dim, 2), in, ws->split_candidates.get(),
+                       v.counts, b, static_cast<uint32_t>(index->rows), ws->split_sums.get(),
+                       v.done, results, exact, ws->counters.get(), stream);
+    return launches + 1;
+}
+
 uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
                        uha::Result* results, double* exact, bool time_scan,
                        cudaEvent_t scan_start, cudaEvent_t scan_stop)
@@ -1562,6 +1793,12 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
             check_cuda(cudaEventRecord(scan_stop, stream), "event");
         }
         return 1;
+    }
+    const uha::SplitRows* split = nullptr;
+    uha::SplitPlan split_plan{};
+    if (split_applies(c, n, &split, &split_plan)) {
+        return enqueue_split_batch(c, *split, split_plan, source, n, results, exact, time_scan,
+                                   scan_start, scan_stop);
     }
     float* prepared = c.prepared != nullptr ? c.prepared : ws->prepared.get();
     const float* scan_queries = prepared;
@@ -1661,7 +1898,7 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     }
     const bool median = hierarchical && index->metric == UHA_L1;
     const TunedPlan* tuned = ws->find_tuned(n, static_cast<int>(c.strategy));
-    uha::ScanPlan plan = tuned != nullptr && !tuned->lowp && !tuned->median
+    uha::ScanPlan plan = tuned != nullptr && !tuned->lowp && !tuned->median && !tuned->split
                              ? tuned->scan
                              : uha::plan_scan(index->rows, index->padded_dim, n,
                                               index->sm_count);
@@ -1864,7 +2101,8 @@ void prepare_pipeline(const uha_index* index, uha_workspace* ws, uha_strategy st
     uint64_t per_slot = 0;
     for (uint64_t n = 1; n <= batch; ++n) {
         const TunedPlan* tuned = ws->find_tuned(n, static_cast<int>(strategy));
-        const uha::ScanPlan plan = tuned != nullptr && !tuned->lowp && !tuned->median
+        const uha::ScanPlan plan = tuned != nullptr && !tuned->lowp && !tuned->median &&
+                                           !tuned->split
                                        ? tuned->scan
                                        : uha::plan_scan(index->rows, index->padded_dim, n,
                                                         index->sm_count);

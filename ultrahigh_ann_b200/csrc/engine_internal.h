@@ -22,6 +22,15 @@ const uha::LowpRows& lowp_rows(const uha_index* index, uha::LowpType type,
 void ensure_lowp_workspace(uha_workspace* ws, const uha_index* index,
                            cudaStream_t stream);
 
+// Batches of n queries that the certified split scan (split_scan.cu) can serve;
+// the split form of the index's rows (null: the index keeps the binary32 scan);
+// and the workspace buffers of a batch of n with this plan (false when the device
+// has no room).
+bool split_shape(const uha_index* index, uha_strategy strategy, uint64_t n);
+const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream);
+bool ensure_split_workspace(uha_workspace* ws, const uha_index* index, uint64_t pitch,
+                            uint64_t n, const uha::SplitPlan& plan);
+
 struct BatchContext {
     const uha_index* index;
     uha_workspace* ws;
@@ -39,9 +48,10 @@ struct BatchContext {
     uint32_t* rescore_done = nullptr;
     cudaStream_t finish_stream = nullptr;
     cudaEvent_t handoff = nullptr;
-    // The precision strategies may take the fused candidate selection: the
-    // caller answers the call again without it when a candidate list
-    // overflows (error bit uha::kCandidateOverflow).
+    // The precision strategies may take the fused candidate selection, and the
+    // direct strategy the split scan: the caller answers the call again without
+    // them (ws->filter_disabled) when a candidate list overflows (error bit
+    // uha::kCandidateOverflow).
     bool filter_candidates = false;
     // The fused flat query of this batch runs on stream lane `flat_lane`
     // (0: ws->stream; others: ws->flat_streams, forked and joined by the

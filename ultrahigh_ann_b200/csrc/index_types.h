@@ -29,6 +29,22 @@ struct LowpRows {
     bool ready = false;
 };
 
+// The split form of an L2 index's scanned rows (split_scan.cu), built on first
+// use: lowp_padded_count(rows) vectors of 2 x pitch BF16 values, their centre,
+// squared norms and roots. `usable` is false when the memory for it was not
+// available or a norm is past the bound's range; such an index keeps the
+// binary32 scan.
+struct SplitRows {
+    DeviceBuffer<unsigned char> data;
+    DeviceBuffer<float> centre;
+    DeviceBuffer<float> norms;
+    DeviceBuffer<float> roots;
+    uint64_t pitch = 0;
+    float scale = 1.f;
+    bool ready = false;
+    bool usable = false;
+};
+
 // Relative and absolute certification bound for a binary32 distance (defined
 // in engine.cu).
 Bound make_bound(uint32_t depth, uint64_t terms, int term_roundings);
@@ -74,6 +90,7 @@ struct uha_index {
     mutable std::mutex lowp_mutex;
     mutable uha::LowpRows lowp[2];
     mutable uha::LowpRows lowp_projection[2];  // L2 hierarchy: the p x k projection
+    mutable uha::SplitRows split;
 };
 
 // A scan shape chosen by the autotuner for one (batch size, strategy) of a
@@ -83,8 +100,10 @@ struct TunedPlan {
     int strategy = 0;
     bool lowp = false;
     bool median = false;  // median_plan holds the L1 hierarchy's median passes
+    bool split = false;   // split_plan holds the tensor-core certified scan
     uha::ScanPlan scan{};
     uha::LowpPlan lowp_plan{};
+    uha::SplitPlan split_plan{};
     uha::MedianPlan median_plan{};
     double ms = 0.0;
     int candidates = 0;
@@ -126,6 +145,19 @@ struct uha_workspace {
     uha::DeviceBuffer<uint32_t> filter_sample;
     uha::DeviceBuffer<float> filter_norms;  // the sample rows' norms
     bool filter_disabled = false;  // answering again after an overflow
+    // certified split scan (allocated on first use): split queries and their
+    // squared norms, partial estimates, per-query words (listed rows, smallest
+    // e + E, finished settlement blocks), candidate lists, the filter's
+    // keys, settlement sums. split_disabled: this workspace keeps the
+    // binary32 scan (persistent batches; no memory for these).
+    uha::DeviceBuffer<unsigned char> split_queries;
+    uha::DeviceBuffer<double> split_squares;
+    uha::DeviceBuffer<float> split_partials;
+    uha::DeviceBuffer<uint32_t> split_words;
+    uha::DeviceBuffer<uint32_t> split_candidates;
+    uha::DeviceBuffer<unsigned long long> split_keys;
+    uha::DeviceBuffer<double> split_sums;
+    bool split_disabled = false;
     uha::DeviceBuffer<uint32_t> candidates;       // [batch][candidates_per_query]
     uha::DeviceBuffer<double> cand_dist;          // [batch][candidates_per_query]
     uha::DeviceBuffer<uint32_t> rescore_done;     // per query, zero between calls

@@ -311,11 +311,12 @@ void launch_project_queries64(const float* x, uint64_t batch, uint64_t padded_k,
                               int* error_flag, cudaStream_t stream);
 // Per query, the candidate with the smallest (reference binary64 squared
 // distance of the projected row rows64[row] to y64[q], row): results[q] and
-// exact_distances[q]. Candidates 0xffffffff are skipped.
+// exact_distances[q]. Candidates 0xffffffff are skipped; with counts, query q
+// has counts[q] of its k slots filled.
 void launch_rescore_projected(const uint32_t* candidates, uint32_t k, uint32_t batch,
                               const double* rows64, const double* y64, uint32_t p,
                               Result* results, double* exact_distances,
-                              cudaStream_t stream);
+                              cudaStream_t stream, const uint32_t* counts = nullptr);
 // Binary64 certification interval [S (1 - rel) - abs, S (1 + rel) + abs] of
 // a parallel binary64 sum S of the reference CPU's own terms.
 struct Bound64 {
@@ -343,6 +344,120 @@ void launch_rescore32(Bound bound, ReplayInputs in, const uint32_t* candidates,
                       uint32_t k, uint32_t batch, uint32_t rows, float* cand_dist,
                       uint32_t* done, Result* results, double* exact_distances,
                       uint32_t* replay_count, cudaStream_t stream);
+
+// ---- certified L2 scan on the tensor cores (split_scan.cu)
+struct SplitPlan {
+    int bn;                      // queries per tile: 64, 128 or 256
+    uint32_t splits;             // column splits (partial-estimate slabs)
+    uint32_t kblocks;            // 64-column stages per vector
+    uint32_t kblocks_per_split;
+};
+// Columns of a split vector (a multiple of 64): it is stored as 2 x this many
+// BF16 values, in buffers of lowp_padded_count() vectors.
+uint64_t split_pitch(uint64_t dim);
+// The largest vector norm the estimates' bound covers.
+float split_largest_norm();
+// The centre (pitch floats) of the rows, and of the centred rows times `scale`
+// (a power of two) the split parts, squared norms and roots; *largest: bits of the largest root (infinity when one is not finite).
+// `out` is zero where no value is stored.
+void launch_split_rows(const float* rows, uint64_t row_count, uint64_t src_pitch, uint64_t dim,
+                       void* out, uint64_t pitch, float scale, float* centre, float* norms,
+                       float* roots, unsigned int* largest, cudaStream_t stream);
+void launch_split_rows(const double* rows, uint64_t row_count, uint64_t src_pitch, uint64_t dim,
+                       void* out, uint64_t pitch, float scale, float* centre, float* norms,
+                       float* roots, unsigned int* largest, cudaStream_t stream);
+// Candidate slots per query (at most max_rerank_candidates()), keys per query
+// of the filter's lists, and slices of a query's split at most.
+constexpr uint32_t kSplitCandidates = 64;
+constexpr uint32_t kSplitListKeys = 512;
+constexpr uint32_t kSplitSlices = 8;
+// Vectors to split (split_vectors_kernel): the source (source_pitch elements
+// apart; `columns` gathers, times `scales`), the rows' centre and scale, the
+// split parts; for rows their norms and roots, for queries the prepared
+// vectors (a pitch of a multiple of 4), the slices' squared norms
+// (kSplitSlices per query) and the per-query words to clear.
+struct SplitVectors {
+    const void* source;
+    uint64_t source_pitch;
+    uint64_t dim;
+    const uint32_t* columns;
+    const float* scales;
+    const float* centre;
+    float scale;
+    void* out;
+    uint64_t pitch;
+    uint64_t slice;
+    bool vector_loads;
+    float* norms;
+    float* roots;
+    float* prepared;
+    uint64_t prepared_pitch;
+    double* squares;
+    uint32_t* counts;
+    unsigned int* upper;
+    uint32_t* done;
+    int* error_flag;
+};
+uint32_t split_slices(uint64_t pitch, uint64_t batch);
+// Splits a batch of queries: dense or gathered binary32 ones (validated and
+// prepared on the way), or binary64 projected ones.
+void launch_split_queries(SplitVectors v, uint64_t batch, bool projected, cudaStream_t stream);
+// What the selection reads of the rows and the queries.
+struct SplitQuery {
+    const float* norms;      // rows
+    const float* roots;
+    const double* squares;   // queries: slices per query
+    uint32_t slices;
+    float rel;               // split_error_rel()
+    unsigned int* upper;     // per query: ordered bits of the smallest e + E (in
+                             // the filtered form without the query's own square)
+    uint32_t* counts;        // per query: rows listed
+};
+// The filtered keys: cap per query.
+struct SplitList {
+    unsigned long long* keys;
+    uint32_t cap;
+};
+SplitPlan split_plan(uint64_t pitch, int bn, uint64_t splits);
+SplitPlan plan_split(uint64_t rows, uint64_t pitch, uint64_t batch, int sm_count);
+// Plans the autotuner times: the heuristic plan first.
+std::vector<SplitPlan> split_candidates(uint64_t rows, uint64_t pitch, uint64_t batch,
+                                        int sm_count);
+// partials[split][q][row]: estimates of the centred q.r over the split's
+// columns. error_flag |= 8 when a pipeline wait ran out.
+void launch_split_scores(const SplitPlan& plan, const void* rows, uint64_t row_count,
+                         const void* queries, uint64_t batch, uint64_t pitch, float* partials,
+                         int* error_flag, int sm_count, cudaStream_t stream);
+float split_error_rel(const SplitPlan& plan, uint64_t row_count);
+// The split scan of a prepared batch: every row that can be a query's minimum
+// into its list (kSplitCandidates slots, sq.counts[q] filled, any order); error
+// bit kCandidateOverflow when a list overflows or a query's norm is not
+// covered. partials: splits x batch x rows.
+void launch_split_scan(const SplitPlan& plan, const void* rows, uint64_t row_count,
+                       const void* queries, uint64_t batch, uint64_t pitch, float* partials,
+                       const SplitQuery& sq, uint32_t* candidates, int* error_flag,
+                       int sm_count, cudaStream_t stream);
+// The same without the slab, where one split of few stages covers the columns
+// and the rows are at least kSplitFilterRows: some of the tiles give each query
+// a threshold, then only the keys below it are kept (keys: batch x
+// kSplitListKeys).
+constexpr uint64_t kSplitFilterRows = 8192;
+bool split_filter_applies(const SplitPlan& plan, uint64_t row_count);
+void launch_split_filter_scan(const SplitPlan& plan, const void* rows, uint64_t row_count,
+                              const void* queries, uint64_t batch, uint64_t pitch,
+                              const SplitQuery& sq, unsigned long long* keys,
+                              uint32_t* candidates, int* error_flag, int sm_count,
+                              cudaStream_t stream);
+// Certified argmin of each query over its listed candidates, from the original
+// binary32 rows (l2_sequential inputs; in.emulated: bound32, else bound64, both
+// of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
+uint32_t settle_depth(uint64_t padded_dim);
+uint64_t settle_sums(uint64_t batch);
+void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32_t* candidates,
+                   const uint32_t* counts, uint32_t batch, uint32_t rows, double* sums,
+                   uint32_t* done, Result* results, double* exact_distances,
+                   uint32_t* replay_count, cudaStream_t stream);
+
 // ---- hierarchical index (projection)
 // Binary64 projected rows reps[row][j] = sum_i double(sampled[row][i]) *
 // projection[j][i] in i order; `bad` is set when a result is not finite.
