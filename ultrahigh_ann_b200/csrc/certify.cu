@@ -18,6 +18,7 @@
 #include "exact64.h"
 #include "hier_body.cuh"
 #include "kernels.h"
+#include "median64.cuh"
 #include "stage_bodies.h"
 #include "tile_body.cuh"
 
@@ -326,49 +327,7 @@ __device__ double replay_projected_l2(const double* row, const double* y,
     return s;
 }
 
-// Number of j < p with |row_j - y_j| (as binary64 bits) below `bound`.
-__device__ uint32_t count_below(const double* row, const double* y, uint64_t p,
-                                unsigned long long bound, int lane)
-{
-    uint32_t c = 0;
-    for (uint64_t j = lane; j < p; j += 32) {
-        const unsigned long long bits = static_cast<unsigned long long>(
-            __double_as_longlong(fabs(__dsub_rn(row[j], y[j]))));
-        c += bits < bound ? 1u : 0u;
-    }
-    return __reduce_add_sync(0xffffffffu, c);
-}
-
-// The k-th smallest (0-based) |row_j - y_j|: binary search on the bit pattern
-// (nonnegative binary64 values order like their bits).
-__device__ double select_abs_diff(const double* row, const double* y,
-                                  uint64_t p, uint32_t k, int lane)
-{
-    unsigned long long prefix = 0;
-    for (int bit = 62; bit >= 0; --bit) {
-        const unsigned long long trial = prefix | (1ull << bit);
-        if (count_below(row, y, p, trial, lane) <= k) {
-            prefix = trial;
-        }
-    }
-    return __longlong_as_double(static_cast<long long>(prefix));
-}
-
-// Reference median of |r_j - y_j| with the even-p midpoint
-// (hierarchical_l1_ann_index.cpp:65-99): nth_element puts the (p/2)-th
-// smallest at the upper middle; the lower middle is the largest of the
-// smaller half; median = lower + (upper - lower) * 0.5.
-__device__ double replay_median(const double* row, const double* y, uint64_t p,
-                                int lane)
-{
-    const uint32_t mid = static_cast<uint32_t>(p / 2);
-    const double upper = select_abs_diff(row, y, p, mid, lane);
-    if (p % 2 != 0) {
-        return upper;
-    }
-    const double lower = select_abs_diff(row, y, p, mid - 1, lane);
-    return __dadd_rn(lower, __dmul_rn(__dsub_rn(upper, lower), 0.5));
-}
+using median64::replay_median;
 
 __device__ __forceinline__ bool lex_less(double a, uint32_t ar, double b,
                                          uint32_t br)
@@ -1095,19 +1054,19 @@ __global__ void __launch_bounds__(kFinalizeThreads)
 // replayed). One CTA per query: the binary64 projected query, then one warp
 // replays the selected row.
 __global__ void __launch_bounds__(kFinalizeThreads)
-    refine_kernel(ReplayInputs in, Bound bound, const Result* results,
+    refine_kernel(ReplayInputs in, Bound bound, float tolerance, const Result* results,
                   double* exact_distances)
 {
     const uint32_t q = blockIdx.x;
     // replayed by the argmin already, or the certified interval is within the
-    // 1e-5 relative tolerance: the binary32 distance stands
+    // relative tolerance: the binary32 distance stands
     const double known = exact_distances[q];
     if (known == known) {
         return;
     }
     const Result res = results[q];
     const Bounds2 b = bound_of(res.distance, bound, res.row, q);
-    if (__fsub_ru(b.upper, b.lower) <= __fmul_rd(0.999e-5f, b.lower)) {
+    if (__fsub_ru(b.upper, b.lower) <= __fmul_rd(tolerance, b.lower)) {
         return;
     }
     extern __shared__ double projected_query[];
@@ -1129,9 +1088,11 @@ __global__ void __launch_bounds__(kFinalizeThreads)
 // of the binary64 projection is read once for the group; each query's sum
 // keeps the reference order), then one warp per such query replays its row.
 constexpr int kRefineGroup = 8;
+// a certified binary32 distance this narrow (relative) is reported as it is
+constexpr float kRefineTolerance = 0.999e-5f;
 
 __device__ __forceinline__ void refine_group_block(const ReplayInputs& in, const Bound& bound,
-                                                   const Result* results,
+                                                   float tolerance, const Result* results,
                                                    double* exact_distances, uint32_t batch,
                                                    uint32_t bx, unsigned char* refine_smem)
 {
@@ -1153,7 +1114,7 @@ __device__ __forceinline__ void refine_group_block(const ReplayInputs& in, const
             }
             const Result res = results[q];
             const Bounds2 b = bound_of(res.distance, bound, res.row, q);
-            if (__fsub_ru(b.upper, b.lower) <= __fmul_rd(0.999e-5f, b.lower)) {
+            if (__fsub_ru(b.upper, b.lower) <= __fmul_rd(tolerance, b.lower)) {
                 continue;
             }
             members[c++] = q;
@@ -1210,11 +1171,11 @@ __device__ __forceinline__ void refine_group_block(const ReplayInputs& in, const
 }
 
 __global__ void __launch_bounds__(kFinalizeThreads)
-    refine_group_kernel(ReplayInputs in, Bound bound, const Result* results,
+    refine_group_kernel(ReplayInputs in, Bound bound, float tolerance, const Result* results,
                         double* exact_distances, uint32_t batch)
 {
     extern __shared__ unsigned char refine_group_smem[];
-    refine_group_block(in, bound, results, exact_distances, batch, blockIdx.x,
+    refine_group_block(in, bound, tolerance, results, exact_distances, batch, blockIdx.x,
                        refine_group_smem);
 }
 
@@ -2449,7 +2410,8 @@ __device__ void persistent_unit(const PersistentPair& d, uint32_t kind, uint32_t
         break;
     }
     case kUnitRefine: {
-        refine_group_block(d.replay, d.bound, d.results, d.exact_distances, d.batch, u, smem);
+        refine_group_block(d.replay, d.bound, kRefineTolerance, d.results, d.exact_distances,
+                           d.batch, u, smem);
         break;
     }
     default:
@@ -2630,20 +2592,22 @@ FinalizeScratch finalize_scratch(void* base, uint32_t capacity, uint32_t rows)
 
 void launch_refine_winners(ReplayInputs in, Bound bound, const Result* results,
                            uint32_t batch, double* exact_distances,
-                           cudaStream_t stream)
+                           cudaStream_t stream, bool every)
 {
+    // every: no interval is narrow enough
+    const float tolerance = every ? -1.f : kRefineTolerance;
     static_assert(kRefineGroup <= kFinalizeThreads / 32, "one warp per group member");
     const size_t group_smem =
         kRefineGroup * (in.proj_dim * sizeof(double) + in.dim * sizeof(float));
     if (group_smem <= 200 * 1024) {
         set_dynamic_smem(reinterpret_cast<const void*>(refine_group_kernel), group_smem);
         refine_group_kernel<<<(batch + kRefineGroup - 1) / kRefineGroup, kFinalizeThreads,
-                              group_smem, stream>>>(in, bound, results, exact_distances,
-                                                    batch);
+                              group_smem, stream>>>(in, bound, tolerance, results,
+                                                    exact_distances, batch);
     } else {
         const size_t smem = replay_smem(in);
         set_dynamic_smem(reinterpret_cast<const void*>(refine_kernel), smem);
-        refine_kernel<<<batch, kFinalizeThreads, smem, stream>>>(in, bound, results,
+        refine_kernel<<<batch, kFinalizeThreads, smem, stream>>>(in, bound, tolerance, results,
                                                                  exact_distances);
     }
     check_cuda(cudaGetLastError(), "cannot launch refine kernel");

@@ -784,15 +784,15 @@ void create_hierarchical_index(int device, uha_metric metric, const RowSource& s
     }
     const uint64_t f = sizeof(float);
     const uint64_t column_bytes = 2 * sizeof(uint64_t) + sizeof(double);
-    if (metric == UHA_L2) {
-        // the precision strategies' binary64 query projection reads it
-        std::vector<double> proj_t(p * k);
-        for (uint64_t j = 0; j < p; ++j) {
-            for (uint64_t i = 0; i < k; ++i) {
-                proj_t[i * p + j] = projection[j * k + i];
-            }
+    // the binary64 query projections read it
+    std::vector<double> proj_t(p * k);
+    for (uint64_t j = 0; j < p; ++j) {
+        for (uint64_t i = 0; i < k; ++i) {
+            proj_t[i * p + j] = projection[j * k + i];
         }
-        upload(index->projection64_t, proj_t.data(), proj_t.size());
+    }
+    upload(index->projection64_t, proj_t.data(), proj_t.size());
+    if (metric == UHA_L2) {
         compute_row_norms(*index);
         index->usage.index_payload_bytes = row_count * p * f + row_count * f +
                                            k * column_bytes + p * k * f;
@@ -1386,7 +1386,10 @@ const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
     }
     // the word past the roots receives the largest of them
     unsigned int* largest = reinterpret_cast<unsigned int*>(sp.roots.get() + index->rows);
-    check_cuda(cudaMemsetAsync(sp.data.get(), 0, bytes, stream), "cannot clear split rows");
+    // the split writes every row's whole pitch; the vectors past the rows are zero
+    const uint64_t used = index->rows * sp.pitch * 4;
+    check_cuda(cudaMemsetAsync(sp.data.get() + used, 0, bytes - used, stream),
+               "cannot clear split rows");
     auto split = [&] {
         if (hierarchical) {
             uha::launch_split_rows(index->rows64.get(), index->rows, index->scan_dim,
@@ -1416,6 +1419,109 @@ const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
         sp.data.release();
     }
     return sp.usable ? &sp : nullptr;
+}
+
+// The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use on
+// `stream` and synchronised before they are published; null when the index
+// keeps the binary32 passes.
+const uha::RowBits* row_bits(const uha_index* index, cudaStream_t stream)
+{
+    std::lock_guard<std::mutex> lock(index->lowp_mutex);
+    uha::RowBits& rb = index->bits;
+    if (!rb.ready) {
+        const uint64_t p = index->projection_dimension;
+        rb.ready = true;
+        rb.usable = rb.boundaries.try_allocate(uha::bits_boundaries(p)) &&
+                    rb.data.try_allocate(uha::bits_bytes(index->rows, p));
+        if (rb.usable) {
+            uha::launch_row_bits(index->scan_rows.get(), index->rows, index->padded_dim, p,
+                                 rb.boundaries.get(), rb.data.get(), stream);
+            check_cuda(cudaStreamSynchronize(stream), "cannot build row bitmaps");
+        } else {
+            rb.boundaries.release();
+        }
+    }
+    return rb.usable ? &rb : nullptr;
+}
+
+// The bitmap form of this batch's median scan (everything it needs allocated
+// here), or null when it takes the binary32 passes.
+const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+        index->kind != IndexKind::hierarchical || index->metric != UHA_L1 ||
+        !uha::bits_applies(index->rows, index->projection_dimension) ||
+        !uha::bits_batch(index->projection_dimension, n)) {
+        return nullptr;
+    }
+    const uha::RowBits* bits = row_bits(index, ws->stream);
+    if (bits == nullptr) {
+        return nullptr;
+    }
+    auto grow = [&](auto& buffer, uint64_t count) {
+        if (buffer.size() >= count) {
+            return true;
+        }
+        check_cuda(cudaStreamSynchronize(ws->stream), "CUDA query failed");
+        return buffer.try_allocate(count);
+    };
+    const uint64_t b = ws->max_batch;
+    const uint64_t list = checked_mul(b, uha::kBitsList, "row lists");
+    if (!grow(ws->median_min, std::max(n, b)) || !grow(ws->split_words, 3 * b) ||
+        !grow(ws->projected64, checked_mul(b, index->projection_dimension, "queries")) ||
+        !grow(ws->bits_offsets, uha::bits_offsets(b, index->projection_dimension)) ||
+        !grow(ws->bits_listed, list) || !grow(ws->bits_medians, list)) {
+        ws->split_disabled = true;
+        return nullptr;
+    }
+    return bits;
+}
+
+// One batch by the bitmap median scan.
+uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, const float* source,
+                            uint64_t n, uha::Result* results, double* exact, bool time_scan,
+                            cudaEvent_t scan_start, cudaEvent_t scan_stop)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    cudaStream_t stream = ws->stream;
+    int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
+    const uint64_t p = index->projection_dimension;
+    uha::launch_gather_project64(source, n, index->dimension, index->columns.get(),
+                                 index->sample_size, index->projection64_t.get(), p,
+                                 ws->projected64.get(), ws->projected.get(), index->padded_dim,
+                                 ws->coord_err.get(), ws->query_err.get(), error_flag, stream);
+    uha::BitsScan s{};
+    s.rows = index->scan_rows.get();
+    s.row_count = index->rows;
+    s.padded_p = index->padded_dim;
+    s.p = p;
+    s.rows64 = index->rows64.get();
+    s.boundaries = bits.boundaries.get();
+    s.bits = bits.data.get();
+    s.queries = ws->projected.get();
+    s.y64 = ws->projected64.get();
+    s.query_err = ws->query_err.get();
+    s.coord_err = ws->coord_err.get();
+    s.row_err_max = index->row_err_max;
+    s.rel = kMedianRel;
+    s.abs_err = kMedianAbs;
+    s.min_bits = ws->median_min.get();
+    s.counts = ws->split_words.get();
+    s.offsets = ws->bits_offsets.get();
+    s.listed = ws->bits_listed.get();
+    s.medians = ws->bits_medians.get();
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_start, stream), "event");
+    }
+    const uint64_t launches = uha::launch_bits_scan(s, n, results, exact, ws->counters.get(),
+                                                    error_flag, stream);
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_stop, stream), "event");
+    }
+    return 1 + launches;
 }
 
 // The split scan of this batch, or false when it takes the binary32 scan: the
@@ -1661,15 +1767,13 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     uint64_t launches = 1;
     if (hierarchical) {
         const uint64_t p = index->projection_dimension;
-        uha::launch_prepare_sampled(source, n, index->dimension, index->columns.get(), nullptr,
-                                    index->sample_size, ws->prepared.get(),
-                                    index->padded_sample, error_flag, stream);
-        uha::launch_project_queries64(ws->prepared.get(), n, index->padded_sample,
-                                      index->sample_size, index->projection64_t.get(), p,
-                                      ws->projected64.get(), error_flag, stream);
+        uha::launch_gather_project64(source, n, index->dimension, index->columns.get(),
+                                     index->sample_size, index->projection64_t.get(), p,
+                                     ws->projected64.get(), nullptr, index->padded_dim, nullptr,
+                                     nullptr, error_flag, stream);
         v.source = ws->projected64.get();
         v.source_pitch = p;
-        launches += 2;
+        ++launches;
     }
     uha::launch_split_queries(v, n, hierarchical, stream);
     const uha::SplitQuery sq{rows.norms.get(),
@@ -1799,6 +1903,10 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     if (split_applies(c, n, &split, &split_plan)) {
         return enqueue_split_batch(c, *split, split_plan, source, n, results, exact, time_scan,
                                    scan_start, scan_stop);
+    }
+    if (const uha::RowBits* bits = bits_scan_applies(c, n); bits != nullptr) {
+        return enqueue_bits_batch(c, *bits, source, n, results, exact, time_scan, scan_start,
+                                  scan_stop);
     }
     float* prepared = c.prepared != nullptr ? c.prepared : ws->prepared.get();
     const float* scan_queries = prepared;
@@ -1968,9 +2076,10 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     ++launches;
     if (hierarchical && c.want_distances) {
         // reported distances of a hierarchy: the reference's binary64 value of
-        // each selected row
+        // each selected row (a call answered again reports them all, like the
+        // listing scans it stands in for)
         uha::launch_refine_winners(in, bound, results, static_cast<uint32_t>(n), exact,
-                                   stream);
+                                   stream, ws->filter_disabled);
         ++launches;
     }
     return launches;
@@ -1997,7 +2106,7 @@ void finish_call(const uha_index* index, uha_workspace* ws, uint64_t n,
         fail(UHA_RUNTIME_ERROR, "tensor-core pipeline wait timed out");
     }
     if (flag & 16u) {
-        fail(UHA_RUNTIME_ERROR, "flat query row copy wait timed out");
+        fail(UHA_RUNTIME_ERROR, "row copy wait timed out");
     }
     if (flag & static_cast<uint32_t>(uha::kCandidateOverflow)) {
         fail(UHA_RUNTIME_ERROR, "filtered candidate list overflowed");

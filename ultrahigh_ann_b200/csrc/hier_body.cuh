@@ -302,18 +302,24 @@ __device__ __forceinline__ void median_sample_loop(
 // <= T (odd p), fewer than p/2 (even p: the lower middle is above T). Such a
 // row stores -T (a negative distance: "at least T, no upper bound"); every
 // other row gets its binary32 median in stage 3.
+__device__ __forceinline__ float threshold_of(unsigned int min_bits, float query_err,
+                                              float row_err_max, float rel, float abs_err)
+{
+    const float u = __uint_as_float(min_bits);
+    if (!(u <= FLT_MAX)) {
+        return __int_as_float(0x7f800000);
+    }
+    const float e = __fadd_ru(row_err_max, query_err);
+    const float num = __fadd_ru(__fadd_ru(__fmul_ru(u, __fadd_ru(1.f, rel)), __fmul_ru(2.f, e)),
+                                __fmul_ru(2.f, abs_err));
+    return __fmul_ru(__fdiv_ru(num, __fsub_rd(1.f, rel)), 1.0000005f);
+}
+
 __device__ __forceinline__ float median_threshold(const unsigned int* min_bits,
                                                   const float* query_err, uint32_t q,
                                                   float row_err_max, float rel, float abs_err)
 {
-    const float u = __uint_as_float(min_bits[q]);
-    if (!(u <= FLT_MAX)) {
-        return __int_as_float(0x7f800000);
-    }
-    const float e = __fadd_ru(row_err_max, query_err[q]);
-    const float num = __fadd_ru(__fadd_ru(__fmul_ru(u, __fadd_ru(1.f, rel)), __fmul_ru(2.f, e)),
-                                __fmul_ru(2.f, abs_err));
-    return __fmul_ru(__fdiv_ru(num, __fsub_rd(1.f, rel)), 1.0000005f);
+    return threshold_of(min_bits[q], query_err[q], row_err_max, rel, abs_err);
 }
 
 // The stage-2 count over the transposed rows (rows_t[j][row], row pitch

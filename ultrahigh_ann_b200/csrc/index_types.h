@@ -45,6 +45,15 @@ struct SplitRows {
     bool usable = false;
 };
 
+// The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use;
+// `usable` is false when the memory for them was not available.
+struct RowBits {
+    DeviceBuffer<unsigned char> data;
+    DeviceBuffer<float> boundaries;
+    bool ready = false;
+    bool usable = false;
+};
+
 // Relative and absolute certification bound for a binary32 distance (defined
 // in engine.cu).
 Bound make_bound(uint32_t depth, uint64_t terms, int term_roundings);
@@ -83,7 +92,7 @@ struct uha_index {
     // L1 hierarchy: scan_rows transposed, padded_dim x rows_pitch
     uha::DeviceBuffer<float> scan_rows_t;
     uint64_t rows_pitch = 0;
-    // L2 hierarchy: projection64 transposed, sample_size x p
+    // projection64 transposed, sample_size x p
     uha::DeviceBuffer<double> projection64_t;
     uha_space_usage usage{};
     // precision strategies: built on first use (index_bf16 / index_fp8)
@@ -91,6 +100,7 @@ struct uha_index {
     mutable uha::LowpRows lowp[2];
     mutable uha::LowpRows lowp_projection[2];  // L2 hierarchy: the p x k projection
     mutable uha::SplitRows split;
+    mutable uha::RowBits bits;  // L1 hierarchy
 };
 
 // A scan shape chosen by the autotuner for one (batch size, strategy) of a
@@ -149,7 +159,7 @@ struct uha_workspace {
     // squared norms, partial estimates, per-query words (listed rows, smallest
     // e + E, finished settlement blocks), candidate lists, the filter's
     // keys, settlement sums. split_disabled: this workspace keeps the
-    // binary32 scan (persistent batches; no memory for these).
+    // binary32 scans (persistent batches; no memory for these or the bitmaps').
     uha::DeviceBuffer<unsigned char> split_queries;
     uha::DeviceBuffer<double> split_squares;
     uha::DeviceBuffer<float> split_partials;
@@ -158,6 +168,11 @@ struct uha_workspace {
     uha::DeviceBuffer<unsigned long long> split_keys;
     uha::DeviceBuffer<double> split_sums;
     bool split_disabled = false;
+    // median scan by bitmaps (allocated on first use): intervals, listed rows
+    // and their medians; the per-query words are median_min and split_words
+    uha::DeviceBuffer<uint32_t> bits_offsets;
+    uha::DeviceBuffer<uint32_t> bits_listed;
+    uha::DeviceBuffer<float2> bits_medians;
     uha::DeviceBuffer<uint32_t> candidates;       // [batch][candidates_per_query]
     uha::DeviceBuffer<double> cand_dist;          // [batch][candidates_per_query]
     uha::DeviceBuffer<uint32_t> rescore_done;     // per query, zero between calls

@@ -203,10 +203,11 @@ void launch_finalize_gemm(PartialView view, const float* row_norms,
 
 // Reference binary64 distance of each query's selected row (projected replay
 // ops only), for the queries that the argmin did not replay and whose
-// certified interval is wider than 1e-5 relative.
+// certified interval is wider than 1e-5 relative; with `every`, for all that it
+// did not replay.
 void launch_refine_winners(ReplayInputs in, Bound bound, const Result* results,
                            uint32_t batch, double* exact_distances,
-                           cudaStream_t stream);
+                           cudaStream_t stream, bool every = false);
 
 // ---- precision form: low-precision scores on the tensor cores, top-k,
 // binary32 re-score of the candidates
@@ -520,6 +521,61 @@ void launch_median_tuning_queries(const float* rows, uint64_t row_count, uint64_
 // out[j][row] = rows[row][j] for j < padded_p (build time).
 void launch_transpose_rows(const float* rows, uint64_t row_count, uint64_t padded_p,
                            float* out, uint64_t r_pitch, cudaStream_t stream);
+
+// ---- the median scan by row bitmaps (median_bits.cu)
+// Gathers a batch's sampled coordinates (error_flag |= 1 for a non-finite one)
+// and projects them in the reference's binary64 order: y64, batch x p
+// (error_flag |= 4 for a non-finite result). y32 (nullable): the binary32
+// roundings, batch x padded_p, with their error per coordinate and per query
+// (error bit kCandidateOverflow when one is past binary32).
+void launch_gather_project64(const float* queries, uint64_t batch, uint64_t dim,
+                             const uint32_t* columns, uint64_t k, const double* proj_t,
+                             uint64_t p, double* y64, float* y32, uint64_t padded_p,
+                             float* coord_err, float* query_err, int* error_flag,
+                             cudaStream_t stream);
+// Indexes with a bitmap form, its size, and its construction from the scanned
+// binary32 rows (boundaries: bits_boundaries(p) floats).
+constexpr uint64_t kBitsRows = 1024;
+// rows listed per query at most, and spread rows of the first threshold
+constexpr uint32_t kBitsList = 1024;
+constexpr uint32_t kBitsSpread = 32;
+bool bits_applies(uint64_t rows, uint64_t p);
+// Batches that the bitmaps answer faster than the binary32 passes.
+bool bits_batch(uint64_t p, uint64_t batch);
+uint32_t bits_columns(uint64_t p);
+uint64_t bits_bytes(uint64_t rows, uint64_t p);
+uint64_t bits_boundaries(uint64_t p);
+uint64_t bits_offsets(uint64_t batch, uint64_t p);
+void launch_row_bits(const float* rows, uint64_t row_count, uint64_t padded_p, uint64_t p,
+                     float* boundaries, void* bits, cudaStream_t stream);
+// Certified argmin of a projected batch; results and exact distances are the
+// reference's. Error bit kCandidateOverflow: answer the call again by the
+// binary32 passes. offsets: bits_offsets(batch, p); listed, medians: batch x
+// kBitsList; min_bits, counts: batch. Returns the kernel launches.
+struct BitsScan {
+    const float* rows;
+    uint64_t row_count;
+    uint64_t padded_p;
+    uint64_t p;
+    const double* rows64;
+    const float* boundaries;
+    const void* bits;
+    const float* queries;
+    const double* y64;
+    const float* query_err;
+    const float* coord_err;
+    float row_err_max;
+    float rel;
+    float abs_err;
+    unsigned int* min_bits;
+    uint32_t* counts;
+    uint32_t* offsets;
+    uint32_t* listed;
+    float2* medians;
+};
+uint64_t launch_bits_scan(const BitsScan& s, uint64_t batch, Result* results,
+                          double* exact_distances, uint32_t* replay_count, int* error_flag,
+                          cudaStream_t stream);
 
 // ---- build-time helpers
 void launch_gather_rows(const float* source, uint64_t row_count, uint64_t dim,

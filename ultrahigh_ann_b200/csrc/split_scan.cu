@@ -67,6 +67,9 @@ using namespace tensorcore;
 constexpr uint32_t kStageColumns = 64;  // one 128-byte swizzle row of BF16
 constexpr int kPrepThreads = 512;
 constexpr int kSelectThreads = 256;
+// rows whose mean is the centre: more do not bring the norms down further, and the
+// kernel's time (one thread per column) is theirs
+constexpr uint64_t kCentreRows = 128;
 constexpr float kLargestNorm = 0x1p40f;
 // rows per thread of the selection kernels, their loads in flight together
 constexpr int kSelectRows = 8;
@@ -949,7 +952,7 @@ void split_rows_typed(const T* rows, uint64_t row_count, uint64_t src_pitch, uin
                       void* out, uint64_t pitch, float scale, float* centre, float* norms,
                       float* roots, unsigned int* largest, cudaStream_t stream)
 {
-    const uint32_t take = static_cast<uint32_t>(std::min<uint64_t>(row_count, 512));
+    const uint32_t take = static_cast<uint32_t>(std::min<uint64_t>(row_count, kCentreRows));
     column_centre_kernel<<<static_cast<uint32_t>((pitch + 255) / 256), 256, 0, stream>>>(
         rows, row_count, src_pitch, dim, take, centre, pitch);
     SplitVectors v{};
