@@ -103,6 +103,7 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
     }
     DeviceGuard guard(index->device);
     cudaStream_t stream = ws->stream;
+    ws->counters_clear = false;  // the timed launches may set the error word
     TunedPlan best{};
     best.batch = batch;
     best.strategy = static_cast<int>(strategy);
@@ -408,6 +409,7 @@ namespace {
 uint64_t enqueue_pair(uha_batch::Pair& p)
 {
     uha_workspace* ws = p.ws;
+    ws->counters_clear = false;
     check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), ws->stream),
                "cannot clear query counters");
     BatchContext ctx{p.index, ws, p.strategy, true};

@@ -43,6 +43,24 @@ void require(bool condition, uha_status status, const char* message)
     }
 }
 
+// Properties of a device, queried once per device and process (they do not
+// change, and cudaGetDeviceProperties takes 2.5 ms a call).
+const cudaDeviceProp& device_properties(int device)
+{
+    static std::mutex lock;
+    static std::unique_ptr<cudaDeviceProp> known[uha::kMaxDevices];
+    require(device >= 0 && device < uha::kMaxDevices, UHA_RUNTIME_ERROR,
+            "device ordinal out of supported range");
+    std::lock_guard<std::mutex> guard(lock);
+    if (known[device] == nullptr) {
+        auto fresh = std::make_unique<cudaDeviceProp>();
+        check_cuda(cudaGetDeviceProperties(fresh.get(), device),
+                   "cannot query CUDA device properties");
+        known[device] = std::move(fresh);
+    }
+    return *known[device];
+}
+
 void select_device(uha_index& index, int device)
 {
     uha::clear_stale_cuda_error();
@@ -53,9 +71,7 @@ void select_device(uha_index& index, int device)
     }
     require(device >= 0 && device < count, UHA_INVALID_ARGUMENT,
             "CUDA device index is out of range");
-    cudaDeviceProp prop{};
-    check_cuda(cudaGetDeviceProperties(&prop, device),
-               "cannot query CUDA device properties");
+    const cudaDeviceProp& prop = device_properties(device);
     index.device = device;
     index.device_name = prop.name;
     index.sm_count = prop.multiProcessorCount;
@@ -178,6 +194,18 @@ void upload_weights_ff(uha_index& index, const std::vector<double>& w64)
     upload(index.weights_ff, ff.data(), ff.size());
 }
 
+// The sampled columns, and the same for queries that arrive gathered.
+void upload_columns(uha_index& index, const std::vector<uint32_t>& columns)
+{
+    upload(index.columns, columns.data(), columns.size());
+    std::vector<uint32_t> identity(columns.size());
+    for (size_t i = 0; i < identity.size(); ++i) {
+        identity[i] = static_cast<uint32_t>(i);
+    }
+    upload(index.gathered_columns, identity.data(), identity.size());
+    index.host_columns = columns;
+}
+
 void compute_row_norms(uha_index& index)
 {
     index.row_norms.allocate(index.rows);
@@ -289,9 +317,7 @@ extern "C" uha_status uha_device_info_get(int device, uha_device_info* out)
             cudaGetLastError();
             fail(UHA_RUNTIME_ERROR, "no usable CUDA device");
         }
-        cudaDeviceProp prop{};
-        check_cuda(cudaGetDeviceProperties(&prop, device),
-                   "cannot query CUDA device properties");
+        const cudaDeviceProp& prop = device_properties(device);
         std::memset(out, 0, sizeof(*out));
         out->device = device;
         std::strncpy(out->device_name, prop.name, sizeof(out->device_name) - 1);
@@ -543,7 +569,7 @@ void create_sampled_index(int device, uha_metric metric, const RowSource& src,
     index->sample_size = sample_size;
     index->sampled_multiplicity = multiplicity_sum;
     index->padded_dim = uha::round_up(sample_size, kColumnAlign);
-    upload(index->columns, cols.data(), cols.size());
+    upload_columns(*index, cols);
     if (metric == UHA_L2) {
         upload(index->scales, scales.data(), scales.size());
     } else {
@@ -726,7 +752,7 @@ void create_hierarchical_index(int device, uha_metric metric, const RowSource& s
     index->projection_dimension = p;
     index->scan_dim = p;
     index->padded_dim = pp;
-    upload(index->columns, cols.data(), cols.size());
+    upload_columns(*index, cols);
     upload(index->projection64, projection, p * k);
     upload(index->projection32, proj32.data(), proj32.size());
 
@@ -933,6 +959,10 @@ extern "C" uha_status uha_workspace_create(const uha_index* index,
         ws->host_results.allocate(b);
         ws->host_exact.allocate(b);
         ws->host_counters.allocate(2);
+        if (index->sample_size != 0 && index->sample_size * b <= 65536) {
+            // small enough to have it ready for the first host queries
+            ws->host_gathered.allocate(index->sample_size * b);
+        }
         for (cudaEvent_t& e : ws->events) {
             check_cuda(cudaEventCreate(&e), "cannot create CUDA event");
         }
@@ -1030,6 +1060,18 @@ bool precision_strategy(uha_strategy s)
 bool fp32_rescore_strategy(uha_strategy s)
 {
     return s == UHA_GEMM_BF16_RERANK_FP32 || s == UHA_GEMM_FP8_RERANK_FP32;
+}
+
+// Length and sampled columns of the query vectors a batch reads: the caller's, or
+// the sampled values alone.
+uint64_t query_dimension(const BatchContext& c)
+{
+    return c.gathered ? c.index->sample_size : c.index->dimension;
+}
+
+const uint32_t* query_columns(const BatchContext& c)
+{
+    return c.gathered ? c.index->gathered_columns.get() : c.index->columns.get();
 }
 
 // Replay inputs of the emulated (FP64-free) replay of exact and flat ops.
@@ -1489,7 +1531,7 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
     cudaStream_t stream = ws->stream;
     int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
     const uint64_t p = index->projection_dimension;
-    uha::launch_gather_project64(source, n, index->dimension, index->columns.get(),
+    uha::launch_gather_project64(source, n, query_dimension(c), query_columns(c),
                                  index->sample_size, index->projection64_t.get(), p,
                                  ws->projected64.get(), ws->projected.get(), index->padded_dim,
                                  ws->coord_err.get(), ws->query_err.get(), error_flag, stream);
@@ -1749,9 +1791,9 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     uint32_t* words = ws->split_words.get();
     uha::SplitVectors v{};
     v.source = source;
-    v.source_pitch = index->dimension;
+    v.source_pitch = query_dimension(c);
     v.dim = index->scan_dim;
-    v.columns = index->columns.get();
+    v.columns = query_columns(c);
     v.scales = index->scales.get();
     v.centre = rows.centre.get();
     v.scale = rows.scale;
@@ -1767,7 +1809,7 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     uint64_t launches = 1;
     if (hierarchical) {
         const uint64_t p = index->projection_dimension;
-        uha::launch_gather_project64(source, n, index->dimension, index->columns.get(),
+        uha::launch_gather_project64(source, n, query_dimension(c), query_columns(c),
                                      index->sample_size, index->projection64_t.get(), p,
                                      ws->projected64.get(), nullptr, index->padded_dim, nullptr,
                                      nullptr, error_flag, stream);
@@ -1843,8 +1885,8 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     if (small_path_applies(index, c.strategy) || flat) {
         uha::SmallQuery sq{};
         sq.queries = source;
-        sq.dim = index->dimension;
-        sq.columns = index->kind == IndexKind::sampled ? index->columns.get() : nullptr;
+        sq.dim = query_dimension(c);
+        sq.columns = index->kind == IndexKind::sampled ? query_columns(c) : nullptr;
         sq.scales = index->kind == IndexKind::sampled && index->metric == UHA_L2
                         ? index->scales.get()
                         : nullptr;
@@ -1911,14 +1953,14 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     float* prepared = c.prepared != nullptr ? c.prepared : ws->prepared.get();
     const float* scan_queries = prepared;
     if (hierarchical && precision_strategy(c.strategy)) {
-        uha::launch_prepare_sampled(source, n, index->dimension, index->columns.get(),
+        uha::launch_prepare_sampled(source, n, query_dimension(c), query_columns(c),
                                     nullptr, index->sample_size, ws->prepared.get(),
                                     index->padded_sample, error_flag, stream);
         enqueue_hierarchical_projection(index, ws, c.strategy, n, error_flag, stream);
         scan_queries = ws->projected.get();
         launches += 6;
     } else if (hierarchical) {
-        uha::launch_prepare_sampled(source, n, index->dimension, index->columns.get(),
+        uha::launch_prepare_sampled(source, n, query_dimension(c), query_columns(c),
                                     nullptr, index->sample_size, ws->prepared.get(),
                                     index->padded_sample, error_flag, stream);
         uha::launch_project_queries(
@@ -1932,7 +1974,7 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
         launches += 3;
     } else if (index->kind == IndexKind::sampled) {
         uha::launch_prepare_sampled(
-            source, n, index->dimension, index->columns.get(),
+            source, n, query_dimension(c), query_columns(c),
             index->metric == UHA_L2 ? index->scales.get() : nullptr,
             index->sample_size, prepared, index->padded_dim, error_flag, stream);
         ++launches;
@@ -2231,6 +2273,35 @@ void prepare_pipeline(const uha_index* index, uha_workspace* ws, uha_strategy st
     check_cuda(cudaStreamWaitEvent(ws->finish_stream, ws->pipe_events[4], 0), "event");
 }
 
+// Host queries of an index that reads few of their columns are gathered on the
+// host: only the sampled values cross PCIe (49 of 60,660 for 33 centroids at
+// T = 8, where the copy of the whole vector was half of a 60 us call). Past an
+// eighth of the columns the scattered reads cost as much as the copy, and past
+// kGatherBytes the pinned staging would outgrow its use.
+constexpr uint64_t kGatherBytes = 64ull << 20;
+
+bool gather_on_host(const uha_index* index, uint64_t n)
+{
+    return index->sample_size != 0 && index->sample_size * 8 <= index->dimension &&
+           n <= kGatherBytes / (index->sample_size * sizeof(float));
+}
+
+void gather_queries(const uha_index* index, uha_workspace* ws, const float* queries, uint64_t n)
+{
+    const uint64_t k = index->sample_size;
+    if (ws->host_gathered.size() < n * k) {
+        ws->host_gathered.allocate(n * k);
+    }
+    const uint32_t* columns = index->host_columns.data();
+    for (uint64_t q = 0; q < n; ++q) {
+        const float* from = queries + q * index->dimension;
+        float* to = ws->host_gathered.get() + q * k;
+        for (uint64_t i = 0; i < k; ++i) {
+            to[i] = from[columns[i]];
+        }
+    }
+}
+
 // Event pairs for timing the scan of every batch of a call.
 void ensure_scan_events(uha_workspace* ws, uint64_t batches)
 {
@@ -2296,10 +2367,18 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
             ensure_scan_events(ws, batches);
             check_cuda(cudaEventRecord(ws->events[0], stream), "event");
         }
-        check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), stream),
-                   "cannot clear query counters");
+        // clear since the last call's delivery, unless something else used them
+        if (!ws->counters_clear) {
+            check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), stream),
+                       "cannot clear query counters");
+        }
+        ws->counters_clear = false;
         BatchContext ctx{index, ws, strategy, out_distances != nullptr};
         ctx.filter_candidates = true;
+        ctx.gathered = !queries_on_device && gather_on_host(index, n);
+        if (ctx.gathered) {
+            gather_queries(index, ws, queries, n);
+        }
         const bool pipelined = pipeline_applies(index, strategy, batch, batches);
         if (pipelined) {
             prepare_pipeline(index, ws, strategy, batch);
@@ -2359,8 +2438,12 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
                 bc.handoff = ws->pipe_events[slot];
             }
             if (!queries_on_device) {
+                const uint64_t length = query_dimension(ctx);
+                if (ctx.gathered) {
+                    source = ws->host_gathered.get() + start * length;
+                }
                 check_cuda(cudaMemcpyAsync(ws->raw_queries.get(), source,
-                                           count * index->dimension * sizeof(float),
+                                           count * length * sizeof(float),
                                            cudaMemcpyHostToDevice, stream),
                            "cannot copy queries to the CUDA device");
                 source = ws->raw_queries.get();
@@ -2384,20 +2467,14 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
             check_cuda(cudaEventRecord(ws->flat_events[i], ws->flat_streams[i]), "event");
             check_cuda(cudaStreamWaitEvent(stream, ws->flat_events[i], 0), "event");
         }
-        check_cuda(cudaMemcpyAsync(ws->host_results.get(), ws->call_results.get(),
-                                   n * sizeof(uha::Result), cudaMemcpyDeviceToHost,
-                                   stream),
-                   "cannot copy query results from the CUDA device");
-        check_cuda(cudaMemcpyAsync(ws->host_exact.get(), ws->call_exact.get(),
-                                   n * sizeof(double), cudaMemcpyDeviceToHost, stream),
-                   "cannot copy query distances from the CUDA device");
-        check_cuda(cudaMemcpyAsync(ws->host_counters.get(), ws->counters.get(),
-                                   ws->counters.bytes(), cudaMemcpyDeviceToHost, stream),
-                   "cannot copy query counters from the CUDA device");
+        uha::launch_deliver(ws->call_results.get(), ws->call_exact.get(), ws->counters.get(), n,
+                            ws->host_results.get(), ws->host_exact.get(),
+                            ws->host_counters.get(), stream);
         if (ws->timing) {
             check_cuda(cudaEventRecord(ws->events[3], stream), "event");
         }
         check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
+        ws->counters_clear = true;
         if (ws->timing) {
             float ms = 0.f;
             double scan = 0.0;
@@ -2477,6 +2554,7 @@ extern "C" uha_status uha_precision_scores(const uha_index* index, uha_workspace
         uha::clear_stale_cuda_error();
         cudaStream_t stream = ws->stream;
         const uint64_t n = query_count;
+        ws->counters_clear = false;
         check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), stream),
                    "cannot clear query counters");
         check_cuda(cudaMemcpyAsync(ws->raw_queries.get(), queries,

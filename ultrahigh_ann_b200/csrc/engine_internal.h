@@ -53,6 +53,8 @@ struct BatchContext {
     // them (ws->filter_disabled) when a candidate list overflows (error bit
     // uha::kCandidateOverflow).
     bool filter_candidates = false;
+    // The batch's queries hold the sampled values alone (gathered on the host).
+    bool gathered = false;
     // The fused flat query of this batch runs on stream lane `flat_lane`
     // (0: ws->stream; others: ws->flat_streams, forked and joined by the
     // caller) with that lane's scratch slots.

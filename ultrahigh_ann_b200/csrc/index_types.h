@@ -80,6 +80,8 @@ struct uha_index {
     uha::DeviceBuffer<double> weights64;  // scan_dim (weighted L1 replay)
     uha::DeviceBuffer<float> weights_ff;  // 2 x scan_dim: weights64 as hi, lo
     uha::DeviceBuffer<uint32_t> columns;  // sample_size (sampled)
+    uha::DeviceBuffer<uint32_t> gathered_columns;  // 0 .. sample_size - 1
+    std::vector<uint32_t> host_columns;            // columns, for host queries
     uha::DeviceBuffer<float> scales;      // sample_size (sampled L2)
     // hierarchical: scan_dim = p; scan_rows = binary32 projected rows
     uint64_t projection_dimension = 0;
@@ -134,6 +136,7 @@ struct uha_workspace {
     uha::DeviceBuffer<uha::Result> call_results;  // one call's answers
     uha::DeviceBuffer<double> call_exact;         // replayed distances (NaN: none)
     uha::DeviceBuffer<uint32_t> counters;  // [0] replayed queries, [1] error flag
+    bool counters_clear = false;  // the last use left the counters at zero
     uha::DeviceBuffer<unsigned char> finalize_scratch;
     // fused flat query (allocated and zeroed on first use): two scratch slots
     // per stream lane (uha::kFlatLanes lanes; lane 0 is `stream`), the slot
@@ -198,6 +201,7 @@ struct uha_workspace {
         }
         return nullptr;
     }
+    uha::PinnedBuffer<float> host_gathered;  // sampled values of host queries
     uha::PinnedBuffer<uha::Result> host_results;
     uha::PinnedBuffer<double> host_exact;
     uha::PinnedBuffer<uint32_t> host_counters;

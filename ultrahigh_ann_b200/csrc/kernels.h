@@ -77,6 +77,11 @@ void launch_prepare_sampled(const float* queries, uint64_t batch, uint64_t dim,
 // one contiguous batch).
 void launch_gather_vectors(const float* const* sources, uint64_t count, uint64_t dim,
                            float* out, cudaStream_t stream);
+// A call's answers and status words to pinned host memory (written by the device
+// through its mapping: one launch instead of three copies); clears the words.
+void launch_deliver(const Result* results, const double* exact_distances, uint32_t* counters,
+                    uint64_t count, Result* host_results, double* host_exact,
+                    uint32_t* host_counters, cudaStream_t stream);
 void launch_query_norms(const float* prepared, uint64_t batch,
                         uint64_t padded_dim, float* norms, cudaStream_t stream);
 

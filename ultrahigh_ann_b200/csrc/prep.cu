@@ -85,6 +85,23 @@ __global__ void prepare_sampled_kernel(const float* __restrict__ queries,
                          error_flag, blockIdx.x, gridDim.x, blockDim.x);
 }
 
+__global__ void deliver_kernel(const Result* __restrict__ results,
+                               const double* __restrict__ exact, uint32_t* counters,
+                               uint64_t count, Result* __restrict__ host_results,
+                               double* __restrict__ host_exact,
+                               uint32_t* __restrict__ host_counters)
+{
+    const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    if (i < count) {
+        host_results[i] = results[i];
+        host_exact[i] = exact[i];
+    }
+    if (i < 2) {
+        host_counters[i] = counters[i];
+        counters[i] = 0;
+    }
+}
+
 __global__ void query_norms_kernel(const float* __restrict__ prepared,
                                    uint64_t batch, uint64_t padded_dim,
                                    float* __restrict__ norms)
@@ -233,6 +250,16 @@ void launch_prepare_dense(const float* queries, uint64_t batch, uint64_t dim,
             queries, batch, dim, out, padded_dim, error_flag);
     }
     check_cuda(cudaGetLastError(), "cannot launch query preparation kernel");
+}
+
+void launch_deliver(const Result* results, const double* exact_distances, uint32_t* counters,
+                    uint64_t count, Result* host_results, double* host_exact,
+                    uint32_t* host_counters, cudaStream_t stream)
+{
+    const uint64_t blocks = (std::max<uint64_t>(count, 2) + kThreads - 1) / kThreads;
+    deliver_kernel<<<static_cast<uint32_t>(blocks), kThreads, 0, stream>>>(
+        results, exact_distances, counters, count, host_results, host_exact, host_counters);
+    check_cuda(cudaGetLastError(), "cannot launch the answer delivery kernel");
 }
 
 void launch_prepare_sampled(const float* queries, uint64_t batch, uint64_t dim,

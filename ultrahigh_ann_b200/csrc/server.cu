@@ -226,6 +226,7 @@ struct uha_server {
             check_cuda(cudaMemsetAsync(ws->raw_queries.get(), 0, ws->raw_queries.bytes(),
                                        ws->stream),
                        "cannot clear the query buffer");
+            ws->counters_clear = false;
             check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), ws->stream),
                        "cannot clear query counters");
             const BatchContext ctx{e.index, ws, e.strategy, true};
@@ -304,6 +305,7 @@ struct uha_server {
                                "cannot copy queries to the CUDA device");
                 }
             }
+            ws->counters_clear = false;
             check_cuda(cudaMemsetAsync(ws->counters.get(), 0, ws->counters.bytes(), ws->stream),
                        "cannot clear query counters");
             const BatchContext ctx{e.index, ws, e.strategy, true};
