@@ -1836,6 +1836,43 @@ __device__ double block_l2_64(const float* q, const float* r, uint64_t padded_di
                                __dadd_rn(scratch[6], scratch[7])));
 }
 
+// Binary64 L1 distance of one row summed by the whole block with the structure of
+// block_l2_64: the reference CPU's own terms, |q - r| or w |q - r| (weights: null
+// or the columns' binary64 weights), past the columns 0.
+__device__ double block_l1_64(const float* q, const float* r, const double* weights,
+                              uint64_t columns, uint64_t padded_dim, double* scratch)
+{
+    const uint64_t groups = padded_dim / 4;
+    const float4* q4 = reinterpret_cast<const float4*>(q);
+    const float4* r4 = reinterpret_cast<const float4*>(r);
+    auto term = [&](float a, float b, uint64_t j) {
+        const double d = fabs(__dsub_rn(static_cast<double>(a), static_cast<double>(b)));
+        return weights != nullptr ? (j < columns ? __dmul_rn(weights[j], d) : 0.0) : d;
+    };
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+#pragma unroll 4
+    for (uint64_t g = threadIdx.x; g < groups; g += kFinalizeThreads) {
+        const float4 x = q4[g];
+        const float4 y = __ldg(r4 + g);
+        a0 = __dadd_rn(a0, term(x.x, y.x, 4 * g));
+        a1 = __dadd_rn(a1, term(x.y, y.y, 4 * g + 1));
+        a2 = __dadd_rn(a2, term(x.z, y.z, 4 * g + 2));
+        a3 = __dadd_rn(a3, term(x.w, y.w, 4 * g + 3));
+    }
+    double t = __dadd_rn(__dadd_rn(a0, a1), __dadd_rn(a2, a3));
+    for (int o = 16; o > 0; o /= 2) {
+        t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+    }
+    if (threadIdx.x % 32 == 0) {
+        scratch[threadIdx.x / 32] = t;
+    }
+    __syncthreads();
+    return __dadd_rn(__dadd_rn(__dadd_rn(scratch[0], scratch[1]),
+                               __dadd_rn(scratch[2], scratch[3])),
+                     __dadd_rn(__dadd_rn(scratch[4], scratch[5]),
+                               __dadd_rn(scratch[6], scratch[7])));
+}
+
 struct Interval64 {
     double lower;
     double upper;
@@ -2144,7 +2181,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
              replay_count);
 }
 
-// The candidate lists of the split scan (split_scan.cu). grid = (parts, batch):
+// The candidate lists of the split and fixed-point scans. grid = (parts, batch):
 // each block sums its part of the columns for every candidate of the query
 // (usually one or two), from the original binary32 rows; the query's last block
 // adds the parts in order and settles the query, in binary64 or, with
@@ -2190,8 +2227,13 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         T d;
         if constexpr (kEmulated) {
             d = block_l2_32(qrow + begin, rrow + begin, end - begin, scratch);
-        } else {
+        } else if (in.op == ReplayOp::l2_sequential) {
             d = block_l2_64(qrow + begin, rrow + begin, end - begin, scratch);
+        } else {
+            const bool weighted = in.op == ReplayOp::l1_weighted_sequential;
+            d = block_l1_64(qrow + begin, rrow + begin,
+                            weighted ? in.weights64 + begin : nullptr,
+                            in.dim > begin ? in.dim - begin : 0, end - begin, scratch);
         }
         __syncthreads();  // scratch is free again
         if (threadIdx.x == 0) {

@@ -1566,6 +1566,168 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
     return 1 + launches;
 }
 
+// The fixed-point form of an exact or flat L1 index's rows, built on first use on
+// `stream` and synchronised before it is published; null when the index keeps
+// the binary32 scan.
+const uha::FixedRows* fixed_rows(const uha_index* index, cudaStream_t stream)
+{
+    std::lock_guard<std::mutex> lock(index->lowp_mutex);
+    uha::FixedRows& fx = index->fixed;
+    if (fx.ready) {
+        return fx.usable ? &fx : nullptr;
+    }
+    fx.ready = true;
+    fx.pitch = uha::fixed_pitch(index->scan_dim);
+    // in units of 16 bytes
+    const uint64_t head = index->rows + (fx.pitch + 4) / 4;
+    const uint64_t scratch = (uha::fixed_scratch_words(index->scan_dim) + 3) / 4;
+    const uint64_t values = checked_mul(index->rows, fx.pitch / 8, "fixed-point rows");
+    if (!fx.store.try_allocate(head + scratch + values)) {
+        return nullptr;
+    }
+    float* offsets = reinterpret_cast<float*>(fx.store.get() + index->rows);
+    unsigned int* words = reinterpret_cast<unsigned int*>(fx.store.get() + head);
+    uint16_t* data = reinterpret_cast<uint16_t*>(fx.store.get() + head + scratch);
+    fx.offsets = offsets;
+    fx.data = data;
+    uha::launch_fixed_rows(index->scan_rows.get(), index->rows, index->padded_dim,
+                           index->scan_dim, index->weights64.get(), data, fx.pitch, offsets,
+                           offsets + fx.pitch, fx.store.get(), words, stream);
+    fx.usable = uha::fixed_usable(words, index->scan_dim, fx.store.get(), index->rows,
+                                  offsets + fx.pitch, stream);
+    if (!fx.usable) {
+        fx.store.release();
+    }
+    return fx.usable ? &fx : nullptr;
+}
+
+// The fixed-point scan of this batch (everything it needs allocated here), or
+// null when it takes the binary32 scan: every direct L1 batch past the streaming
+// scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers a
+// call again when a candidate list overflows. An index's first such call also
+// builds the rows (7,028 x 60,660: 0.8 ms; 65,536 x 250: 0.1 ms and an allocation
+// of 0.35 ms), which the large calls win back at once.
+struct FixedBuffers {
+    uha::FixedParts* parts;
+    unsigned long long* upper;
+    unsigned long long* least;
+    uint16_t* queries;
+    uint32_t* sums;
+};
+const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::FixedPlan* plan,
+                                    FixedBuffers* buffers)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+        ws->emulated_replay || index->kind == IndexKind::hierarchical ||
+        index->metric != UHA_L1 || precision_strategy(c.strategy) || n <= 8 || n > 65535 ||
+        index->rows < 2 || index->rows > (1u << 24)) {
+        return nullptr;
+    }
+    const uha::FixedRows* fx = fixed_rows(index, ws->stream);
+    if (fx == nullptr) {
+        return nullptr;
+    }
+    *plan = uha::plan_fixed(index->rows, fx->pitch, n, index->sm_count);
+    auto grow = [&](auto& buffer, uint64_t count) {
+        if (buffer.size() >= count) {
+            return true;
+        }
+        check_cuda(cudaStreamSynchronize(ws->stream), "CUDA query failed");
+        return buffer.try_allocate(count);
+    };
+    const uint64_t b = ws->max_batch;
+    // each part in 16-byte units; FixedParts is 24 bytes
+    const uint64_t parts = (24 * n * uha::kSplitSlices + 15) / 16;
+    const uint64_t upper = (n + 1) / 2;
+    const uint64_t least = (checked_mul(n, uha::fixed_tiles(index->rows), "partials") + 1) / 2;
+    const uint64_t queries = checked_mul(n, fx->pitch / 8, "query buffer");
+    const uint64_t sums =
+        (checked_mul(checked_mul(plan->splits, n, "partials"), index->rows, "partials") + 3) / 4;
+    const uint64_t total = parts + upper + least + queries + sums;
+    if (!grow(ws->fixed_store, (16 * total + 23) / 24) ||
+        !grow(ws->split_words, 3 * b) ||
+        !grow(ws->split_candidates, b * uha::kSplitCandidates) ||
+        !grow(ws->split_sums, uha::settle_sums(b))) {
+        ws->split_disabled = true;
+        return nullptr;
+    }
+    unsigned char* at = reinterpret_cast<unsigned char*>(ws->fixed_store.get());
+    auto take = [&](uint64_t units) {
+        unsigned char* here = at;
+        at += 16 * units;
+        return here;
+    };
+    buffers->parts = reinterpret_cast<uha::FixedParts*>(take(parts));
+    buffers->upper = reinterpret_cast<unsigned long long*>(take(upper));
+    buffers->least = reinterpret_cast<unsigned long long*>(take(least));
+    buffers->queries = reinterpret_cast<uint16_t*>(take(queries));
+    buffers->sums = reinterpret_cast<uint32_t*>(take(sums));
+    return fx;
+}
+
+// One batch by the fixed-point scan.
+uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
+                             const uha::FixedPlan& plan, const FixedBuffers& buffers,
+                             const float* source, uint64_t n,
+                             uha::Result* results, double* exact, bool time_scan,
+                             cudaEvent_t scan_start, cudaEvent_t scan_stop)
+{
+    const uha_index* index = c.index;
+    uha_workspace* ws = c.ws;
+    cudaStream_t stream = ws->stream;
+    int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
+    uint32_t* words = ws->split_words.get();
+    uha::FixedVectors v{};
+    v.source = source;
+    v.source_pitch = query_dimension(c);
+    v.dim = index->scan_dim;
+    v.columns = query_columns(c);
+    v.weights = index->weights64.get();
+    v.offsets = rows.offsets;
+    v.step = rows.offsets + rows.pitch;
+    v.out = buffers.queries;
+    v.pitch = rows.pitch;
+    v.prepared = ws->prepared.get();
+    v.prepared_pitch = index->padded_dim;
+    v.query_parts = buffers.parts;
+    v.counts = words;
+    v.upper = buffers.upper;
+    v.done = words + 2 * ws->max_batch;
+    v.error_flag = error_flag;
+    uha::launch_fixed_queries(v, n, stream);
+    const uha::FixedQuery f{rows.store.get(),
+                            v.query_parts,
+                            uha::fixed_slices(rows.pitch, n),
+                            v.upper,
+                            v.counts,
+                            index->scan_dim};
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_start, stream), "event");
+    }
+    uha::launch_fixed_scan(plan, rows.data, index->rows, buffers.queries, n, rows.pitch,
+                           buffers.sums, buffers.least, f, ws->split_candidates.get(),
+                           error_flag, stream);
+    if (time_scan) {
+        check_cuda(cudaEventRecord(scan_stop, stream), "event");
+    }
+    uha::ReplayInputs in{};
+    in.op = index->weights64.size() != 0 ? uha::ReplayOp::l1_weighted_sequential
+                                         : uha::ReplayOp::l1_grouped4;
+    in.rows = index->scan_rows.get();
+    in.queries = ws->prepared.get();
+    in.dim = index->scan_dim;
+    in.padded_dim = index->padded_dim;
+    in.weights64 = index->weights64.get();
+    const uint32_t depth = uha::settle_depth(index->padded_dim);
+    uha::launch_settle(uha::make_bound64(depth, index->scan_dim), uha::Bound{}, in,
+                       ws->split_candidates.get(), v.counts, static_cast<uint32_t>(n),
+                       static_cast<uint32_t>(index->rows), ws->split_sums.get(), v.done,
+                       results, exact, ws->counters.get(), stream);
+    return plan.splits > 1 ? 5 : 4;
+}
+
 // The split scan of this batch, or false when it takes the binary32 scan: the
 // direct strategy on L2 indexes, batches past the streaming scan's, whose
 // caller answers a call again when a candidate list overflows. Everything the
@@ -1945,6 +2107,13 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     if (split_applies(c, n, &split, &split_plan)) {
         return enqueue_split_batch(c, *split, split_plan, source, n, results, exact, time_scan,
                                    scan_start, scan_stop);
+    }
+    uha::FixedPlan fixed_plan{};
+    FixedBuffers fixed_buffers{};
+    if (const uha::FixedRows* fixed = fixed_applies(c, n, &fixed_plan, &fixed_buffers);
+        fixed != nullptr) {
+        return enqueue_fixed_batch(c, *fixed, fixed_plan, fixed_buffers, source, n, results,
+                                   exact, time_scan, scan_start, scan_stop);
     }
     if (const uha::RowBits* bits = bits_scan_applies(c, n); bits != nullptr) {
         return enqueue_bits_batch(c, *bits, source, n, results, exact, time_scan, scan_start,

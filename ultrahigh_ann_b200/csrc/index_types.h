@@ -45,6 +45,19 @@ struct SplitRows {
     bool usable = false;
 };
 
+// The fixed-point form of an exact or flat L1 index's rows (fixed_scan.cu),
+// built on first use, in one allocation: each row's terms, the column offsets and
+// the step, the build's scratch, rows x pitch 16-bit values. `usable` is false when the memory was not
+// available or the step does not resolve the index's distances.
+struct FixedRows {
+    DeviceBuffer<FixedTerms> store;
+    const float* offsets = nullptr;  // pitch values, then the step
+    const uint16_t* data = nullptr;
+    uint64_t pitch = 0;
+    bool ready = false;
+    bool usable = false;
+};
+
 // The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use;
 // `usable` is false when the memory for them was not available.
 struct RowBits {
@@ -103,6 +116,7 @@ struct uha_index {
     mutable uha::LowpRows lowp_projection[2];  // L2 hierarchy: the p x k projection
     mutable uha::SplitRows split;
     mutable uha::RowBits bits;  // L1 hierarchy
+    mutable uha::FixedRows fixed;  // exact and flat L1
 };
 
 // A scan shape chosen by the autotuner for one (batch size, strategy) of a
@@ -170,6 +184,9 @@ struct uha_workspace {
     uha::DeviceBuffer<uint32_t> split_candidates;
     uha::DeviceBuffer<unsigned long long> split_keys;
     uha::DeviceBuffer<double> split_sums;
+    // fixed-point scan, one allocation: queries' parts, upper ends, tiles' least
+    // values, queries, sums (its other buffers are the split scan's)
+    uha::DeviceBuffer<uha::FixedParts> fixed_store;
     bool split_disabled = false;
     // median scan by bitmaps (allocated on first use): intervals, listed rows
     // and their medians; the per-query words are median_min and split_words

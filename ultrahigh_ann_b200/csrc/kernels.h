@@ -454,9 +454,79 @@ void launch_split_filter_scan(const SplitPlan& plan, const void* rows, uint64_t 
                               const SplitQuery& sq, unsigned long long* keys,
                               uint32_t* candidates, int* error_flag, int sm_count,
                               cudaStream_t stream);
+// ---- certified L1 scan in fixed point (fixed_scan.cu)
+// A row's sum of integers and its error in steps; a query's parts per slice.
+struct FixedTerms {
+    long long sum;
+    long long error;
+};
+struct FixedParts {
+    double sum;
+    double error;
+    double past;
+};
+// Vectors to bring into fixed point (fixed_vectors_kernel): rows get terms,
+// queries the prepared vectors, parts per slice and cleared words.
+struct FixedVectors {
+    const float* source;
+    uint64_t source_pitch;
+    uint64_t dim;
+    const uint32_t* columns;   // nullable: gathered
+    const double* weights;     // nullable: 1
+    const float* offsets;
+    const float* step;
+    uint16_t* out;
+    uint64_t pitch;
+    uint64_t slice;
+    bool vector_loads;
+    FixedTerms* terms;
+    float* prepared;
+    uint64_t prepared_pitch;
+    FixedParts* query_parts;
+    uint32_t* counts;
+    unsigned long long* upper;
+    uint32_t* done;
+    int* error_flag;
+};
+// What the selection reads of the rows and the queries.
+struct FixedQuery {
+    const FixedTerms* terms;    // rows
+    const FixedParts* parts;    // queries: slices per query
+    uint32_t slices;
+    unsigned long long* upper;
+    uint32_t* counts;
+    uint64_t dim;
+};
+struct FixedPlan {
+    uint32_t queries;            // per tile: 32 or 64
+    uint32_t splits;             // column splits (slabs of sums)
+    uint32_t columns_per_split;
+};
+uint64_t fixed_pitch(uint64_t dim);
+uint64_t fixed_scratch_words(uint64_t dim);
+// The rows (padded, weights nullable) in fixed point: row_count x pitch values,
+// offsets (pitch), the step and each row's terms; scratch:
+// fixed_scratch_words(dim).
+void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, uint64_t dim,
+                       const double* weights, uint16_t* out, uint64_t pitch, float* offsets,
+                       float* step, FixedTerms* terms, unsigned int* scratch, cudaStream_t stream);
+// Whether the step resolves this index's distances (synchronises `stream`).
+bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* terms,
+                  uint64_t row_count, const float* step, cudaStream_t stream);
+uint32_t fixed_slices(uint64_t pitch, uint64_t batch);
+void launch_fixed_queries(FixedVectors v, uint64_t batch, cudaStream_t stream);
+FixedPlan plan_fixed(uint64_t rows, uint64_t pitch, uint64_t batch, int sm_count);
+uint64_t fixed_tiles(uint64_t rows);
+// As launch_split_scan; sums: splits x batch x rows; least: batch x
+// fixed_tiles(rows).
+void launch_fixed_scan(const FixedPlan& plan, const uint16_t* rows, uint64_t row_count,
+                       const uint16_t* queries, uint64_t batch, uint64_t pitch, uint32_t* sums,
+                       unsigned long long* least, const FixedQuery& f, uint32_t* candidates, int* error_flag,
+                       cudaStream_t stream);
+
 // Certified argmin of each query over its listed candidates, from the original
-// binary32 rows (l2_sequential inputs; in.emulated: bound32, else bound64, both
-// of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
+// binary32 rows (exact and flat ops; in.emulated, L2 only: bound32, else
+// bound64, both of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
 uint32_t settle_depth(uint64_t padded_dim);
 uint64_t settle_sums(uint64_t batch);
 void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32_t* candidates,
