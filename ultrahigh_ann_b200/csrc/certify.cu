@@ -1371,6 +1371,8 @@ constexpr uint32_t kFlatCopySpins = 1u << 22;
 constexpr int kFlatCopyTimeout = 16;
 // bytes of rows per bulk copy of the flat query kernel (two buffers per CTA)
 constexpr uint64_t kFlatChunkBytes = 32 * 1024;
+// columns of the longest rows that are copied (plan_flat_query)
+constexpr uint64_t kFlatCopyColumns = 128;
 // query entries a flat query thread gathers at a time
 constexpr int kFlatGather = 8;
 // float4 loads in flight per lane when rows are read from global memory
@@ -1405,9 +1407,9 @@ __device__ __forceinline__ float flat_terms(int op, float acc, const float4 a,
 // grid = (row blocks, batch), kFinalizeThreads threads. At entry one thread
 // of every CTA starts bulk copies (the TMA engine, cp.async.bulk) of its row
 // block into shared memory: `chunk_rows` rows per copy, two buffers, the next
-// chunk copied while one is scanned (rows too long for a pass of the CTA in
-// one copy, chunk_rows 0, are instead loaded from global memory into
-// registers, kFlatDirectLoads per lane in flight). Meanwhile the CTA gathers its query's
+// chunk copied while one is scanned (rows past kFlatCopyColumns, chunk_rows 0,
+// are instead loaded from global memory into registers, kFlatDirectLoads per
+// lane in flight). Meanwhile the CTA gathers its query's
 // sampled (or all) coordinates into shared memory with the preparation
 // kernels' finiteness flags (and the column weights of a weighted L1 index).
 // Then it computes the binary32 distance of each row with kLanes lanes per row
@@ -1451,8 +1453,8 @@ __global__ void __launch_bounds__(kFinalizeThreads, 3)
     const uint32_t first_row = blockIdx.x * span;
     const uint32_t end_row = min(sq.row_count, first_row + span);
     const uint32_t row_words = static_cast<uint32_t>(sq.padded_dim);
-    // chunk_rows 0: rows too long for a pass of the CTA in one copy are read
-    // straight from global memory instead
+    // chunk_rows 0: rows past kFlatCopyColumns are read straight from global
+    // memory instead
     const uint32_t nchunks =
         chunk_rows != 0 ? (end_row - first_row + chunk_rows - 1) / chunk_rows : 0u;
     auto issue = [&](uint32_t c) {
@@ -1478,7 +1480,8 @@ __global__ void __launch_bounds__(kFinalizeThreads, 3)
     int local_bad = 0;
     // kFlatGather entries per thread at a time: their column indices (and
     // scales, weights) in flight together, then their query values together,
-    // so the gather costs two memory round trips, not two per entry
+    // so the gather costs two memory round trips, not two per entry; the steps
+    // past the columns are left out (a fifth of the kernel's instructions at 300)
     for (uint64_t base = threadIdx.x; base < sq.padded_dim;
          base += static_cast<uint64_t>(kFinalizeThreads) * kFlatGather) {
         uint32_t col[kFlatGather];
@@ -1487,6 +1490,9 @@ __global__ void __launch_bounds__(kFinalizeThreads, 3)
 #pragma unroll
         for (int u = 0; u < kFlatGather; ++u) {
             const uint64_t i = base + static_cast<uint64_t>(u) * kFinalizeThreads;
+            if (i - threadIdx.x >= sq.padded_dim) {
+                break;
+            }
             const bool sampled = sq.columns != nullptr && i < sq.sample_size;
             col[u] = sampled ? sq.columns[i] : 0u;
             scale[u] = sampled && sq.scales != nullptr ? sq.scales[i] : 1.f;
@@ -1496,6 +1502,9 @@ __global__ void __launch_bounds__(kFinalizeThreads, 3)
 #pragma unroll
         for (int u = 0; u < kFlatGather; ++u) {
             const uint64_t i = base + static_cast<uint64_t>(u) * kFinalizeThreads;
+            if (i - threadIdx.x >= sq.padded_dim) {
+                break;
+            }
             value[u] = 0.f;
             if (sq.columns == nullptr) {
                 if (i < sq.dim) {
@@ -1508,6 +1517,9 @@ __global__ void __launch_bounds__(kFinalizeThreads, 3)
 #pragma unroll
         for (int u = 0; u < kFlatGather; ++u) {
             const uint64_t i = base + static_cast<uint64_t>(u) * kFinalizeThreads;
+            if (i - threadIdx.x >= sq.padded_dim) {
+                break;
+            }
             if (i >= sq.padded_dim) {
                 continue;
             }
@@ -2825,7 +2837,7 @@ bool flat_query_fits(uint64_t rows, uint64_t padded_dim, uint64_t batch)
 }
 
 FlatPlan plan_flat_query(uint64_t rows, uint64_t padded_dim, uint64_t batch,
-                         int sm_count)
+                         int sm_count, bool shared)
 {
     const uint64_t groups = padded_dim / 4;
     // lanes per row: enough float4 groups per lane (about four or more) to
@@ -2835,8 +2847,16 @@ FlatPlan plan_flat_query(uint64_t rows, uint64_t padded_dim, uint64_t batch,
         lanes = groups < 16 * 4 ? 8 : 16;
     }
     const uint32_t step = kFinalizeThreads / lanes;  // rows per CTA pass
-    // about three CTAs per SM over the whole launch (one wave)
-    const uint64_t target = static_cast<uint64_t>(sm_count) * 3;
+    // CTAs over the whole launch. A launch alone on the chip takes three per SM
+    // (one wave). Where launches share it (several streams), what bounds them is
+    // the instructions that every CTA spends on the gather, the reduction and the
+    // merge: one CTA per SM, half as many again when the queries' scans are large
+    // (64 MB), for the loads in flight. us per query, one query per launch of
+    // 7,028 rows, three / one: 303 columns 5.2 / 3.2, 969: 8.5 / 4.6; 65,536 rows
+    // of 969 columns, 8 queries: one 192, one and a half 184.
+    const bool large = rows * padded_dim * sizeof(float) * batch > (64ull << 20);
+    const uint64_t target =
+        static_cast<uint64_t>(sm_count) * (!shared ? 6 : large ? 3 : 2) / 2;
     const uint64_t per_query = std::max<uint64_t>(1, target / batch);
     uint64_t span = (rows + per_query - 1) / per_query;
     span = std::max<uint64_t>(step, (span + step - 1) / step * step);
@@ -2844,12 +2864,15 @@ FlatPlan plan_flat_query(uint64_t rows, uint64_t padded_dim, uint64_t batch,
     plan.lanes = lanes;
     plan.span = static_cast<uint32_t>(span);
     plan.blocks = static_cast<uint32_t>((rows + span - 1) / span);
-    // rows per bulk copy: whole passes of the CTA up to kFlatChunkBytes; rows
-    // too long for one pass in a copy (a pass would leave most threads idle
-    // and serialise many small copies) are read from global memory directly
-    // (chunk_rows 0)
+    // Rows per bulk copy: whole passes of the CTA up to kFlatChunkBytes, for rows
+    // of at most kFlatCopyColumns; longer rows are read from global memory
+    // directly (chunk_rows 0): a lane then has enough loads of its own, and no
+    // shared memory limits the CTAs per SM (7,028 rows, 8 queries, one launch at a
+    // time, copies / direct: 54 columns 27.7 / 27.6 us, 969: 54 / 44; 65,536 rows,
+    // 54 columns 44 / 56, 303: 105 / 108, 969: 266 / 213).
     const uint64_t row_bytes = padded_dim * sizeof(float);
-    const uint64_t chunk = kFlatChunkBytes / row_bytes / step * step;
+    const uint64_t chunk =
+        padded_dim <= kFlatCopyColumns ? kFlatChunkBytes / row_bytes / step * step : 0;
     plan.chunk_rows = static_cast<uint32_t>(std::min<uint64_t>(chunk, span));
     plan.buffers = plan.chunk_rows == 0 ? 0u : plan.chunk_rows >= span ? 1u : 2u;
     uint32_t log_lanes = 0;

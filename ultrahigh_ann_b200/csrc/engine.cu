@@ -2063,7 +2063,8 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
         }
         sq.op = static_cast<int>(op);
         const uha::FlatPlan flat_plan =
-            flat ? uha::plan_flat_query(index->rows, index->padded_dim, n, index->sm_count)
+            flat ? uha::plan_flat_query(index->rows, index->padded_dim, n, index->sm_count,
+                                        c.flat_shared)
                  : uha::FlatPlan{};
         const uha::Bound bound =
             make_bound(flat ? flat_plan.depth : uha::small_query_depth(index->padded_dim),
@@ -2619,6 +2620,7 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
             }
             const bool timed = ws->timing && b % ws->timing_stride == 0;
             bc.flat_lane = static_cast<int>(b % static_cast<uint64_t>(lanes));
+            bc.flat_shared = lanes > 1;
             launches += enqueue_batch(bc, source, count, ws->call_results.get() + start,
                                       ws->call_exact.get() + start, timed,
                                       timed ? ws->scan_events[2 * b] : nullptr,

@@ -59,6 +59,7 @@ struct BatchContext {
     // (0: ws->stream; others: ws->flat_streams, forked and joined by the
     // caller) with that lane's scratch slots.
     int flat_lane = 0;
+    bool flat_shared = false;  // other lanes' launches run beside it
 };
 
 // Allocates and clears (on ws->stream) the fused flat query's scratch of

@@ -192,7 +192,7 @@ struct FlatPlan {
 };
 bool flat_query_fits(uint64_t rows, uint64_t padded_dim, uint64_t batch);
 FlatPlan plan_flat_query(uint64_t rows, uint64_t padded_dim, uint64_t batch,
-                         int sm_count);
+                         int sm_count, bool shared);
 // Scratch for a workspace of `capacity` queries, `slots` slots (two per
 // stream lane); zero when created, left with its counters at zero by every
 // launch.
