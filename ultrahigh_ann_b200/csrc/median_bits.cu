@@ -36,6 +36,7 @@
 #include "hier_body.cuh"
 #include "kernels.h"
 #include "median64.cuh"
+#include "tile_body.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -61,8 +62,10 @@ constexpr uint32_t kBlockQueries = kCountWarps * kWarpQueries;
 constexpr uint32_t kOffsetBytes = kBlockQueries * kGroup * 4;
 constexpr uint32_t kFullStage = kStageBytes + kOffsetBytes;
 constexpr int kBoundarySample = 1024;
-constexpr int kProjectQueries = 8;
-constexpr int kProjectColumns = 256;     // sampled columns staged at a time
+constexpr int kProjectQueries = 4;   // per warp of the projection kernel
+constexpr int kProjectThreads = 128;  // and columns per chunk
+constexpr int kProjectColumns = 8;   // columns of the projection per stage
+constexpr int kProjectStages = 3;
 constexpr int kThreads = 256;
 // polls of a copy wait before it gives up, and the error bit it then sets
 constexpr uint32_t kCopySpins = 1u << 22;
@@ -139,93 +142,191 @@ __global__ void __launch_bounds__(kChunkRows)
 
 // ------------------------------------------------------------- query side
 
-// grid (query groups): the sampled values of kProjectQueries queries gathered
-// into shared memory (with the finiteness flag) and their binary64 projection
-// in the reference's order, y = sum_i x_i P_i in i order, one thread per
-// coordinate and an independent chain per query. y64[q][p]; and, where y32 is
-// given, its binary32 rounding (zero past p), that rounding's error per
-// coordinate and its maximum. Bound: the chains' latency; the gather's scattered
-// reads overlap across blocks.
-__global__ void __launch_bounds__(kThreads)
+// 8 bytes copied asynchronously into shared memory, or zeros
+__device__ __forceinline__ void copy8(double* to, const double* from, bool ok)
+{
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(to));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(from),
+                 "r"(ok ? 8 : 0)
+                 : "memory");
+}
+
+// grid (query groups), kProjectThreads threads: the sampled values of the group's
+// queries gathered into shared memory (with the finiteness flag) and their
+// binary64 projection in the reference's order, y = sum_i x_i P_i in i order. A
+// warp takes kProjectQueries queries and C coordinates per lane (lane, lane + 32,
+// ...), an independent chain per query and coordinate; `blocks` warps (a power of
+// two) share a query over its coordinates, the rest of the CTA's warps take more
+// queries. y64[q][p]; and, where y32 is given, its binary32 rounding (zero past
+// p), that rounding's error per coordinate and its maximum.
+//
+// Bound: shared-memory reads of the queries (a broadcast of 8 bytes costs the
+// return bandwidth of 32, two cycles per query and column; C coordinates share
+// it), then the FP64 pipe (two instructions per query, coordinate and column).
+// A chunk's scattered reads are all in flight at once, and the next chunk's
+// behind the sums: one thread per column, one query value each. The projection's
+// columns, which every CTA reads at about the same time, come kProjectColumns a
+// stage through shared memory, two stages ahead (register loads four columns
+// ahead left the warps waiting for them). 4,096 queries x about 350 columns,
+// p = 64: 120 us with one coordinate and 8 queries per thread, the gather a load
+// at a time and the weights from global memory; 62 us so (184 MB of DRAM lines
+// for the scattered values).
+template <int C>
+__global__ void __launch_bounds__(kProjectThreads)
     gather_project64_kernel(const float* __restrict__ queries, uint32_t batch, uint64_t dim,
                             const uint32_t* __restrict__ columns, uint32_t k,
-                            const double* __restrict__ proj_t, uint32_t p,
+                            const double* __restrict__ proj_t, uint32_t p, uint32_t blocks,
                             double* __restrict__ y64, float* __restrict__ y32,
                             uint32_t padded_p, float* __restrict__ coord_err,
                             float* __restrict__ query_err, int* error_flag)
 {
-    __shared__ double x[kProjectColumns][kProjectQueries];
-    __shared__ unsigned int largest[kProjectQueries];
-    const uint32_t q0 = blockIdx.x * kProjectQueries;
-    if (threadIdx.x < kProjectQueries) {
+    constexpr int kWarps = kProjectThreads / 32;
+    constexpr int kMost = kWarps * kProjectQueries;  // queries of a CTA, at most
+    extern __shared__ __align__(16) double staged[];  // kProjectStages x columns x width
+    __shared__ __align__(16) double x[kMost][kProjectThreads];
+    __shared__ unsigned int largest[kMost];
+    const uint32_t groups = kWarps / blocks;
+    const uint32_t here = groups * kProjectQueries;  // queries of this CTA
+    const uint32_t q0 = blockIdx.x * here;
+    const uint32_t warp = threadIdx.x / 32;
+    const uint32_t lane = threadIdx.x % 32;
+    const uint32_t m0 = warp / blocks * kProjectQueries;
+    if (threadIdx.x < kMost) {
         largest[threadIdx.x] = 0;
     }
-    const uint32_t threads = blockDim.x;
-    // coordinates in rounds of the block's threads (one round up to 256)
-    for (uint32_t j0 = 0; j0 < padded_p; j0 += threads) {
-        const uint32_t j = j0 + threadIdx.x;
-        double acc[kProjectQueries];
+    float next[kMost];
+    auto fetch = [&](uint32_t i0) {
+        const uint32_t i = i0 + threadIdx.x;
+        const uint32_t column = i < k ? columns[i] : 0;
+#pragma unroll
+        for (int m = 0; m < kMost; ++m) {
+            next[m] = i < k && m < here && q0 + m < batch ? queries[(q0 + m) * dim + column]
+                                                          : 0.f;
+        }
+    };
+    // coordinates in rounds of 32 C blocks (one round up to 512)
+    for (uint32_t j0 = 0; j0 < padded_p; j0 += 32 * C * blocks) {
+        const uint32_t j = j0 + warp % blocks * 32 * C + lane;
+        double acc[kProjectQueries][C];
 #pragma unroll
         for (int m = 0; m < kProjectQueries; ++m) {
-            acc[m] = 0.0;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                acc[m][c] = 0.0;
+            }
         }
-        for (uint32_t i0 = 0; i0 < k; i0 += kProjectColumns) {
+        const uint32_t width = 32 * C * blocks;  // a power of two
+        const uint32_t shift = __ffs(width) - 1;
+        const uint32_t stages = (k + kProjectColumns - 1) / kProjectColumns;
+        auto stage = [&](uint32_t at) {
+            if (at < stages) {
+                double* to = staged + at % kProjectStages * kProjectColumns * width;
+                for (uint32_t e = threadIdx.x; e < kProjectColumns * width;
+                     e += kProjectThreads) {
+                    const uint32_t i = at * kProjectColumns + (e >> shift);
+                    const uint32_t c = j0 + (e & (width - 1));
+                    const bool ok = i < k && c < p;
+                    copy8(to + e, proj_t + (ok ? static_cast<uint64_t>(i) * p + c : 0), ok);
+                }
+            }
+            tilebody::cp_async_commit();
+        };
+        __syncthreads();  // the last round's stages are read
+        stage(0);
+        stage(1);
+        fetch(0);
+        const double* mine = staged + warp % blocks * 32 * C + lane;
+        for (uint32_t at = 0; at < stages; ++at) {
+            const uint32_t i0 = at * kProjectColumns;
+            const uint32_t in_chunk = i0 % kProjectThreads;
+            if (in_chunk == 0) {
+                __syncthreads();
+                bool bad = false;
+#pragma unroll
+                for (int m = 0; m < kMost; ++m) {
+                    bad |= !isfinite(next[m]);
+                    x[m][threadIdx.x] = static_cast<double>(next[m]);
+                }
+                if (bad) {
+                    atomicOr(error_flag, 1);
+                }
+                if (i0 + kProjectThreads < k) {
+                    fetch(i0 + kProjectThreads);
+                }
+            }
+            tilebody::cp_async_wait<1>();
+            // stage `at` and the chunk are there, and the stage before is read
+            __syncthreads();
+            stage(at + 2);
+            const double* w = mine + at % kProjectStages * kProjectColumns * width;
             const uint32_t count = min(static_cast<uint32_t>(kProjectColumns), k - i0);
-            __syncthreads();
-            for (uint32_t e = threadIdx.x; e < count * kProjectQueries; e += threads) {
-                const uint32_t i = e % count;
-                const uint32_t m = e / count;
-                float v = 0.f;
-                if (q0 + m < batch) {
-                    v = queries[(q0 + m) * dim + columns[i0 + i]];
-                    if (!isfinite(v)) {
-                        atomicOr(error_flag, 1);
+            auto columns_of = [&](uint32_t u) {
+                double wc[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    wc[c] = w[u * width + 32 * c];
+                }
+#pragma unroll
+                for (int m = 0; m < kProjectQueries; ++m) {
+                    const double v = x[m0 + m][in_chunk + u];
+#pragma unroll
+                    for (int c = 0; c < C; ++c) {
+                        acc[m][c] = __dadd_rn(acc[m][c], __dmul_rn(v, wc[c]));
                     }
                 }
-                x[i][m] = static_cast<double>(v);
-            }
-            __syncthreads();
-            if (j < p) {
-                const double* c = proj_t + static_cast<uint64_t>(i0) * p + j;
-#pragma unroll 8
-                for (uint32_t i = 0; i < count; ++i) {
-                    const double w = c[static_cast<uint64_t>(i) * p];
-#pragma unroll
-                    for (int m = 0; m < kProjectQueries; ++m) {
-                        acc[m] = __dadd_rn(acc[m], __dmul_rn(x[i][m], w));
-                    }
+            };
+            if (count == kProjectColumns) {
+#pragma unroll 4
+                for (uint32_t u = 0; u < kProjectColumns; ++u) {
+                    columns_of(u);
+                }
+            } else {
+                for (uint32_t u = 0; u < count; ++u) {
+                    columns_of(u);
                 }
             }
         }
 #pragma unroll
         for (int m = 0; m < kProjectQueries; ++m) {
-            const uint32_t q = q0 + m;
-            if (q >= batch || j >= padded_p) {
-                continue;
-            }
-            const double y = j < p ? acc[m] : 0.0;
-            if (!isfinite(y)) {
-                atomicOr(error_flag, 4);
-            }
-            if (j < p) {
-                y64[static_cast<uint64_t>(q) * p + j] = y;
-            }
-            if (y32 != nullptr) {
-                const float r = static_cast<float>(y);
-                if (!(fabsf(r) <= FLT_MAX)) {
-                    // past binary32: the binary32 scan answers (or refuses)
-                    atomicOr(error_flag, kCandidateOverflow);
+            const uint32_t q = q0 + m0 + m;
+            float worst = 0.f;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const uint32_t at = j + 32 * c;
+                if (q >= batch || at >= padded_p) {
+                    continue;
                 }
-                // exact: y and its rounding differ by at most half an ulp
-                const float e = __double2float_ru(fabs(__dsub_rn(y, static_cast<double>(r))));
-                y32[static_cast<uint64_t>(q) * padded_p + j] = r;
-                coord_err[static_cast<uint64_t>(q) * padded_p + j] = e;
-                atomicMax(largest + m, __float_as_uint(e));
+                const double y = at < p ? acc[m][c] : 0.0;
+                if (!isfinite(y)) {
+                    atomicOr(error_flag, 4);
+                }
+                if (at < p) {
+                    y64[static_cast<uint64_t>(q) * p + at] = y;
+                }
+                if (y32 != nullptr) {
+                    const float r = static_cast<float>(y);
+                    if (!(fabsf(r) <= FLT_MAX)) {
+                        // past binary32: the binary32 scan answers (or refuses)
+                        atomicOr(error_flag, kCandidateOverflow);
+                    }
+                    // exact: y and its rounding differ by at most half an ulp
+                    const float e =
+                        __double2float_ru(fabs(__dsub_rn(y, static_cast<double>(r))));
+                    y32[static_cast<uint64_t>(q) * padded_p + at] = r;
+                    coord_err[static_cast<uint64_t>(q) * padded_p + at] = e;
+                    worst = e > worst || isnan(e) ? e : worst;
+                }
+            }
+            // the bit patterns of nonnegative values (and NaN above them) order
+            // as integers
+            const unsigned int most = __reduce_max_sync(0xffffffffu, __float_as_uint(worst));
+            if (lane == 0) {
+                atomicMax(largest + m0 + m, most);
             }
         }
     }
     __syncthreads();
-    if (y32 != nullptr && threadIdx.x < kProjectQueries && q0 + threadIdx.x < batch) {
+    if (y32 != nullptr && threadIdx.x < here && q0 + threadIdx.x < batch) {
         query_err[q0 + threadIdx.x] = __uint_as_float(largest[threadIdx.x]);
     }
 }
@@ -739,13 +840,29 @@ void launch_gather_project64(const float* queries, uint64_t batch, uint64_t dim,
                              float* coord_err, float* query_err, int* error_flag,
                              cudaStream_t stream)
 {
-    const uint32_t threads = static_cast<uint32_t>(
-        std::min<uint64_t>(kThreads, std::max<uint64_t>(64, round_up(padded_p, 32))));
-    gather_project64_kernel<<<static_cast<uint32_t>((batch + kProjectQueries - 1) /
-                                                    kProjectQueries),
-                              threads, 0, stream>>>(
+    // coordinates per lane, then warps per query, by the coordinates there are
+    const uint32_t each = padded_p <= 32 ? 1 : padded_p <= 64 ? 2 : 4;
+    const uint32_t blocks = padded_p <= 128 ? 1 : padded_p <= 256 ? 2 : 4;
+    const uint32_t here = kProjectThreads / 32 / blocks * kProjectQueries;
+    const uint32_t grid = static_cast<uint32_t>((batch + here - 1) / here);
+    const auto kernel = each == 1   ? gather_project64_kernel<1>
+                        : each == 2 ? gather_project64_kernel<2>
+                                    : gather_project64_kernel<4>;
+    const size_t smem = sizeof(double) * kProjectStages * kProjectColumns * 32 * each * blocks;
+    if (smem > 32 * 1024) {
+        static std::once_flag once[kMaxDevices];
+        std::call_once(once[current_device()], [&] {
+            // the most: 4 coordinates per lane, 4 warps per query
+            check_cuda(cudaFuncSetAttribute(gather_project64_kernel<4>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(sizeof(double) * kProjectStages *
+                                                             kProjectColumns * 32 * 4 * 4)),
+                       "cannot configure the gathering projection kernel");
+        });
+    }
+    kernel<<<grid, kProjectThreads, smem, stream>>>(
         queries, static_cast<uint32_t>(batch), dim, columns, static_cast<uint32_t>(k), proj_t,
-        static_cast<uint32_t>(p), y64, y32, static_cast<uint32_t>(padded_p), coord_err,
+        static_cast<uint32_t>(p), blocks, y64, y32, static_cast<uint32_t>(padded_p), coord_err,
         query_err, error_flag);
     check_cuda(cudaGetLastError(), "cannot launch the gathering projection kernel");
 }
