@@ -1510,7 +1510,7 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
         return buffer.try_allocate(count);
     };
     const uint64_t b = ws->max_batch;
-    const uint64_t list = checked_mul(b, uha::kBitsList, "row lists");
+    const uint64_t list = checked_mul(b, uha::bits_list(index->rows), "row lists");
     if (!grow(ws->median_min, std::max(n, b)) || !grow(ws->split_words, 3 * b) ||
         !grow(ws->projected64, checked_mul(b, index->projection_dimension, "queries")) ||
         !grow(ws->bits_offsets, uha::bits_offsets(b, index->projection_dimension)) ||
@@ -1605,7 +1605,7 @@ const uha::FixedRows* fixed_rows(const uha_index* index, cudaStream_t stream)
 // null when it takes the binary32 scan: every direct L1 batch past the streaming
 // scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers a
 // call again when a candidate list overflows. An index's first such call also
-// builds the rows (7,028 x 60,660: 0.8 ms; 65,536 x 250: 0.1 ms and an allocation
+// builds the rows (7,028 x 60,660: 0.8 ms; 65,536 x 128: 0.1 ms and an allocation
 // of 0.35 ms), which the large calls win back at once.
 struct FixedBuffers {
     uha::FixedParts* parts;

@@ -611,8 +611,9 @@ void launch_gather_project64(const float* queries, uint64_t batch, uint64_t dim,
 // Indexes with a bitmap form, its size, and its construction from the scanned
 // binary32 rows (boundaries: bits_boundaries(p) floats).
 constexpr uint64_t kBitsRows = 1024;
-// rows listed per query at most, and spread rows of the first threshold
-constexpr uint32_t kBitsList = 1024;
+// rows listed per query at most (1,024 or 4,096)
+uint32_t bits_list(uint64_t rows);
+// spread rows of the first threshold, within every list
 constexpr uint32_t kBitsSpread = 32;
 bool bits_applies(uint64_t rows, uint64_t p);
 // Batches that the bitmaps answer faster than the binary32 passes.
@@ -626,7 +627,7 @@ void launch_row_bits(const float* rows, uint64_t row_count, uint64_t padded_p, u
 // Certified argmin of a projected batch; results and exact distances are the
 // reference's. Error bit kCandidateOverflow: answer the call again by the
 // binary32 passes. offsets: bits_offsets(batch, p); listed, medians: batch x
-// kBitsList; min_bits, counts: batch. Returns the kernel launches.
+// bits_list(rows); min_bits, counts: batch. Returns the kernel launches.
 struct BitsScan {
     const float* rows;
     uint64_t row_count;

@@ -27,7 +27,7 @@
 // (l1_hierarchical_projection.cpp's order) is formed first, and the binary32
 // queries are its roundings, so a query value's error is its own rounding only.
 //
-// Measured (B200, 65,536 rows, p = 64, 4,096 queries): 0.79 ms a call against
+// Measured (B200, 65,536 rows, p = 64, 4,096 queries): 0.78 ms a call against
 // 5.4 ms by the binary32 passes; the last count 278 us against 2,527 us, the
 // medians 330 us in all against 2,030 us (about 160 rows listed per query, 10 of
 // them within the threshold), no slab of 65,536 x 4,096 distances.
@@ -167,7 +167,7 @@ __device__ __forceinline__ void copy8(double* to, const double* from, bool ok)
 // behind the sums: one thread per column, one query value each. The projection's
 // columns, which every CTA reads at about the same time, come kProjectColumns a
 // stage through shared memory, two stages ahead (register loads four columns
-// ahead left the warps waiting for them). 4,096 queries x about 350 columns,
+// ahead left the warps waiting for them). 4,096 queries x about 370 columns,
 // p = 64: 120 us with one coordinate and 8 queries per thread, the gather a load
 // at a time and the weights from global memory; 62 us so (184 MB of DRAM lines
 // for the scattered values).
@@ -346,9 +346,11 @@ struct Bits {
     float abs_err;
     unsigned int* min_bits;   // per query: bits of the smallest median so far
     uint32_t* counts;         // per query: rows listed
-    uint32_t* listed;         // batch x kBitsList rows
-    float2* medians;          // batch x kBitsList: median, its error
+    uint32_t* listed;         // batch x list rows
+    float2* medians;          // batch x list: median, its error
+    uint32_t list;            // rows listed per query at most
     int* error_flag;
+    bool complete;            // the pass whose lists are settled
 };
 
 // grid (queries, parts), a warp per row: the binary32 medians of the query's
@@ -367,11 +369,11 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t q = blockIdx.x;
     const int lane = threadIdx.x % 32;
     const uint32_t warps = gridDim.y * (kThreads / 32);
-    const uint32_t n = spread != 0 ? spread : min(a.counts[q], kBitsList);
+    const uint32_t n = spread != 0 ? spread : min(a.counts[q], a.list);
     const float* y = a.queries + static_cast<uint64_t>(q) * a.padded_p;
     const float* ye = a.coord_err + static_cast<uint64_t>(q) * a.padded_p;
-    uint32_t* list = a.listed + static_cast<uint64_t>(q) * kBitsList;
-    float2* medians = a.medians + static_cast<uint64_t>(q) * kBitsList;
+    uint32_t* list = a.listed + static_cast<uint64_t>(q) * a.list;
+    float2* medians = a.medians + static_cast<uint64_t>(q) * a.list;
     const volatile unsigned int* best = a.min_bits + q;
     for (uint32_t i = blockIdx.y * (kThreads / 32) + threadIdx.x / 32; i < n; i += warps) {
         const uint32_t row =
@@ -625,7 +627,8 @@ __global__ void __launch_bounds__(kCountThreads, 1)
     uint32_t base = 0;
     if (mine != 0) {
         base = atomicAdd(a.counts + q0 + lane, mine);
-        if (base + mine > kBitsList) {
+        // an earlier pass only tightens the threshold: any rows do
+        if (a.complete && base + mine > a.list) {
             atomicOr(a.error_flag, kCandidateOverflow);
         }
     }
@@ -642,9 +645,9 @@ __global__ void __launch_bounds__(kCountThreads, 1)
             before += lane >= o ? other : 0u;
         }
         at += before - __popc(keep[m]);
-        uint32_t* list = a.listed + static_cast<uint64_t>(q0 + m) * kBitsList;
+        uint32_t* list = a.listed + static_cast<uint64_t>(q0 + m) * a.list;
         for (uint32_t bitsleft = keep[m]; bitsleft != 0u; bitsleft &= bitsleft - 1u, ++at) {
-            if (at < kBitsList) {
+            if (at < a.list) {
                 list[at] = chunk * kChunkRows + lane * 32 + (__ffs(bitsleft) - 1);
             }
         }
@@ -666,9 +669,9 @@ __global__ void __launch_bounds__(kThreads)
     if (q >= a.batch) {
         return;
     }
-    const uint32_t n = min(a.counts[q], kBitsList);
-    const float2* medians = a.medians + static_cast<uint64_t>(q) * kBitsList;
-    const uint32_t* list = a.listed + static_cast<uint64_t>(q) * kBitsList;
+    const uint32_t n = min(a.counts[q], a.list);
+    const float2* medians = a.medians + static_cast<uint64_t>(q) * a.list;
+    const uint32_t* list = a.listed + static_cast<uint64_t>(q) * a.list;
     // |reference median - m| <= rel m + err + abs
     auto reach = [&](float2 m) {
         return __fadd_ru(__fadd_ru(__fmul_ru(a.rel, m.x), m.y), a.abs_err);
@@ -772,7 +775,9 @@ uint64_t launch_passes(const Bits& a, const BitsScan& s, Result* results,
         const bool all = chunks <= (taken == 1 ? 1 : 2 * taken);
         intervals_kernel<<<padded, std::min<uint32_t>(256, columns), 0, stream>>>(
             a, s.boundaries, columns, s.offsets);
-        launch_count<PLANES>(a, static_cast<const unsigned char*>(s.bits), columns, s.offsets,
+        Bits pass = a;
+        pass.complete = all;
+        launch_count<PLANES>(pass, static_cast<const unsigned char*>(s.bits), columns, s.offsets,
                              all ? chunks : taken, all ? 1 : chunks / taken, needed, stream);
         launch_list_medians<PER_LANE>(a, 0, needed, stream);
         launches += 3;
@@ -792,6 +797,15 @@ uint64_t launch_passes(const Bits& a, const BitsScan& s, Result* results,
 bool bits_applies(uint64_t rows, uint64_t p)
 {
     return rows >= kBitsRows && rows <= 0xffffffffull - kChunkRows && p >= 1 && p <= 256;
+}
+
+uint32_t bits_list(uint64_t rows)
+{
+    // The last pass lists about 160 of 65,536 rows per query at p = 64. At p = 256
+    // a query far from every row can list more than 1,024 (one or so in 4,096
+    // queries, whose whole call the binary32 passes then answered again: 16.4 ms
+    // against 2.3), so indexes of many rows get four times the slots.
+    return rows <= 16384 ? 1024 : 4096;
 }
 
 bool bits_batch(uint64_t p, uint64_t batch)
@@ -887,7 +901,9 @@ uint64_t launch_bits_scan(const BitsScan& s, uint64_t batch, Result* results,
                  s.counts,
                  s.listed,
                  s.medians,
-                 error_flag};
+                 bits_list(s.row_count),
+                 error_flag,
+                 false};
     check_cuda(cudaMemsetAsync(a.min_bits, 0xff, batch * sizeof(unsigned int), stream),
                "cannot clear median thresholds");
     if (s.p <= 32) {
