@@ -50,10 +50,14 @@ typedef enum uha_metric {
  * CudaDenseL2QueryStrategy / CudaSampledCoordinateL2QueryStrategy /
  * CudaHierarchicalL{1,2}QueryStrategy (include/ultrahigh_ann/core/
  * cuda_dense_l2_scan_index.hpp:17-23); the precision forms are appended.
- *   UHA_DIRECT: binary32 scan on CUDA cores with a certified error bound per
- *     distance; queries whose winner is not certified are re-scored by
+ *   UHA_DIRECT: a scan whose every distance has a certified error bound:
+ *     binary32 on CUDA cores, or, for batches past 8 queries, estimates on
+ *     the tensor cores (L2), in 16-bit fixed point (L1) or by row bitmaps (L1
+ *     hierarchies) whose candidates are settled from the original values in
+ *     binary64. Queries whose winner is not certified are re-scored by
  *     replaying the reference CPU's binary64 operation sequence, so the
- *     returned index equals the reference CPU index on every query.
+ *     returned index equals the reference CPU index on every query. The row
+ *     forms of the batch scans are built on the first query that needs them.
  *   UHA_GEMM: the reference's unrefined binary32 norm identity
  *     ||r||^2 + ||q||^2 - 2 r.q (L2 only; L1 treats it as DIRECT).
  *   UHA_GEMM_BF16_RERANK, UHA_GEMM_FP8_RERANK (exact, flat and
@@ -388,7 +392,9 @@ typedef struct uha_tune_report {
 /* Times every candidate scan shape for batches of exactly `batch` queries with
  * `strategy` on this workspace (CUDA events, median of 3 launches) and keeps
  * the fastest: later queries of that batch size on this workspace use it.
- * Answers do not change (the certification bound follows the shape).
+ * Answers do not change (the certification bound follows the shape). For L1
+ * batches past 8 queries it is the shape of the binary32 scan, which answers
+ * only where the estimates do not.
  * L1 hierarchies time their median passes (sample, pruning count,
  * survivors) on stand-in queries, midpoints of pairs of the index's own
  * projected rows, since their cost depends on the data; the workspace's query

@@ -21,11 +21,11 @@
 // original values in binary64 (certify.cu).
 //
 // Measured, device queries, one call: 7,028 rows x 60,660 columns, 333 queries:
-// 14.1 -> 6.1 ms (the tile kernel 13.0 -> 5.9 ms, the rate of its two
-// instructions); 65,536 rows x 250 sampled columns, 256 queries: 430 -> 183 us
-// (tiles 117 us, the same rate). It was the faster one at every size tried (33 to
-// 40,000 rows, 64 to 60,660 columns, 9 to 400 queries: 1.1 to 9 times), so every
-// direct L1 batch past the streaming scan's 8 queries takes it.
+// 14.1 -> 6.1 ms (the tile kernel 13.0 -> 5.9 ms); 65,536 rows x 128 columns (a
+// flat index), 256 queries: 430 -> 183 us (tiles 117 us). It was the faster one at
+// every size tried (33 to 40,000 rows, 64 to 60,660 columns, 9 to 400 queries: 1.1
+// to 9 times), so every direct L1 batch past the streaming scan's 8 queries takes
+// it.
 #include "common.h"
 #include "kernels.h"
 #include "tile_body.cuh"
@@ -292,8 +292,12 @@ __device__ __forceinline__ QueryTerms query_terms(const FixedQuery& f, uint32_t 
 // grid (row tiles, query tiles, splits): sums[split][q][row] = sum of the larger
 // of the two integers over the split's columns (at most 65,536 of them: below
 // 2^32). 128 rows x 8 J queries per CTA, an 8 x J micro-tile per thread, 64-column
-// stages double-buffered with cp.async. Bound: issue, two instructions per pair
-// of columns; the 16-byte shared-memory reads serve 8 x J outputs. The column
+// stages double-buffered with cp.async. Bound: the two instructions per pair of
+// columns, 79 % of the issue slots busy (333 queries x 7,028 x 60,660; 72 % at
+// 65,536 rows x 128 columns), the dot product's pipe, which runs at half rate,
+// being nearly full. (14-bit values, four maxima added before one dot product,
+// are 7 instructions for 8 but took 7.0 ms for 5.9: the additions share the
+// maxima's pipe.) The 16-byte shared-memory reads serve 8 x J outputs. The column
 // loop stays rolled past 8 columns: unrolled it does not fit the instruction
 // cache.
 // With one split, `least` [q][row tile] is the smallest T - error over the tile's

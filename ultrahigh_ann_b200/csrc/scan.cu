@@ -9,7 +9,8 @@
 // * stream kernel (batch <= 8): HBM-bound regime. A CTA owns 16 rows x one
 //   2048-column chunk; the query chunk is staged in shared memory once and each
 //   warp streams two rows with 128-bit non-allocating loads.
-// * tile kernel (batch > 8): CUDA-core-bound regime. A CTA computes a 128-row x
+// * tile kernel (batch > 8 where the estimating scans of split_scan.cu,
+//   fixed_scan.cu and median_bits.cu do not apply): CUDA-core-bound regime. A CTA computes a 128-row x
 //   64-query tile with an 8x8 register micro-tile per thread; 32-column stages
 //   are double-buffered through shared memory with cp.async, and the K range
 //   may be split across CTAs (split-K) to fill the 148 SMs.
