@@ -129,3 +129,27 @@ def test_captured_batches_answer_new_queries(oracle_module):
     for q in (near, plain, near):
         want, _ = oracle_module.exact("l1", rows, q)
         assert np.array_equal(batch.run([q])[0][0], want)
+
+
+@pytest.mark.parametrize("d", [32000, 32001])
+def test_both_widths_of_the_epilogue(d):
+    # 444 tiles fill the chip at one column split; the binary32 scan (FP64-free
+    # settlement) answers the same queries
+    torch = pytest.importorskip("torch")
+    torch.manual_seed(d)
+    rows = torch.rand(444 * 128 - 5, d, device="cuda")
+    queries = torch.rand(64, d, device="cuda")
+    queries[:32] = rows[1000:57000:1750][:32] + 0.02 * torch.rand(32, d, device="cuda")
+    torch.cuda.synchronize()
+    index = uha.CudaExactL1Index(rows)
+    answers = []
+    for emulated in (False, True):
+        ws = index.make_query_workspace(64)
+        ws.set_replay(emulated)
+        dist = np.zeros(64)
+        out = np.zeros(64, np.uint64)
+        index.query_device_batch(queries.data_ptr(), 64, out, ws, distances=dist)
+        answers.append((out, dist))
+    assert np.array_equal(answers[0][0], answers[1][0])
+    assert np.array_equal(answers[0][0][:32], np.arange(1000, 57000, 1750)[:32])
+    np.testing.assert_allclose(answers[0][1], answers[1][1], rtol=1e-5)

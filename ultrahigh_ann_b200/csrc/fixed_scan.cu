@@ -22,10 +22,10 @@
 //
 // Measured, device queries, one call: 7,028 rows x 60,660 columns, 333 queries:
 // 14.1 -> 6.1 ms (the tile kernel 13.0 -> 5.9 ms); 65,536 rows x 128 columns (a
-// flat index), 256 queries: 430 -> 183 us (tiles 117 us). It was the faster one at
-// every size tried (33 to 40,000 rows, 64 to 60,660 columns, 9 to 400 queries: 1.1
-// to 9 times), so every direct L1 batch past the streaming scan's 8 queries takes
-// it.
+// flat index), 256 queries: 430 -> 154-188 us (tiles 107 us). It was the faster
+// one at every size tried (33 to 40,000 rows, 64 to 60,660 columns, 9 to 400
+// queries: 1.1 to 9 times), so every direct L1 batch past the streaming scan's 8
+// queries takes it.
 #include "common.h"
 #include "kernels.h"
 #include "tile_body.cuh"
@@ -34,6 +34,7 @@
 #include <cfloat>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 namespace uha {
 namespace {
@@ -53,6 +54,8 @@ constexpr int kSelectRows = 8;
 constexpr uint32_t kRangeRows = 256;     // rows per block of the range kernel
 // steps of error per column that the binary32 arithmetic of the conversion adds
 constexpr double kColumnSlack = 0x1p-6;
+// up to here T and a row's error (at most a step per column) stay below 2^31
+constexpr uint64_t kNarrowColumns = 32000;
 constexpr uint32_t kPairs = 64;          // row pairs of the quality estimate
 constexpr float kLevels = 65535.f;
 
@@ -293,7 +296,7 @@ __device__ __forceinline__ QueryTerms query_terms(const FixedQuery& f, uint32_t 
 // of the two integers over the split's columns (at most 65,536 of them: below
 // 2^32). 128 rows x 8 J queries per CTA, an 8 x J micro-tile per thread, 64-column
 // stages double-buffered with cp.async. Bound: the two instructions per pair of
-// columns, 79 % of the issue slots busy (333 queries x 7,028 x 60,660; 72 % at
+// columns, 79 % of the issue slots busy (333 queries x 7,028 x 60,660; 73 % at
 // 65,536 rows x 128 columns), the dot product's pipe, which runs at half rate,
 // being nearly full. (14-bit values, four maxima added before one dot product,
 // are 7 instructions for 8 but took 7.0 ms for 5.9: the additions share the
@@ -302,8 +305,10 @@ __device__ __forceinline__ QueryTerms query_terms(const FixedQuery& f, uint32_t 
 // cache.
 // With one split, `least` [q][row tile] is the smallest T - error over the tile's
 // rows (0 if negative) and f.upper[q] the smallest T + error, so the selection
-// visits only the tiles that hold candidates.
-template <int J>
+// visits only the tiles that hold candidates. Up to kNarrowColumns that epilogue
+// is in 32-bit differences (NARROW): at 128 columns it was a fifth of the kernel in
+// 64 bits (65,536 rows, 256 queries: 117 us, 107 so).
+template <int J, bool NARROW>
 __global__ void __launch_bounds__(kTileThreads, J == 8 ? 3 : 4)
     fixed_tile_kernel(const uint16_t* __restrict__ rows, uint32_t row_count,
                       const uint16_t* __restrict__ queries, uint32_t batch, uint64_t pitch,
@@ -383,7 +388,13 @@ __global__ void __launch_bounds__(kTileThreads, J == 8 ? 3 : 4)
         __syncthreads();
     }
     const bool single = gridDim.z == 1;
-    FixedTerms terms[8];
+    using Difference = std::conditional_t<NARROW, int, long long>;
+    using Wrapping = std::make_unsigned_t<Difference>;
+    constexpr Difference kMost =
+        static_cast<Difference>(NARROW ? 0x7fffffffll : 0x7fffffffffffffffll);
+    // T - error = 2 M - (query's sum) - under, T + error = 2 M - (query's sum) - over
+    Wrapping under[8];
+    Wrapping over[8];
     if (single) {
         if (tid < kQueries && q0 + tid < batch) {
             query_sums[tid] = query_terms(f, q0 + tid).sum;
@@ -391,7 +402,9 @@ __global__ void __launch_bounds__(kTileThreads, J == 8 ? 3 : 4)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const uint32_t row = row0 + tr + 16 * i;
-            terms[i] = f.terms[min(row, row_count - 1)];
+            const FixedTerms t = f.terms[min(row, row_count - 1)];
+            under[i] = static_cast<Wrapping>(t.sum + t.error);
+            over[i] = static_cast<Wrapping>(t.sum - t.error);
         }
         __syncthreads();
     }
@@ -401,15 +414,16 @@ __global__ void __launch_bounds__(kTileThreads, J == 8 ? 3 : 4)
         if (single) {
             // the 16 threads of a half-warp share the query; lanes past the batch
             // take part in the shuffles with values that are not stored
-            long long low = 0x7fffffffffffffffll;
-            long long high = 0x7fffffffffffffffll;
+            Difference low = kMost;
+            Difference high = kMost;
+            const Wrapping query = static_cast<Wrapping>(query_sums[tq + 8 * j]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const uint32_t row = row0 + tr + 16 * i;
-                const long long t = 2ll * acc[i][j] - query_sums[tq + 8 * j] - terms[i].sum;
+                const Wrapping t = 2 * static_cast<Wrapping>(acc[i][j]) - query;
                 if (row < row_count) {
-                    low = min(low, t - terms[i].error);
-                    high = min(high, t + terms[i].error);
+                    low = min(low, static_cast<Difference>(t - under[i]));
+                    high = min(high, static_cast<Difference>(t - over[i]));
                 }
             }
             for (int o = 8; o > 0; o /= 2) {
@@ -418,8 +432,9 @@ __global__ void __launch_bounds__(kTileThreads, J == 8 ? 3 : 4)
             }
             if (tr == 0 && qq < batch) {
                 least[static_cast<uint64_t>(qq) * gridDim.x + blockIdx.x] =
-                    static_cast<unsigned long long>(max(low, 0ll));
-                atomicMin(f.upper + qq, static_cast<unsigned long long>(max(high, 0ll)));
+                    static_cast<unsigned long long>(max(low, Difference(0)));
+                atomicMin(f.upper + qq,
+                          static_cast<unsigned long long>(max(high, Difference(0))));
             }
         }
         if (qq >= batch) {
@@ -539,7 +554,7 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-template <int J>
+template <int J, bool NARROW>
 void launch_fixed_tiles(const FixedPlan& plan, const uint16_t* rows, uint32_t row_count,
                         const uint16_t* queries, uint32_t batch, uint64_t pitch, uint32_t* sums,
                         unsigned long long* least, const FixedQuery& f, cudaStream_t stream)
@@ -547,13 +562,13 @@ void launch_fixed_tiles(const FixedPlan& plan, const uint16_t* rows, uint32_t ro
     const size_t smem = kStages * (kRows + 8 * J) * kStageStride;
     static std::once_flag once[kMaxDevices];
     std::call_once(once[current_device()], [&] {
-        check_cuda(cudaFuncSetAttribute(fixed_tile_kernel<J>,
+        check_cuda(cudaFuncSetAttribute(fixed_tile_kernel<J, NARROW>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(smem)),
                    "cannot configure the fixed-point scan kernel");
     });
     const dim3 grid((row_count + kRows - 1) / kRows, (batch + 8 * J - 1) / (8 * J), plan.splits);
-    fixed_tile_kernel<J><<<grid, kTileThreads, smem, stream>>>(
+    fixed_tile_kernel<J, NARROW><<<grid, kTileThreads, smem, stream>>>(
         rows, row_count, queries, batch, pitch, plan.columns_per_split, sums, least, f);
     check_cuda(cudaGetLastError(), "cannot launch the fixed-point scan kernel");
 }
@@ -711,11 +726,12 @@ void launch_fixed_scan(const FixedPlan& plan, const uint16_t* rows, uint64_t row
 {
     const uint32_t rc = static_cast<uint32_t>(row_count);
     const uint32_t b = static_cast<uint32_t>(batch);
-    if (plan.queries == 32) {
-        launch_fixed_tiles<4>(plan, rows, rc, queries, b, pitch, sums, least, f, stream);
-    } else {
-        launch_fixed_tiles<8>(plan, rows, rc, queries, b, pitch, sums, least, f, stream);
-    }
+    const bool narrow = f.dim <= kNarrowColumns;
+    const auto launch =
+        plan.queries == 32
+            ? (narrow ? launch_fixed_tiles<4, true> : launch_fixed_tiles<4, false>)
+            : (narrow ? launch_fixed_tiles<8, true> : launch_fixed_tiles<8, false>);
+    launch(plan, rows, rc, queries, b, pitch, sums, least, f, stream);
     const uint32_t tiles = (rc + kRows - 1) / kRows;
     const dim3 grid((rc + kThreads * kSelectRows - 1) / (kThreads * kSelectRows), b);
     if (plan.splits > 1) {
