@@ -421,8 +421,10 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                     __syncwarp();
                     for (int c = lane; c < kColumns; c += 32) {
                         float2 side = make_float2(0.f, -inf);
-                        if (q0 + c < batch) {
-                            const float a = root_of(sq, q0 + c);
+                        const float a = q0 + c < batch ? root_of(sq, q0 + c) : inf;
+                        // a norm the bound does not cover (split_narrow_kernel
+                        // reports it) lists nothing: its sides may be infinite
+                        if (a <= kLargestNorm) {
                             side.x = slope_of(a, sq.rel);
                             if (MODE == Score::filter) {
                                 // tau is the word plus the query's own square
@@ -438,7 +440,8 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                 if (!accumulated()) {
                     break;
                 }
-                // the row's side; a row past the end never passes or is least
+                // the row's side. A row past the end has none: it is masked out
+                // below (the least pass takes whole tiles only)
                 const float square = __fmul_ru(0x1p-21f, __fmul_ru(b, b));
                 const float low = MODE == Score::filter ? __fsub_rd(norm, square)
                                                         : __fadd_ru(norm, square);
@@ -471,7 +474,7 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                             most = fmaxf(most, fmaxf(filter_side(l.x, l.y, b, v[j]),
                                                      filter_side(l.z, l.w, b, v[j + 1])));
                         }
-                        if (!__any_sync(0xffffffffu, most >= low)) {
+                        if (!__any_sync(0xffffffffu, row_ok && most >= low)) {
                             continue;
                         }
                         // the lane's passing columns, taken one per turn
@@ -482,6 +485,7 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                             bits |= filter_side(l.x, l.y, b, v[j]) >= low ? 1u << j : 0u;
                             bits |= filter_side(l.z, l.w, b, v[j + 1]) >= low ? 2u << j : 0u;
                         }
+                        bits = row_ok ? bits : 0u;
                         for (uint32_t mask = __ballot_sync(0xffffffffu, bits != 0u); mask != 0u;
                              mask = __ballot_sync(0xffffffffu, bits != 0u)) {
                             if (bits != 0u) {
@@ -880,6 +884,7 @@ __global__ void __launch_bounds__(kSelectThreads)
     if (lane == 0) {
         if (listed > list_cap || kept > cap || !(a <= kLargestNorm)) {
             atomicOr(error_flag, kCandidateOverflow);
+            kept = 0;  // not settled: the call is answered again
         }
         sq.counts[q] = kept;
     }
