@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -54,8 +55,17 @@ constexpr int kSelectRows = 8;
 constexpr uint32_t kRangeRows = 256;     // rows per block of the range kernel
 // steps of error per column that the binary32 arithmetic of the conversion adds
 constexpr double kColumnSlack = 0x1p-6;
-// up to here T and a row's error (at most a step per column) stay below 2^31
+// The most a row's error can be in steps: half a step per column, the roundings'
+// slack and the two of rounding up, unless w (x - o) left binary32. An index with
+// a row past this is not usable, which the 32-bit epilogue relies on.
+__host__ __device__ constexpr double largest_error(uint64_t dim)
+{
+    return 2.0 * static_cast<double>(dim) + 64.0;
+}
+// up to here T and a row's error stay below 2^31
 constexpr uint64_t kNarrowColumns = 32000;
+static_assert(65535.0 * kNarrowColumns + largest_error(kNarrowColumns) < 2147483647.0,
+              "the narrow epilogue's differences fit 32 bits");
 constexpr uint32_t kPairs = 64;          // row pairs of the quality estimate
 constexpr float kLevels = 65535.f;
 
@@ -166,7 +176,7 @@ __global__ void __launch_bounds__(kThreads)
 // past dim), the sum of their integers and of their errors |w (x - o) - s v|
 // (past the range: of what the clamp cuts off, kept apart).
 // ROWS: index rows (one slice), terms[i] = the sum and the error in steps, rounded
-// up. Else queries (gathered through `columns` when given, validated, the prepared
+// up (error_flag is set where it is past largest_error()). Else queries (gathered through `columns` when given, validated, the prepared
 // binary32 vector written on the way): parts per slice, and the first slice
 // clears the query's words.
 //
@@ -246,6 +256,9 @@ __global__ void __launch_bounds__(kPrepThreads) fixed_vectors_kernel(const Fixed
         return;
     }
     if (ROWS) {
+        if (!(r <= largest_error(v.dim) - 2.0)) {
+            atomicOr(v.error_flag, 1);
+        }
         v.terms[i] = FixedTerms{static_cast<long long>(n),
                                 static_cast<long long>(fmin(ceil(r) + 1.0, 0x1p60))};
     } else {
@@ -588,8 +601,8 @@ uint64_t fixed_pitch(uint64_t dim)
 
 uint64_t fixed_scratch_words(uint64_t dim)
 {
-    // column ranges, then the sampled pairs' distances
-    return round_up(2 * dim, 2) + 2 * kPairs;
+    // column ranges, the sampled pairs' distances, the coarse-row flag
+    return round_up(2 * dim, 2) + 2 * kPairs + 2;
 }
 
 void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, uint64_t dim,
@@ -605,6 +618,8 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     check_cuda(cudaMemsetAsync(high, 0, dim * sizeof(unsigned int), stream),
                "cannot clear column ranges");
     check_cuda(cudaMemsetAsync(step, 0, sizeof(float), stream), "cannot clear the step");
+    check_cuda(cudaMemsetAsync(pairs + kPairs, 0, sizeof(double), stream),
+               "cannot clear the row error flag");
     const uint32_t column_blocks = static_cast<uint32_t>((dim + kThreads - 1) / kThreads);
     column_range_kernel<<<dim3(column_blocks, (rc + kRangeRows - 1) / kRangeRows), kThreads, 0,
                           stream>>>(rows, rc, padded, dim, low, high);
@@ -621,6 +636,7 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     v.pitch = pitch;
     v.slice = pitch;
     v.vector_loads = true;  // rows are padded to 16-byte boundaries
+    v.error_flag = reinterpret_cast<int*>(pairs + kPairs);
     for (uint64_t at = 0; at < row_count; at += 65535) {
         const uint64_t count = std::min<uint64_t>(65535, row_count - at);
         v.source = rows + at * padded;
@@ -635,7 +651,7 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
 bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* terms,
                   uint64_t row_count, const float* device_step, cudaStream_t stream)
 {
-    double pairs[kPairs];
+    double pairs[kPairs + 1];  // the last: the flag
     FixedTerms errors[kPairs];
     float step = 0.f;
     const uint64_t count = std::min<uint64_t>(row_count, kPairs);
@@ -648,9 +664,11 @@ bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* t
     check_cuda(cudaMemcpyAsync(&step, device_step, sizeof(step), cudaMemcpyDeviceToHost, stream),
                "cannot copy the step from the CUDA device");
     check_cuda(cudaStreamSynchronize(stream), "cannot build fixed-point rows");
+    int coarse = 0;
+    std::memcpy(&coarse, pairs + kPairs, sizeof(coarse));
     double distance = 0.0;
-    for (double d : pairs) {
-        distance += d / kPairs;
+    for (uint32_t i = 0; i < kPairs; ++i) {
+        distance += pairs[i] / kPairs;
     }
     double error = 0.0;
     for (uint64_t i = 0; i < count; ++i) {
@@ -658,7 +676,7 @@ bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* t
     }
     // two vectors' errors within 1/512 of a typical distance: rows closer together
     // than that are rare enough for the candidate lists
-    return std::isfinite(step) && std::isfinite(distance) && step >= 0x1p-100f &&
+    return coarse == 0 && std::isfinite(step) && std::isfinite(distance) && step >= 0x1p-100f &&
            1024.0 * error * static_cast<double>(step) <= distance;
 }
 
