@@ -69,3 +69,23 @@ def test_both_epilogues(oracle_module, columns):
     queries = np.zeros((40, columns), np.float32)
     queries[:, :2] = 1.3e38
     _check(oracle_module, rows, queries, None, 200)
+
+
+@pytest.mark.parametrize("count", [(1 << 24) - 256, (1 << 24) - 200, 1 << 24, (1 << 24) + 1])
+def test_most_rows(count):
+    # around the most rows the fixed-point scan takes; past 2^24 the binary32 scan
+    torch = pytest.importorskip("torch")
+    torch.manual_seed(count)
+    rows = torch.rand(count, 4, device="cuda")
+    at = torch.linspace(0, count - 1, 12, dtype=torch.float64).long().cuda()
+    rows[at] += 100 * torch.arange(1, 13, device="cuda")[:, None]
+    queries = (rows[at] + 0.25).contiguous()
+    torch.cuda.synchronize()
+    index = uha.CudaExactL1Index(rows)
+    ws = index.make_query_workspace(12)
+    dist = np.zeros(12)
+    out = np.zeros(12, np.uint64)
+    index.query_device_batch(queries.data_ptr(), 12, out, ws, distances=dist)
+    assert np.array_equal(out, at.cpu().numpy().astype(np.uint64))
+    # 0.25 in each of four columns, up to the rounding of the query
+    np.testing.assert_allclose(dist, 1.0, rtol=4 * 1200 * 2.0 ** -24)

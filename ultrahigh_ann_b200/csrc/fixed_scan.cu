@@ -52,7 +52,8 @@ constexpr uint32_t kStageStride = 144;   // bytes, conflict-free 16-byte reads
 constexpr int kTileThreads = 128;
 constexpr int kStages = 2;
 constexpr int kSelectRows = 8;
-constexpr uint32_t kRangeRows = 256;     // rows per block of the range kernel
+constexpr uint32_t kRangeRows = 256;     // rows per slice of the range kernel
+constexpr uint32_t kRangeSlices = 32768; // and slices of its grid at most (the limit is 65,535)
 // steps of error per column that the binary32 arithmetic of the conversion adds
 constexpr double kColumnSlack = 0x1p-6;
 // The most a row's error can be in steps: half a step per column, the roundings'
@@ -99,8 +100,8 @@ __device__ __forceinline__ double block_total(double v, double* scratch)
 
 // ---------------------------------------------------------------- index side
 
-// Ordered bits of each column's smallest and largest value over the rows of a
-// block's slice.
+// Ordered bits of each column's smallest and largest value. grid (columns, slices
+// of kRangeRows rows); a grid of kRangeSlices takes every so many-th slice.
 __global__ void __launch_bounds__(kThreads)
     column_range_kernel(const float* __restrict__ rows, uint32_t row_count, uint64_t padded,
                         uint64_t dim, unsigned int* __restrict__ low,
@@ -110,15 +111,18 @@ __global__ void __launch_bounds__(kThreads)
     if (j >= dim) {
         return;
     }
-    const uint32_t first = blockIdx.y * kRangeRows;
-    const uint32_t end = min(row_count, first + kRangeRows);
     float a = __int_as_float(0x7f800000);
     float b = -a;
+    for (uint64_t first = uint64_t(blockIdx.y) * kRangeRows; first < row_count;
+         first += uint64_t(gridDim.y) * kRangeRows) {
+        const uint32_t end =
+            static_cast<uint32_t>(min(uint64_t(row_count), first + kRangeRows));
 #pragma unroll 8
-    for (uint32_t r = first; r < end; ++r) {
-        const float x = rows[r * padded + j];
-        a = fminf(a, x);
-        b = fmaxf(b, x);
+        for (uint32_t r = static_cast<uint32_t>(first); r < end; ++r) {
+            const float x = rows[r * padded + j];
+            a = fminf(a, x);
+            b = fmaxf(b, x);
+        }
     }
     atomicMin(low + j, ordered(a));
     atomicMax(high + j, ordered(b));
@@ -621,8 +625,10 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     check_cuda(cudaMemsetAsync(pairs + kPairs, 0, sizeof(double), stream),
                "cannot clear the row error flag");
     const uint32_t column_blocks = static_cast<uint32_t>((dim + kThreads - 1) / kThreads);
-    column_range_kernel<<<dim3(column_blocks, (rc + kRangeRows - 1) / kRangeRows), kThreads, 0,
-                          stream>>>(rows, rc, padded, dim, low, high);
+    const uint32_t slices = std::min((rc + kRangeRows - 1) / kRangeRows, kRangeSlices);
+    column_range_kernel<<<dim3(column_blocks, slices), kThreads, 0, stream>>>(rows, rc, padded,
+                                                                              dim, low, high);
+    check_cuda(cudaGetLastError(), "cannot launch the column range kernel");
     column_offset_kernel<<<static_cast<uint32_t>((pitch + kThreads - 1) / kThreads), kThreads, 0,
                            stream>>>(low, high, dim, pitch, weights, offsets,
                                      reinterpret_cast<unsigned int*>(step));
