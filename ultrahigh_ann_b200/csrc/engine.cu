@@ -1411,10 +1411,11 @@ uint64_t enqueue_lowp_candidates(const BatchContext& c, uint64_t n, const uha::L
 const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
 {
     std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    uha::SplitRows& sp = index->split;
-    if (sp.ready) {
-        return sp.usable ? &sp : nullptr;
+    if (index->split.ready) {
+        return index->split.usable ? &index->split : nullptr;
     }
+    uha::SplitRows sp;  // published only once it is built
+    sp.ready = true;
     const bool hierarchical = index->kind == IndexKind::hierarchical;
     sp.pitch = uha::split_pitch(index->scan_dim);
     const uint64_t bytes = checked_mul(
@@ -1422,8 +1423,8 @@ const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
         "split rows");
     if (!sp.data.try_allocate(bytes) || !sp.norms.try_allocate(index->rows) ||
         !sp.roots.try_allocate(index->rows + 1) || !sp.centre.try_allocate(sp.pitch)) {
-        sp = uha::SplitRows{};
-        sp.ready = true;
+        index->split = uha::SplitRows{};
+        index->split.ready = true;
         return nullptr;
     }
     // the word past the roots receives the largest of them
@@ -1455,12 +1456,12 @@ const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
         sp.scale = std::ldexp(1.f, -std::clamp(std::ilogb(root), -126, 126));
         root = split();
     }
-    sp.ready = true;
     sp.usable = root <= uha::split_largest_norm();
     if (!sp.usable) {
         sp.data.release();
     }
-    return sp.usable ? &sp : nullptr;
+    index->split = std::move(sp);
+    return index->split.usable ? &index->split : nullptr;
 }
 
 // The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use on
@@ -1469,9 +1470,9 @@ const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
 const uha::RowBits* row_bits(const uha_index* index, cudaStream_t stream)
 {
     std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    uha::RowBits& rb = index->bits;
-    if (!rb.ready) {
+    if (!index->bits.ready) {
         const uint64_t p = index->projection_dimension;
+        uha::RowBits rb;  // published only once it is built
         rb.ready = true;
         rb.usable = rb.boundaries.try_allocate(uha::bits_boundaries(p)) &&
                     rb.data.try_allocate(uha::bits_bytes(index->rows, p));
@@ -1482,8 +1483,9 @@ const uha::RowBits* row_bits(const uha_index* index, cudaStream_t stream)
         } else {
             rb.boundaries.release();
         }
+        index->bits = std::move(rb);
     }
-    return rb.usable ? &rb : nullptr;
+    return index->bits.usable ? &index->bits : nullptr;
 }
 
 // The bitmap form of this batch's median scan (everything it needs allocated
@@ -1572,33 +1574,33 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
 const uha::FixedRows* fixed_rows(const uha_index* index, cudaStream_t stream)
 {
     std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    uha::FixedRows& fx = index->fixed;
-    if (fx.ready) {
-        return fx.usable ? &fx : nullptr;
+    if (index->fixed.ready) {
+        return index->fixed.usable ? &index->fixed : nullptr;
     }
+    uha::FixedRows fx;  // published only once it is built
     fx.ready = true;
     fx.pitch = uha::fixed_pitch(index->scan_dim);
     // in units of 16 bytes
     const uint64_t head = index->rows + (fx.pitch + 4) / 4;
     const uint64_t scratch = (uha::fixed_scratch_words(index->scan_dim) + 3) / 4;
     const uint64_t values = checked_mul(index->rows, fx.pitch / 8, "fixed-point rows");
-    if (!fx.store.try_allocate(head + scratch + values)) {
-        return nullptr;
+    if (fx.store.try_allocate(head + scratch + values)) {
+        float* offsets = reinterpret_cast<float*>(fx.store.get() + index->rows);
+        unsigned int* words = reinterpret_cast<unsigned int*>(fx.store.get() + head);
+        uint16_t* data = reinterpret_cast<uint16_t*>(fx.store.get() + head + scratch);
+        fx.offsets = offsets;
+        fx.data = data;
+        uha::launch_fixed_rows(index->scan_rows.get(), index->rows, index->padded_dim,
+                               index->scan_dim, index->weights64.get(), data, fx.pitch, offsets,
+                               offsets + fx.pitch, fx.store.get(), words, stream);
+        fx.usable = uha::fixed_usable(words, index->scan_dim, fx.store.get(), index->rows,
+                                      offsets + fx.pitch, stream);
+        if (!fx.usable) {
+            fx.store.release();
+        }
     }
-    float* offsets = reinterpret_cast<float*>(fx.store.get() + index->rows);
-    unsigned int* words = reinterpret_cast<unsigned int*>(fx.store.get() + head);
-    uint16_t* data = reinterpret_cast<uint16_t*>(fx.store.get() + head + scratch);
-    fx.offsets = offsets;
-    fx.data = data;
-    uha::launch_fixed_rows(index->scan_rows.get(), index->rows, index->padded_dim,
-                           index->scan_dim, index->weights64.get(), data, fx.pitch, offsets,
-                           offsets + fx.pitch, fx.store.get(), words, stream);
-    fx.usable = uha::fixed_usable(words, index->scan_dim, fx.store.get(), index->rows,
-                                  offsets + fx.pitch, stream);
-    if (!fx.usable) {
-        fx.store.release();
-    }
-    return fx.usable ? &fx : nullptr;
+    index->fixed = std::move(fx);
+    return index->fixed.usable ? &index->fixed : nullptr;
 }
 
 // The fixed-point scan of this batch (everything it needs allocated here), or
