@@ -201,9 +201,11 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
         rep.kernel = 2;
         rep.tile_queries = static_cast<uint32_t>(best.lowp_plan.bn);
         rep.splits = best.lowp_plan.splits;
-    } else if (const uha::SplitRows* sp = !ws->split_disabled && split_shape(index, strategy, batch)
-                                              ? split_rows(index, stream)
-                                              : nullptr;
+    } else if (const uha::SplitRows* sp =
+                   !ws->split_disabled && split_shape(index, strategy, batch) &&
+                           (!ws->emulated_replay || index->kind == IndexKind::hierarchical)
+                       ? split_rows(index, stream)
+                       : nullptr;
                sp != nullptr) {
         // the certified split scan: its tile widths and column splits
         std::vector<uha::SplitPlan> cands =

@@ -27,7 +27,6 @@
 #include <cmath>
 #include <map>
 #include <mutex>
-#include <type_traits>
 #include <utility>
 
 namespace uha {
@@ -2196,24 +2195,21 @@ __global__ void __launch_bounds__(kFinalizeThreads)
 // The candidate lists of the split and fixed-point scans. grid = (parts, batch):
 // each block sums its part of the columns for every candidate of the query
 // (usually one or two), from the original binary32 rows; the query's last block
-// adds the parts in order and settles the query, in binary64 or, with
-// kEmulated, without FP64 instructions. Bound: memory (a candidate's row and
+// adds the parts in order and settles the query in binary64. Bound: memory (a candidate's row and
 // the query); the parts spread a small batch over the chip (64 queries x
 // 60,660 columns: 58 us with one block per query, 19 us with 16). A query
 // without candidates (its list overflowed, so the call is answered again) gets
 // row 0.
-template <bool kEmulated>
 __global__ void __launch_bounds__(kFinalizeThreads)
-    settle_kernel(Bound64 bound64, Bound bound32, ReplayInputs in,
+    settle_kernel(Bound64 bound, ReplayInputs in,
                   const uint32_t* __restrict__ candidates,
                   const uint32_t* __restrict__ counts, uint32_t row_count, double* sums,
                   uint32_t* done, Result* results, double* exact_distances,
                   uint32_t* replay_count)
 {
-    using T = std::conditional_t<kEmulated, float, double>;
     static_assert(kSplitCandidates <= kMaxCandidates, "candidate lists fit the settlement");
-    __shared__ T scratch[kFinalizeThreads / 32];
-    __shared__ T dist[kSplitCandidates];
+    __shared__ double scratch[kFinalizeThreads / 32];
+    __shared__ double dist[kSplitCandidates];
     __shared__ uint32_t cand[kSplitCandidates];
     __shared__ bool is_last;
     const uint32_t q = blockIdx.y;
@@ -2230,16 +2226,13 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     const uint64_t width = (in.padded_dim / 4 + parts - 1) / parts * 4;
     const uint64_t begin = min(in.padded_dim, blockIdx.x * width);
     const uint64_t end = min(in.padded_dim, begin + width);
-    // parts[q][candidate][part]; the emulated form keeps binary32 sums there
-    T* mine = reinterpret_cast<T*>(sums) +
-              static_cast<uint64_t>(q) * kSplitCandidates * parts;
+    // parts[q][candidate][part]
+    double* mine = sums + static_cast<uint64_t>(q) * kSplitCandidates * parts;
     for (uint32_t i = 0; i < k; ++i) {
         const uint32_t row = candidates[static_cast<uint64_t>(q) * kSplitCandidates + i];
         const float* rrow = in.rows + static_cast<uint64_t>(row) * in.padded_dim;
-        T d;
-        if constexpr (kEmulated) {
-            d = block_l2_32(qrow + begin, rrow + begin, end - begin, scratch);
-        } else if (in.op == ReplayOp::l2_sequential) {
+        double d;
+        if (in.op == ReplayOp::l2_sequential) {
             d = block_l2_64(qrow + begin, rrow + begin, end - begin, scratch);
         } else {
             const bool weighted = in.op == ReplayOp::l1_weighted_sequential;
@@ -2262,22 +2255,16 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     }
     __threadfence();
     for (uint32_t i = threadIdx.x; i < k; i += kFinalizeThreads) {
-        T d = static_cast<volatile T*>(mine)[i * parts];
+        double d = static_cast<volatile double*>(mine)[i * parts];
         for (uint32_t p = 1; p < parts; ++p) {
-            d = kEmulated ? __fadd_rn(d, static_cast<volatile T*>(mine)[i * parts + p])
-                          : d + static_cast<volatile T*>(mine)[i * parts + p];
+            d += static_cast<volatile double*>(mine)[i * parts + p];
         }
         dist[i] = d;
         cand[i] = candidates[static_cast<uint64_t>(q) * kSplitCandidates + i];
     }
     __syncthreads();
-    if constexpr (kEmulated) {
-        settle32(bound32, in, qrow, cand, dist, k, row_count, q, results + q,
-                 exact_distances + q, replay_count);
-    } else {
-        settle64(bound64, in, qrow, cand, dist, k, row_count, results + q,
-                 exact_distances + q, replay_count);
-    }
+    settle64(bound, in, qrow, cand, dist, k, row_count, results + q, exact_distances + q,
+             replay_count);
 }
 
 // ------------------------------------------ the persistent multi-index batch
@@ -2772,7 +2759,7 @@ uint64_t settle_sums(uint64_t batch)
     return kSplitCandidates * std::max<uint64_t>(kSettleBlocks, batch);
 }
 
-void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32_t* candidates,
+void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
                    const uint32_t* counts, uint32_t batch, uint32_t rows, double* sums,
                    uint32_t* done, Result* results, double* exact_distances,
                    uint32_t* replay_count, cudaStream_t stream)
@@ -2782,10 +2769,8 @@ void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32
     }
     // short rows are one part
     const uint32_t parts = in.padded_dim >= 8192 ? settle_parts(batch) : 1;
-    const auto kernel = in.emulated ? settle_kernel<true> : settle_kernel<false>;
-    kernel<<<dim3(parts, batch), kFinalizeThreads, 0, stream>>>(
-        bound64, bound32, in, candidates, counts, rows, sums, done, results, exact_distances,
-        replay_count);
+    settle_kernel<<<dim3(parts, batch), kFinalizeThreads, 0, stream>>>(
+        bound, in, candidates, counts, rows, sums, done, results, exact_distances, replay_count);
     check_cuda(cudaGetLastError(), "cannot launch the settlement kernel");
 }
 

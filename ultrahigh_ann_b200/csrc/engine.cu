@@ -1723,7 +1723,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
     in.padded_dim = index->padded_dim;
     in.weights64 = index->weights64.get();
     const uint32_t depth = uha::settle_depth(index->padded_dim);
-    uha::launch_settle(uha::make_bound64(depth, index->scan_dim), uha::Bound{}, in,
+    uha::launch_settle(uha::make_bound64(depth, index->scan_dim), in,
                        ws->split_candidates.get(), v.counts, static_cast<uint32_t>(n),
                        static_cast<uint32_t>(index->rows), ws->split_sums.get(), v.done,
                        results, exact, ws->counters.get(), stream);
@@ -1732,14 +1732,16 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
 
 // The split scan of this batch, or false when it takes the binary32 scan: the
 // direct strategy on L2 indexes, batches past the streaming scan's, whose
-// caller answers a call again when a candidate list overflows. Everything the
-// batch needs is allocated here.
+// caller answers a call again when a candidate list overflows, unless the
+// settlement has to do without FP64 instructions (the norms, roots and sums of
+// the split scan are binary64). Everything the batch needs is allocated here.
 bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** rows,
                    uha::SplitPlan* plan)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
     if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+        (ws->emulated_replay && index->kind != IndexKind::hierarchical) ||
         !split_shape(index, c.strategy, n)) {
         return false;
     }
@@ -2022,13 +2024,9 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     in.queries = ws->prepared.get();
     in.dim = index->scan_dim;
     in.padded_dim = index->padded_dim;
-    if (ws->emulated_replay) {
-        set_emulated(in, index);
-    }
     const uint32_t depth = uha::settle_depth(index->padded_dim);
-    uha::launch_settle(uha::make_bound64(depth, index->scan_dim),
-                       make_bound(depth, index->scan_dim, 2), in, ws->split_candidates.get(),
-                       v.counts, b, static_cast<uint32_t>(index->rows), ws->split_sums.get(),
+    uha::launch_settle(uha::make_bound64(depth, index->scan_dim), in,
+                       ws->split_candidates.get(), v.counts, b, static_cast<uint32_t>(index->rows), ws->split_sums.get(),
                        v.done, results, exact, ws->counters.get(), stream);
     return launches + 1;
 }

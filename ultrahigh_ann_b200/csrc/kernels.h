@@ -525,11 +525,10 @@ void launch_fixed_scan(const FixedPlan& plan, const uint16_t* rows, uint64_t row
                        cudaStream_t stream);
 
 // Certified argmin of each query over its listed candidates, from the original
-// binary32 rows (exact and flat ops; in.emulated, L2 only: bound32, else
-// bound64, both of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
+// binary32 rows (exact and flat ops; the bound of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
 uint32_t settle_depth(uint64_t padded_dim);
 uint64_t settle_sums(uint64_t batch);
-void launch_settle(Bound64 bound64, Bound bound32, ReplayInputs in, const uint32_t* candidates,
+void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
                    const uint32_t* counts, uint32_t batch, uint32_t rows, double* sums,
                    uint32_t* done, Result* results, double* exact_distances,
                    uint32_t* replay_count, cudaStream_t stream);
