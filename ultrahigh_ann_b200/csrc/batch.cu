@@ -345,6 +345,13 @@ struct uha_batch {
         uint64_t offset = 0;
         bool trivial = false;
         cudaEvent_t join = nullptr;
+        // The workspace that answers the queries the captured scans leave open
+        // (the graph reads and writes `ws`, which such a call would change).
+        uha_workspace* again = nullptr;
+        // Whether the graph holds the estimating scans, and else the runs until it
+        // does again (0: never).
+        bool estimates = true;
+        uint32_t wait = 0;
         uha_tune_report tuning{};
     };
     int device = 0;
@@ -384,8 +391,10 @@ struct uha_batch {
             if (p.join != nullptr) {
                 cudaEventDestroy(p.join);
             }
-            if (p.ws != nullptr) {
-                uha_workspace_destroy(p.ws);
+            for (uha_workspace* ws : {p.ws, p.again}) {
+                if (ws != nullptr) {
+                    uha_workspace_destroy(ws);
+                }
             }
         }
         for (cudaEvent_t e : {fork, start, stop}) {
@@ -416,6 +425,8 @@ uint64_t enqueue_pair(uha_batch::Pair& p)
                "cannot clear query counters");
     BatchContext ctx{p.index, ws, p.strategy, true};
     ctx.filter_candidates = true;
+    ctx.estimates = p.estimates;
+    ctx.refine_every = !p.estimates;
     const uint64_t launches =
         enqueue_batch(ctx, ws->raw_queries.get(), p.count, ws->call_results.get(),
                       ws->call_exact.get(), false, nullptr, nullptr);
@@ -480,6 +491,123 @@ void build_persistent(uha_batch* batch)
                 "the persistent batch kernel cannot be resident with its shared memory");
     }
     batch->persistent = true;
+}
+
+// Captures the batch's graph: fork every pair from the batch stream, join back (or
+// the persistent kernel and the result copies). The former graph, if there is one,
+// is replaced once the new one is there.
+void capture_batch(uha_batch* batch)
+{
+    check_cuda(cudaStreamBeginCapture(batch->stream, cudaStreamCaptureModeThreadLocal),
+               "cannot capture the batch");
+    uint64_t launches = 0;
+    try {
+        if (batch->persistent) {
+            uha::launch_persistent_batch(*batch->params, batch->grid, batch->stream);
+            launches = uha::kPersistentKernels;
+            for (uha_batch::Pair& p : batch->pairs) {
+                if (p.trivial) {
+                    continue;
+                }
+                uha_workspace* ws = p.ws;
+                check_cuda(cudaMemcpyAsync(ws->host_results.get(), ws->call_results.get(),
+                                           p.count * sizeof(uha::Result),
+                                           cudaMemcpyDeviceToHost, batch->stream),
+                           "cannot copy query results from the CUDA device");
+                check_cuda(cudaMemcpyAsync(ws->host_exact.get(), ws->call_exact.get(),
+                                           p.count * sizeof(double), cudaMemcpyDeviceToHost,
+                                           batch->stream),
+                           "cannot copy query distances from the CUDA device");
+                check_cuda(cudaMemcpyAsync(ws->host_counters.get(), ws->counters.get(),
+                                           ws->counters.bytes(), cudaMemcpyDeviceToHost,
+                                           batch->stream),
+                           "cannot copy query counters from the CUDA device");
+            }
+            check_cuda(cudaMemcpyAsync(batch->host_status.get(), batch->params->plan.status,
+                                       sizeof(int), cudaMemcpyDeviceToHost, batch->stream),
+                       "cannot copy the persistent batch status");
+            check_cuda(cudaMemcpyAsync(batch->host_clock.get(), batch->clock.get(),
+                                       batch->clock.bytes(), cudaMemcpyDeviceToHost,
+                                       batch->stream),
+                       "cannot copy the persistent batch stage clock");
+        }
+        check_cuda(cudaEventRecord(batch->fork, batch->stream), "event");
+        for (uha_batch::Pair& p : batch->pairs) {
+            if (p.trivial || batch->persistent) {
+                continue;
+            }
+            check_cuda(cudaStreamWaitEvent(p.ws->stream, batch->fork, 0), "event");
+            launches += enqueue_pair(p);
+            check_cuda(cudaEventRecord(p.join, p.ws->stream), "event");
+            check_cuda(cudaStreamWaitEvent(batch->stream, p.join, 0), "event");
+        }
+    } catch (...) {
+        cudaGraph_t g = nullptr;
+        cudaStreamEndCapture(batch->stream, &g);
+        if (g != nullptr) {
+            cudaGraphDestroy(g);
+        }
+        throw;
+    }
+    cudaGraph_t graph = nullptr;
+    check_cuda(cudaStreamEndCapture(batch->stream, &graph), "cannot capture the batch");
+    cudaGraphExec_t exec = nullptr;
+    size_t nodes = 0;
+    const cudaError_t counted = cudaGraphGetNodes(graph, nullptr, &nodes);
+    const cudaError_t ready = cudaGraphInstantiate(&exec, graph, 0);
+    if (ready != cudaSuccess || counted != cudaSuccess) {
+        if (exec != nullptr) {
+            cudaGraphExecDestroy(exec);
+        }
+        cudaGraphDestroy(graph);
+        check_cuda(ready, "cannot instantiate the batch graph");
+        check_cuda(counted, "cannot inspect the batch graph");
+    }
+    if (batch->exec != nullptr) {
+        cudaGraphExecDestroy(batch->exec);
+        cudaGraphDestroy(batch->graph);
+    }
+    batch->graph = graph;
+    batch->exec = exec;
+    batch->graph_nodes = nodes;
+    batch->launches = launches;
+}
+
+// Runs that a pair stays on the binary32 scans after one whose estimates left over
+// half of its queries open; both captures are paid back by then.
+constexpr uint32_t kPairWait = 64;
+
+// Answers the queries that a run left open (all of the pair's where a precision
+// strategy's list overflowed) in the pair's second workspace, into the host mirrors
+// of its results; returns the count of open queries.
+uint64_t answer_pair(uha_batch::Pair& p)
+{
+    uha_workspace* ws = p.ws;
+    std::vector<uint64_t> open = open_queries(ws->host_results.get(), p.count);
+    const uint64_t left = open.size();
+    if (open.empty()) {
+        for (uint64_t q = 0; q < p.count; ++q) {
+            open.push_back(q);
+        }
+    }
+    if (p.again == nullptr || p.again->max_batch < open.size()) {
+        if (p.again != nullptr) {
+            uha_workspace_destroy(p.again);
+            p.again = nullptr;
+        }
+        const uha_status status = uha_workspace_create(p.index, open.size(), &p.again);
+        if (status != UHA_OK) {
+            fail(status, uha_last_error());
+        }
+        p.again->candidates_per_query = ws->candidates_per_query;
+    }
+    const uha_query_stats more =
+        answer_open(p.index, p.again, ws->raw_queries.get(), open, open.size(), p.strategy, true,
+                    ws->host_results.get(), ws->host_exact.get());
+    uint32_t* words = ws->host_counters.get();
+    words[0] = (left != 0 ? words[0] : 0u) + static_cast<uint32_t>(more.replayed_queries);
+    words[1] &= ~static_cast<uint32_t>(uha::kCandidateOverflow);
+    return left;
 }
 
 uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_counts,
@@ -547,66 +675,7 @@ uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_c
         if (persistent) {
             build_persistent(batch.get());
         }
-        // capture: fork every pair from the batch stream, join back (or the
-        // persistent kernel and the result copies)
-        check_cuda(cudaStreamBeginCapture(batch->stream, cudaStreamCaptureModeThreadLocal),
-                   "cannot capture the batch");
-        uint64_t launches = 0;
-        try {
-            if (batch->persistent) {
-                uha::launch_persistent_batch(*batch->params, batch->grid, batch->stream);
-                launches = uha::kPersistentKernels;
-                for (uha_batch::Pair& p : batch->pairs) {
-                    if (p.trivial) {
-                        continue;
-                    }
-                    uha_workspace* ws = p.ws;
-                    check_cuda(cudaMemcpyAsync(ws->host_results.get(), ws->call_results.get(),
-                                               p.count * sizeof(uha::Result),
-                                               cudaMemcpyDeviceToHost, batch->stream),
-                               "cannot copy query results from the CUDA device");
-                    check_cuda(cudaMemcpyAsync(ws->host_exact.get(), ws->call_exact.get(),
-                                               p.count * sizeof(double), cudaMemcpyDeviceToHost,
-                                               batch->stream),
-                               "cannot copy query distances from the CUDA device");
-                    check_cuda(cudaMemcpyAsync(ws->host_counters.get(), ws->counters.get(),
-                                               ws->counters.bytes(), cudaMemcpyDeviceToHost,
-                                               batch->stream),
-                               "cannot copy query counters from the CUDA device");
-                }
-                check_cuda(cudaMemcpyAsync(batch->host_status.get(), batch->params->plan.status,
-                                           sizeof(int), cudaMemcpyDeviceToHost, batch->stream),
-                           "cannot copy the persistent batch status");
-                check_cuda(cudaMemcpyAsync(batch->host_clock.get(), batch->clock.get(),
-                                           batch->clock.bytes(), cudaMemcpyDeviceToHost,
-                                           batch->stream),
-                           "cannot copy the persistent batch stage clock");
-            }
-            check_cuda(cudaEventRecord(batch->fork, batch->stream), "event");
-            for (uha_batch::Pair& p : batch->pairs) {
-                if (p.trivial || batch->persistent) {
-                    continue;
-                }
-                check_cuda(cudaStreamWaitEvent(p.ws->stream, batch->fork, 0), "event");
-                launches += enqueue_pair(p);
-                check_cuda(cudaEventRecord(p.join, p.ws->stream), "event");
-                check_cuda(cudaStreamWaitEvent(batch->stream, p.join, 0), "event");
-            }
-        } catch (...) {
-            cudaGraph_t g = nullptr;
-            cudaStreamEndCapture(batch->stream, &g);
-            if (g != nullptr) {
-                cudaGraphDestroy(g);
-            }
-            throw;
-        }
-        check_cuda(cudaStreamEndCapture(batch->stream, &batch->graph),
-                   "cannot capture the batch");
-        check_cuda(cudaGraphInstantiate(&batch->exec, batch->graph, 0),
-                   "cannot instantiate the batch graph");
-        check_cuda(cudaGraphGetNodes(batch->graph, nullptr, &batch->graph_nodes),
-                   "cannot inspect the batch graph");
-        batch->launches = launches;
+        capture_batch(batch.get());
         *out = batch.release();
     });
 }
@@ -683,6 +752,7 @@ extern "C" uha_status uha_batch_run(uha_batch* batch, const float* const* querie
         st.graph_nodes = batch->graph_nodes;
         st.kernel_launches = batch->launches;
         st.device_ms = ms;
+        std::vector<uha_batch::Pair*> changed;
         for (uha_batch::Pair& p : batch->pairs) {
             uint64_t* idx = out_indices + p.offset;
             double* dist = out_distances != nullptr ? out_distances + p.offset : nullptr;
@@ -690,31 +760,39 @@ extern "C" uha_status uha_batch_run(uha_batch* batch, const float* const* querie
                 fill_trivial(p.count, idx, dist);
                 continue;
             }
-            if ((p.ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u) {
-                // a candidate list overflowed: this pair again, without the
-                // list, in a workspace of its own (the graph reads and writes
-                // the pair's buffers, which such a run would replace)
-                uha_workspace* again = nullptr;
-                uha_status status = uha_workspace_create(p.index, p.count, &again);
-                if (status == UHA_OK) {
-                    again->filter_disabled = true;
-                    again->candidates_per_query = p.ws->candidates_per_query;
-                    status = uha_query(p.index, again, p.ws->raw_queries.get(), p.count, 1,
-                                       p.strategy, idx, dist);
-                    st.replayed_queries += again->last.replayed_queries;
-                }
-                const std::string message = status != UHA_OK ? uha_last_error() : "";
-                uha_workspace_destroy(again);
-                if (status != UHA_OK) {
-                    fail(status, message);
-                }
-                continue;
+            if ((p.ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u &&
+                2 * answer_pair(p) > p.count) {
+                p.estimates = false;
+                p.wait = kPairWait;
+                changed.push_back(&p);
+            } else if (!p.estimates && p.wait != 0 && --p.wait == 0) {
+                p.estimates = true;
+                changed.push_back(&p);
             }
             finish_call(p.index, p.ws, p.count, p.ws->host_results.get(),
                         p.ws->host_exact.get(), idx, dist);
             st.replayed_queries += p.ws->last.replayed_queries;
         }
         batch->last = st;
+        if (changed.empty()) {
+            return;
+        }
+        try {
+            // buffers reach their sizes before the capture, as at the start
+            for (uha_batch::Pair* p : changed) {
+                enqueue_pair(*p);
+                check_cuda(cudaStreamSynchronize(p->ws->stream), "CUDA batch failed");
+            }
+            capture_batch(batch);
+        } catch (const uha::Error&) {
+            // the former graph stays (its buffers are not the other scans')
+            uha::clear_stale_cuda_error();
+            for (uha_batch::Pair* p : changed) {
+                cudaStreamSynchronize(p->ws->stream);
+                p->estimates = !p->estimates;
+                p->wait = 0;
+            }
+        }
     });
 }
 

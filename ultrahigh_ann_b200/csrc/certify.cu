@@ -639,9 +639,13 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const double* y = y64 + static_cast<uint64_t>(q) * p;
-    const uint32_t k = counts != nullptr ? min(counts[q], stride) : stride;
+    uint32_t k = stride;
+    if (counts != nullptr) {
+        // an overflowed list is not settled: best_row stays kOpenQuery
+        k = counts[q] <= stride ? counts[q] : 0u;
+    }
     double best = __longlong_as_double(0x7ff0000000000000ll);
-    uint32_t best_row = 0xffffffffu;
+    uint32_t best_row = kOpenQuery;
     for (uint32_t i = warp; i < k; i += warps) {
         const uint32_t row = candidates[static_cast<uint64_t>(q) * stride + i];
         if (row == 0xffffffffu) {
@@ -2198,8 +2202,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
 // adds the parts in order and settles the query in binary64. Bound: memory (a candidate's row and
 // the query); the parts spread a small batch over the chip (64 queries x
 // 60,660 columns: 58 us with one block per query, 19 us with 16). A query
-// without candidates (its list overflowed, so the call is answered again) gets
-// row 0.
+// whose list overflowed, or is empty, stays open.
 __global__ void __launch_bounds__(kFinalizeThreads)
     settle_kernel(Bound64 bound, ReplayInputs in,
                   const uint32_t* __restrict__ candidates,
@@ -2214,10 +2217,10 @@ __global__ void __launch_bounds__(kFinalizeThreads)
     __shared__ bool is_last;
     const uint32_t q = blockIdx.y;
     const uint32_t parts = gridDim.x;
-    const uint32_t k = min(counts[q], kSplitCandidates);
-    if (k == 0) {
+    const uint32_t k = counts[q];
+    if (k == 0 || k > kSplitCandidates) {
         if (threadIdx.x == 0 && blockIdx.x == 0) {
-            results[q] = Result{0, 0.f};
+            results[q] = Result{kOpenQuery, 0.f};
             exact_distances[q] = __longlong_as_double(0x7ff8000000000000ll);
         }
         return;

@@ -1494,7 +1494,7 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
-    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+    if (!c.estimates || ws->split_disabled ||
         index->kind != IndexKind::hierarchical || index->metric != UHA_L1 ||
         !uha::bits_applies(index->rows, index->projection_dimension) ||
         !uha::bits_batch(index->projection_dimension, n)) {
@@ -1605,8 +1605,8 @@ const uha::FixedRows* fixed_rows(const uha_index* index, cudaStream_t stream)
 
 // The fixed-point scan of this batch (everything it needs allocated here), or
 // null when it takes the binary32 scan: every direct L1 batch past the streaming
-// scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers a
-// call again when a candidate list overflows. An index's first such call also
+// scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers the
+// queries it leaves open. An index's first such call also
 // builds the rows (7,028 x 60,660: 0.8 ms; 65,536 x 128: 0.1 ms and an allocation
 // of 0.35 ms), which the large calls win back at once.
 struct FixedBuffers {
@@ -1621,7 +1621,7 @@ const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::Fixe
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
-    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+    if (!c.estimates || ws->split_disabled ||
         ws->emulated_replay || index->kind == IndexKind::hierarchical ||
         index->metric != UHA_L1 || precision_strategy(c.strategy) || n <= 8 || n > 65535 ||
         index->rows < 2 || index->rows > (1u << 24)) {
@@ -1732,7 +1732,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
 
 // The split scan of this batch, or false when it takes the binary32 scan: the
 // direct strategy on L2 indexes, batches past the streaming scan's, whose
-// caller answers a call again when a candidate list overflows, unless the
+// caller answers the queries it leaves open, unless the
 // settlement has to do without FP64 instructions (the norms, roots and sums of
 // the split scan are binary64). Everything the batch needs is allocated here.
 bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** rows,
@@ -1740,7 +1740,7 @@ bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** row
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
-    if (!c.filter_candidates || ws->filter_disabled || ws->split_disabled ||
+    if (!c.estimates || ws->split_disabled ||
         (ws->emulated_replay && index->kind != IndexKind::hierarchical) ||
         !split_shape(index, c.strategy, n)) {
         return false;
@@ -2288,10 +2288,9 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     ++launches;
     if (hierarchical && c.want_distances) {
         // reported distances of a hierarchy: the reference's binary64 value of
-        // each selected row (a call answered again reports them all, like the
-        // listing scans it stands in for)
+        // each selected row
         uha::launch_refine_winners(in, bound, results, static_cast<uint32_t>(n), exact,
-                                   stream, ws->filter_disabled);
+                                   stream, c.refine_every);
         ++launches;
     }
     return launches;
@@ -2347,6 +2346,62 @@ void finish_call(const uha_index* index, uha_workspace* ws, uint64_t n,
     const uint32_t replayed = ws->host_counters.get()[0];
     ws->last.replayed_queries = replayed;
     ws->last.certified_queries = n - std::min<uint64_t>(n, replayed);
+}
+
+std::vector<uint64_t> open_queries(const uha::Result* results, uint64_t n)
+{
+    std::vector<uint64_t> open;
+    for (uint64_t q = 0; q < n; ++q) {
+        if (results[q].row == uha::kOpenQuery) {
+            open.push_back(q);
+        }
+    }
+    return open;
+}
+
+uha_query_stats answer_open(const uha_index* index, uha_workspace* ws, const float* queries,
+                            const std::vector<uint64_t>& open, uint64_t batch,
+                            uha_strategy strategy, bool want_distances, uha::Result* results,
+                            double* exact)
+{
+    const uint64_t d = index->dimension;
+    const uint64_t most = std::min<uint64_t>({batch, ws->max_batch, open.size()});
+    std::vector<uint64_t> rows(most);
+    std::vector<double> distances(want_distances ? most : 0);
+    uha_query_stats total{};
+    for (uint64_t at = 0; at < open.size(); at += most) {
+        const uint64_t count = std::min<uint64_t>(most, open.size() - at);
+        // runs of consecutive queries, one copy each
+        for (uint64_t i = 0, run = 0; i < count; i += run) {
+            run = 1;
+            while (i + run < count && open[at + i + run] == open[at + i] + run) {
+                ++run;
+            }
+            check_cuda(cudaMemcpyAsync(ws->raw_queries.get() + i * d,
+                                       queries + open[at + i] * d, run * d * sizeof(float),
+                                       cudaMemcpyDefault, ws->stream),
+                       "cannot copy queries to the CUDA device");
+        }
+        ws->filter_disabled = true;
+        const uha_status status =
+            uha_query_many(index, ws, ws->raw_queries.get(), count, count, 1, strategy,
+                           rows.data(), want_distances ? distances.data() : nullptr);
+        ws->filter_disabled = false;
+        if (status != UHA_OK) {
+            fail(status, uha_last_error());
+        }
+        for (uint64_t i = 0; i < count; ++i) {
+            const uint64_t q = open[at + i];
+            results[q].row = static_cast<uint32_t>(rows[i]);
+            exact[q] = want_distances ? distances[i] : 0.0;
+        }
+        total.kernel_launches += ws->last.kernel_launches;
+        total.replayed_queries += ws->last.replayed_queries;
+        total.scan_ms += ws->last.scan_ms;
+        total.timed_scans += ws->last.timed_scans;
+        total.device_ms += ws->last.device_ms;
+    }
+    return total;
 }
 
 void validate_query_call(const uha_index* index, uha_workspace* ws,
@@ -2449,6 +2504,8 @@ void prepare_pipeline(const uha_index* index, uha_workspace* ws, uha_strategy st
 // eighth of the columns the scattered reads cost as much as the copy, and past
 // kGatherBytes the pinned staging would outgrow its use.
 constexpr uint64_t kGatherBytes = 64ull << 20;
+// calls in a row without the estimating scans at most (uha_workspace)
+constexpr uint32_t kLongestWait = 64;
 
 bool gather_on_host(const uha_index* index, uint64_t n)
 {
@@ -2470,6 +2527,17 @@ void gather_queries(const uha_index* index, uha_workspace* ws, const float* quer
             to[i] = from[columns[i]];
         }
     }
+}
+
+// Calls that the estimating scans may answer: direct batches past the streaming
+// scan's 8 queries, and of L1 hierarchies (which have no streaming scan) any.
+bool estimates_serve(const uha_index* index, uha_strategy strategy, uint64_t batch)
+{
+    if (index->metric == UHA_L1) {
+        return !precision_strategy(strategy) &&
+               (batch > 8 || index->kind == IndexKind::hierarchical);
+    }
+    return strategy == UHA_DIRECT && batch > 8;
 }
 
 // Event pairs for timing the scan of every batch of a call.
@@ -2545,6 +2613,11 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
         ws->counters_clear = false;
         BatchContext ctx{index, ws, strategy, out_distances != nullptr};
         ctx.filter_candidates = true;
+        const bool estimable = !ws->filter_disabled && estimates_serve(index, strategy, batch);
+        const bool skipped = estimable && ws->estimates_skip > 0;
+        ws->estimates_skip -= skipped ? 1 : 0;
+        ctx.estimates = estimable && !skipped;
+        ctx.refine_every = ws->filter_disabled || skipped;
         ctx.gathered = !queries_on_device && gather_on_host(index, n);
         if (ctx.gathered) {
             gather_queries(index, ws, queries, n);
@@ -2665,6 +2738,35 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
         ws->last.kernel_launches = launches;
         if ((ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u &&
             !ws->filter_disabled) {
+            const std::vector<uint64_t> open = open_queries(ws->host_results.get(), n);
+            if (!open.empty()) {
+                std::vector<uha::Result> results(ws->host_results.get(),
+                                                 ws->host_results.get() + n);
+                std::vector<double> settled(ws->host_exact.get(), ws->host_exact.get() + n);
+                const uint32_t replayed = ws->host_counters.get()[0];
+                const uint32_t flag = ws->host_counters.get()[1] &
+                                      ~static_cast<uint32_t>(uha::kCandidateOverflow);
+                uha_query_stats st = ws->last;
+                const uha_query_stats more =
+                    answer_open(index, ws, queries, open, batch, strategy,
+                                out_distances != nullptr, results.data(), settled.data());
+                st.kernel_launches += more.kernel_launches;
+                st.scan_ms += more.scan_ms;
+                st.timed_scans += more.timed_scans;
+                st.device_ms += more.device_ms;
+                ws->last = st;
+                ws->host_counters.get()[0] =
+                    replayed + static_cast<uint32_t>(more.replayed_queries);
+                ws->host_counters.get()[1] = flag;
+                ws->estimates_wait =
+                    2 * open.size() > n
+                        ? std::clamp<uint32_t>(2 * ws->estimates_wait, 1, kLongestWait)
+                        : 0;
+                ws->estimates_skip = ws->estimates_wait;
+                finish_call(index, ws, n, results.data(), settled.data(), out_indices,
+                            out_distances);
+                return;
+            }
             // a query's filtered candidate list overflowed: answer the whole
             // call again with the slab selection
             ws->filter_disabled = true;
@@ -2676,6 +2778,9 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
                 fail(again, uha_last_error());
             }
             return;
+        }
+        if (ctx.estimates) {
+            ws->estimates_wait = 0;
         }
         finish_call(index, ws, n, ws->host_results.get(), ws->host_exact.get(),
                     out_indices, out_distances);

@@ -48,11 +48,16 @@ struct BatchContext {
     uint32_t* rescore_done = nullptr;
     cudaStream_t finish_stream = nullptr;
     cudaEvent_t handoff = nullptr;
-    // The precision strategies may take the fused candidate selection, and the
-    // direct strategy the split scan: the caller answers the call again without
-    // them (ws->filter_disabled) when a candidate list overflows (error bit
-    // uha::kCandidateOverflow).
+    // The precision strategies may take the fused candidate selection: the caller
+    // answers the call again without it (ws->filter_disabled) when a candidate
+    // list overflows (error bit uha::kCandidateOverflow).
     bool filter_candidates = false;
+    // The direct strategy may take the estimating scans: the caller answers the
+    // queries that they leave open (uha::kOpenQuery) by the binary32 scan.
+    bool estimates = false;
+    // Hierarchies: every reported distance in binary64, as the estimating scans
+    // that this batch's scan stands in for report it.
+    bool refine_every = false;
     // The batch's queries hold the sampled values alone (gathered on the host).
     bool gathered = false;
     // The fused flat query of this batch runs on stream lane `flat_lane`
@@ -98,6 +103,17 @@ void fill_trivial(uint64_t n, uint64_t* out_indices, double* out_distances);
 void finish_call(const uha_index* index, uha_workspace* ws, uint64_t n,
                  const uha::Result* results, const double* exact,
                  uint64_t* out_indices, double* out_distances);
+
+// The queries of a call that the estimating scans left open.
+std::vector<uint64_t> open_queries(const uha::Result* results, uint64_t n);
+// Answers them by the binary32 scans into results and exact, in batches of at most
+// `batch` on ws (whose query buffer, status words and last stats it overwrites);
+// queries: host or device, n x dimension. Returns the stats of these calls, added
+// up.
+uha_query_stats answer_open(const uha_index* index, uha_workspace* ws, const float* queries,
+                            const std::vector<uint64_t>& open, uint64_t batch,
+                            uha_strategy strategy, bool want_distances, uha::Result* results,
+                            double* exact);
 
 void validate_query_call(const uha_index* index, uha_workspace* ws,
                          const float* queries, uint64_t count, uint64_t batch,

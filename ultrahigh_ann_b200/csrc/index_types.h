@@ -172,6 +172,12 @@ struct uha_workspace {
     uha::DeviceBuffer<uint32_t> filter_sample;
     uha::DeviceBuffer<float> filter_norms;  // the sample rows' norms
     bool filter_disabled = false;  // answering again after an overflow
+    // Calls that still skip the estimating scans, and how many the last such
+    // stretch was: a call that they left open for over half of its queries
+    // (equal rows, queries far outside the rows) is followed by 1, 2, 4 .. 64
+    // calls on the binary32 scans, so such data costs little more than those.
+    uint32_t estimates_skip = 0;
+    uint32_t estimates_wait = 0;
     // certified split scan (allocated on first use): split queries and their
     // squared norms, partial estimates, per-query words (listed rows, smallest
     // e + E, finished settlement blocks), candidate lists, the filter's

@@ -281,6 +281,10 @@ uint32_t sample_tile_stride(uint64_t rows, uint64_t sample_rows);
 // is then answered again by the slab path.
 constexpr uint64_t kFilterMinRows = 16384;
 constexpr int kCandidateOverflow = 32;
+// Row of a query that an estimating scan (split, fixed-point, bitmaps) left open:
+// its list overflowed or its values are past the estimates' range. The error bit
+// above is then set, and the caller answers these queries by the binary32 scan.
+constexpr uint32_t kOpenQuery = 0xffffffffu;
 uint64_t filter_sample_rows(uint64_t rows);
 uint32_t filter_capacity(uint64_t rows, uint32_t k);
 // out[i] = norms[the index row sample row i stands for] (a sample of
@@ -318,7 +322,7 @@ void launch_project_queries64(const float* x, uint64_t batch, uint64_t padded_k,
 // Per query, the candidate with the smallest (reference binary64 squared
 // distance of the projected row rows64[row] to y64[q], row): results[q] and
 // exact_distances[q]. Candidates 0xffffffff are skipped; with counts, query q
-// has counts[q] of its k slots filled.
+// has counts[q] of its k slots filled (none or more than k: kOpenQuery).
 void launch_rescore_projected(const uint32_t* candidates, uint32_t k, uint32_t batch,
                               const double* rows64, const double* y64, uint32_t p,
                               Result* results, double* exact_distances,
@@ -525,7 +529,8 @@ void launch_fixed_scan(const FixedPlan& plan, const uint16_t* rows, uint64_t row
                        cudaStream_t stream);
 
 // Certified argmin of each query over its listed candidates, from the original
-// binary32 rows (exact and flat ops; the bound of settle_depth()). sums: settle_sums(batch) doubles; done: per query, zero.
+// binary32 rows (exact and flat ops; the bound of settle_depth()); kOpenQuery where
+// none or more than kSplitCandidates were listed. sums: settle_sums(batch) doubles; done: per query, zero.
 uint32_t settle_depth(uint64_t padded_dim);
 uint64_t settle_sums(uint64_t batch);
 void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
@@ -624,8 +629,8 @@ uint64_t bits_offsets(uint64_t batch, uint64_t p);
 void launch_row_bits(const float* rows, uint64_t row_count, uint64_t padded_p, uint64_t p,
                      float* boundaries, void* bits, cudaStream_t stream);
 // Certified argmin of a projected batch; results and exact distances are the
-// reference's. Error bit kCandidateOverflow: answer the call again by the
-// binary32 passes. offsets: bits_offsets(batch, p); listed, medians: batch x
+// reference's, kOpenQuery (and error bit kCandidateOverflow) where the binary32
+// passes have to answer. offsets: bits_offsets(batch, p); listed, medians: batch x
 // bits_list(rows); min_bits, counts: batch. Returns the kernel launches.
 struct BitsScan {
     const float* rows;

@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(kCountThreads, 1)
 
 // One warp per query, after the last pass: the listed rows whose bounds can hold
 // the minimum, settled by the reference's binary64 medians (lowest row on
-// ties). A query with no listed row (its list overflowed, or its medians are
-// past binary32) is answered again by the binary32 passes.
+// ties). A query whose list overflowed, or whose values or medians are past
+// binary32, stays open.
 template <int PER_LANE>
 __global__ void __launch_bounds__(kThreads)
     bits_settle_kernel(const Bits a, const double* __restrict__ rows64,
@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(kThreads)
     if (q >= a.batch) {
         return;
     }
-    const uint32_t n = min(a.counts[q], a.list);
+    const uint32_t n = a.counts[q] <= a.list && a.query_err[q] <= FLT_MAX ? a.counts[q] : 0u;
     const float2* medians = a.medians + static_cast<uint64_t>(q) * a.list;
     const uint32_t* list = a.listed + static_cast<uint64_t>(q) * a.list;
     // |reference median - m| <= rel m + err + abs
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kThreads)
     if (!(upper <= FLT_MAX)) {
         if (lane == 0) {
             atomicOr(a.error_flag, kCandidateOverflow);
-            results[q] = Result{0, 0.f};
+            results[q] = Result{kOpenQuery, 0.f};
             exact_distances[q] = __longlong_as_double(0x7ff8000000000000ll);
         }
         return;

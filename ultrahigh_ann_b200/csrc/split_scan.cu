@@ -798,8 +798,8 @@ __global__ void __launch_bounds__(kSelectThreads)
 
 // grid (row blocks, queries), after split_upper_kernel over every row: the rows
 // whose e - E is at most the smallest e + E, in any order, into the query's
-// list. More than cap of them, or a query norm the bound does not cover, sets
-// error bit kCandidateOverflow.
+// list. More than cap of them, or a query norm the bound does not cover (counted
+// as cap + 1 rows), sets error bit kCandidateOverflow.
 __global__ void __launch_bounds__(kSelectThreads)
     split_collect_kernel(const float* __restrict__ partials, uint32_t row_count,
                          const SplitQuery sq, uint32_t cap, uint32_t* __restrict__ candidates,
@@ -810,7 +810,9 @@ __global__ void __launch_bounds__(kSelectThreads)
     const float upper = from_ordered(sq.upper[q]);
     const float* base = partials + static_cast<uint64_t>(q) * row_count;
     const uint32_t first = blockIdx.x * kSelectThreads * kSelectRows + threadIdx.x;
+    // rows and cap + 1 together stay below 2^32
     if (threadIdx.x == 0 && blockIdx.x == 0 && !(a <= kLargestNorm)) {
+        atomicAdd(sq.counts + q, cap + 1);
         atomicOr(error_flag, kCandidateOverflow);
     }
     float s[kSelectRows];
@@ -884,7 +886,7 @@ __global__ void __launch_bounds__(kSelectThreads)
     if (lane == 0) {
         if (listed > list_cap || kept > cap || !(a <= kLargestNorm)) {
             atomicOr(error_flag, kCandidateOverflow);
-            kept = 0;  // not settled: the call is answered again
+            kept = 0;  // open
         }
         sq.counts[q] = kept;
     }
