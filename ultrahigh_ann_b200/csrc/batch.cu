@@ -204,7 +204,7 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
     } else if (const uha::SplitRows* sp =
                    !ws->split_disabled && split_shape(index, strategy, batch) &&
                            (!ws->emulated_replay || index->kind == IndexKind::hierarchical)
-                       ? split_rows(index, stream)
+                       ? split_rows(index, FormCall{batch, batch, true}, stream)
                        : nullptr;
                sp != nullptr) {
         // the certified split scan: its tile widths and column splits
@@ -217,34 +217,28 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
             }
             return;
         }
-        // the scores of every candidate go to a slab here
-        uint64_t most = 0;
-        bool room = true;
+        // the scores of every candidate go to a slab here: first the memory for the
+        // largest
+        SplitBuffers buffers{};
         for (const uha::SplitPlan& p : cands) {
-            most = std::max<uint64_t>(most, p.splits);
-            room = room && ensure_split_workspace(ws, index, sp->pitch, batch, p);
+            if (!split_buffers(ws, index, sp->pitch, batch, p, &buffers)) {
+                ws->split_disabled = true;
+                autotune(index, ws, batch, strategy, report);
+                return;
+            }
         }
-        const uint64_t slab = checked_mul(checked_mul(most, batch, "partials"), index->rows,
-                                          "partials");
-        if (room && ws->split_partials.size() < slab) {
-            check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
-            room = ws->split_partials.try_allocate(slab);
-        }
-        if (!room) {
-            ws->split_disabled = true;
-            autotune(index, ws, batch, strategy, report);
-            return;
-        }
-        check_cuda(cudaMemsetAsync(ws->split_queries.get(), 0, ws->split_queries.bytes(),
-                                   stream),
-                   "cannot clear the query buffer");
         int* flag = reinterpret_cast<int*>(ws->counters.get() + 1);
         for (size_t i = 0; i < cands.size(); ++i) {
             const uha::SplitPlan& p = cands[i];
+            split_buffers(ws, index, sp->pitch, batch, p, &buffers);
+            check_cuda(cudaMemsetAsync(buffers.queries, 0,
+                                       uha::round_up(batch, static_cast<uint64_t>(p.bn)) * 4 *
+                                           sp->pitch,
+                                       stream),
+                       "cannot clear the query buffer");
             const double ms = time_launches(stream, reps, [&] {
-                uha::launch_split_scores(p, sp->data.get(), index->rows,
-                                         ws->split_queries.get(), batch, sp->pitch,
-                                         ws->split_partials.get(), flag, index->sm_count,
+                uha::launch_split_scores(p, sp->data, index->rows, buffers.queries, batch,
+                                         sp->pitch, buffers.partials, flag, index->sm_count,
                                          stream);
             });
             if (i == 0) {
@@ -426,6 +420,7 @@ uint64_t enqueue_pair(uha_batch::Pair& p)
     BatchContext ctx{p.index, ws, p.strategy, true};
     ctx.filter_candidates = true;
     ctx.estimates = p.estimates;
+    ctx.build_forms = true;  // a captured batch is run again and again
     ctx.refine_every = !p.estimates;
     const uint64_t launches =
         enqueue_batch(ctx, ws->raw_queries.get(), p.count, ws->call_results.get(),
@@ -595,7 +590,8 @@ uint64_t answer_pair(uha_batch::Pair& p)
             uha_workspace_destroy(p.again);
             p.again = nullptr;
         }
-        const uha_status status = uha_workspace_create(p.index, open.size(), &p.again);
+        const uha_status status =
+            create_workspace(p.index, open.size(), false, &p.again);
         if (status != UHA_OK) {
             fail(status, uha_last_error());
         }
@@ -643,7 +639,7 @@ uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_c
             p.strategy = strategies != nullptr ? strategies[i] : UHA_DIRECT;
             p.offset = batch->total;
             batch->total = uha::checked_add(batch->total, p.count, "batch queries");
-            const uha_status st = uha_workspace_create(p.index, p.count, &p.ws);
+            const uha_status st = create_workspace(p.index, p.count, !persistent, &p.ws);
             if (st != UHA_OK) {
                 fail(st, uha_last_error());
             }
@@ -660,7 +656,8 @@ uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_c
             ws->host_results.allocate(p.count);
             ws->host_exact.allocate(p.count);
             if (!p.trivial) {
-                check_cuda(cudaMemsetAsync(ws->raw_queries.get(), 0, ws->raw_queries.bytes(),
+                check_cuda(cudaMemsetAsync(ws->raw_queries.get(), 0,
+                                           p.count * p.index->dimension * sizeof(float),
                                            ws->stream),
                            "cannot clear the query buffer");
                 if (autotune_shapes) {

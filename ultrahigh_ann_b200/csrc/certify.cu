@@ -2743,10 +2743,13 @@ namespace {
 constexpr uint32_t kSettleBlocks = 8 * 148;
 constexpr uint32_t kSettleParts = 16;
 
-uint32_t settle_parts(uint64_t batch)
+// Parts of the columns; short rows are one.
+uint32_t settle_parts(uint64_t batch, uint64_t padded_dim)
 {
-    return static_cast<uint32_t>(
-        std::max<uint64_t>(1, std::min<uint64_t>(kSettleParts, kSettleBlocks / batch)));
+    return padded_dim < 8192
+               ? 1
+               : static_cast<uint32_t>(std::max<uint64_t>(
+                     1, std::min<uint64_t>(kSettleParts, kSettleBlocks / batch)));
 }
 
 }  // namespace
@@ -2756,10 +2759,9 @@ uint32_t settle_depth(uint64_t padded_dim)
     return rescore_depth(padded_dim) + kSettleParts;
 }
 
-uint64_t settle_sums(uint64_t batch)
+uint64_t settle_sums(uint64_t batch, uint64_t padded_dim)
 {
-    // batch x parts is at most this for every smaller batch
-    return kSplitCandidates * std::max<uint64_t>(kSettleBlocks, batch);
+    return kSplitCandidates * batch * settle_parts(batch, padded_dim);
 }
 
 void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
@@ -2770,8 +2772,7 @@ void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
     if (batch == 0) {
         return;
     }
-    // short rows are one part
-    const uint32_t parts = in.padded_dim >= 8192 ? settle_parts(batch) : 1;
+    const uint32_t parts = settle_parts(batch, in.padded_dim);
     settle_kernel<<<dim3(parts, batch), kFinalizeThreads, 0, stream>>>(
         bound, in, candidates, counts, rows, sums, done, results, exact_distances, replay_count);
     check_cuda(cudaGetLastError(), "cannot launch the settlement kernel");

@@ -153,14 +153,15 @@ std::pair<uint64_t, uint64_t> gather_device_source(const uha_device_matrix* m,
 }
 
 // Uploads a host r x d matrix into the padded r x pd device layout.
-void upload_padded(DeviceBuffer<float>& dst, const float* src, uint64_t r,
-                   uint64_t d, uint64_t pd)
+void upload_scan_rows(uha_index* index, const float* src, uint64_t r,
+                      uint64_t d, uint64_t pd)
 {
-    dst.allocate(checked_mul(r, pd, "padded representative matrix"));
+    uha_engine::allocate_scan_rows(index);
+    DeviceBuffer<float>& dst = index->scan_rows;
     if (dst.size() == 0) {
         return;
     }
-    check_cuda(cudaMemset(dst.get(), 0, dst.bytes()),
+    check_cuda(cudaMemset(dst.get(), 0, r * pd * sizeof(float)),
                "cannot clear representative matrix");
     if (d != 0) {
         check_cuda(cudaMemcpy2D(dst.get(), pd * sizeof(float), src,
@@ -367,12 +368,11 @@ void create_exact_index(int device, uha_metric metric, const RowSource& src,
     require(index->padded_dim <= kMaxExtent, UHA_LENGTH_ERROR,
             "CUDA index dimensions exceed the device grid limits");
     if (src.device == nullptr) {
-        upload_padded(index->scan_rows, src.host, row_count, dimension,
-                      index->padded_dim);
+        upload_scan_rows(index.get(), src.host, row_count, dimension,
+                         index->padded_dim);
     } else {
         require_on_device(src.device, device);
-        index->scan_rows.allocate(
-            checked_mul(row_count, index->padded_dim, "padded representative matrix"));
+        uha_engine::allocate_scan_rows(index.get());
         if (gather_device_source(src.device, nullptr, nullptr, dimension,
                                  index->scan_rows.get(), index->padded_dim)
                 .first != ~0ull) {
@@ -451,8 +451,8 @@ extern "C" uha_status uha_weighted_l1_index_create(int device,
         index->dimension = dimension;
         index->scan_dim = dimension;
         index->padded_dim = uha::round_up(dimension, kColumnAlign);
-        upload_padded(index->scan_rows, rows, row_count, dimension,
-                      index->padded_dim);
+        upload_scan_rows(index.get(), rows, row_count, dimension,
+                         index->padded_dim);
         std::vector<float> w32(index->padded_dim, 0.0f);
         std::vector<double> w64(dimension);
         for (uint64_t i = 0; i < dimension; ++i) {
@@ -580,7 +580,7 @@ void create_sampled_index(int device, uha_metric metric, const RowSource& src,
     // Gather (and scale) the sampled columns of the rows on the device.
     if (src.device != nullptr) {
         require_on_device(src.device, device);
-        index->scan_rows.allocate(row_count * index->padded_dim);
+        uha_engine::allocate_scan_rows(index.get());
         const auto bad = gather_device_source(
             src.device, index->columns.get(),
             metric == UHA_L2 ? index->scales.get() : nullptr, sample_size,
@@ -596,7 +596,7 @@ void create_sampled_index(int device, uha_metric metric, const RowSource& src,
         check_cuda(cudaMemcpy(source.get(), rows, source.bytes(),
                               cudaMemcpyHostToDevice),
                    "cannot copy representatives to the CUDA device");
-        index->scan_rows.allocate(row_count * index->padded_dim);
+        uha_engine::allocate_scan_rows(index.get());
         uha::launch_gather_rows(source.get(), row_count, dimension,
                                 index->columns.get(),
                                 metric == UHA_L2 ? index->scales.get()
@@ -781,7 +781,7 @@ void create_hierarchical_index(int device, uha_metric metric, const RowSource& s
     uha::launch_project_rows64(sampled.get(), row_count, kp, k,
                                index->projection64.get(), p,
                                index->rows64.get(), bad.get(), nullptr);
-    index->scan_rows.allocate(row_count * pp);
+    uha_engine::allocate_scan_rows(index.get());
     index->row_err.allocate(row_count);
     uha::launch_narrow_rows(index->rows64.get(), row_count, p,
                             index->scan_rows.get(), pp, index->row_err.get(),
@@ -917,6 +917,12 @@ extern "C" uha_status uha_workspace_create(const uha_index* index,
                                            uint64_t maximum_batch_size,
                                            uha_workspace** out)
 {
+    return uha_engine::create_workspace(index, maximum_batch_size, true, out);
+}
+
+uha_status uha_engine::create_workspace(const uha_index* index, uint64_t maximum_batch_size,
+                                        bool scans, uha_workspace** out)
+{
     return guarded([&] {
         require(index != nullptr && out != nullptr, UHA_INVALID_ARGUMENT,
                 "index and output must not be null");
@@ -935,7 +941,7 @@ extern "C" uha_status uha_workspace_create(const uha_index* index,
         check_cuda(cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking),
                    "cannot create CUDA stream");
         const uint64_t b = maximum_batch_size;
-        ws->raw_queries.allocate(b * index->dimension);
+        uha_engine::allocate_raw_queries(ws.get(), index, scans);
         if (index->kind == IndexKind::hierarchical) {
             ws->prepared.allocate(b * index->padded_sample);
             ws->projected.allocate(b * index->padded_dim);
@@ -1119,43 +1125,6 @@ bool split_shape(const uha_index* index, uha_strategy strategy, uint64_t n)
 {
     return strategy == UHA_DIRECT && index->metric == UHA_L2 && n > 8 && n <= 65535 &&
            index->rows >= 2 && !small_path_applies(index, strategy);
-}
-
-bool ensure_split_workspace(uha_workspace* ws, const uha_index* index, uint64_t pitch,
-                            uint64_t n, const uha::SplitPlan& plan)
-{
-    cudaStream_t stream = ws->stream;
-    // grows a buffer that earlier work on the stream may still use
-    auto grow = [&](auto& buffer, uint64_t count) {
-        if (buffer.size() >= count) {
-            return true;
-        }
-        check_cuda(cudaStreamSynchronize(stream), "CUDA query failed");
-        return buffer.try_allocate(count);
-    };
-    const uint64_t b = ws->max_batch;
-    const uint64_t bytes = checked_mul(
-        checked_mul(uha::lowp_padded_count(b), pitch, "query buffer"), 4, "query buffer");
-    if (ws->split_queries.size() < bytes) {
-        if (!grow(ws->split_queries, bytes)) {
-            return false;
-        }
-        // vectors past a batch are read by the score kernel (and not stored)
-        check_cuda(cudaMemsetAsync(ws->split_queries.get(), 0, bytes, stream),
-                   "cannot clear the query buffer");
-    }
-    const bool filter = uha::split_filter_applies(plan, index->rows);
-    const uint64_t partials =
-        filter ? 0
-               : checked_mul(checked_mul(plan.splits, n, "partials"), index->rows, "partials");
-    const bool hierarchical = index->kind == IndexKind::hierarchical;
-    return grow(ws->split_squares, b * uha::kSplitSlices) && grow(ws->split_words, 3 * b) &&
-           grow(ws->split_candidates, b * uha::kSplitCandidates) &&
-           grow(ws->split_partials, partials) &&
-           (!filter || grow(ws->split_keys, checked_mul(b, uha::kSplitListKeys, "keys"))) &&
-           (hierarchical
-                ? grow(ws->projected64, checked_mul(b, index->projection_dimension, "queries"))
-                : grow(ws->split_sums, uha::settle_sums(b)));
 }
 
 // Workspace buffers of the precision strategies for batches up to max_batch.
@@ -1405,92 +1374,15 @@ uint64_t enqueue_lowp_candidates(const BatchContext& c, uint64_t n, const uha::L
     return 6;
 }
 
-// The split form of the index's rows (split_scan.cu), built on first use on
-// `stream` and synchronised before it is published; null when the index keeps
-// the binary32 scan.
-const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream)
+// What the row forms are asked for a batch of n.
+FormCall form_call(const BatchContext& c, uint64_t n)
 {
-    std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    if (index->split.ready) {
-        return index->split.usable ? &index->split : nullptr;
-    }
-    uha::SplitRows sp;  // published only once it is built
-    sp.ready = true;
-    const bool hierarchical = index->kind == IndexKind::hierarchical;
-    sp.pitch = uha::split_pitch(index->scan_dim);
-    const uint64_t bytes = checked_mul(
-        checked_mul(uha::lowp_padded_count(index->rows), sp.pitch, "split rows"), 4,
-        "split rows");
-    if (!sp.data.try_allocate(bytes) || !sp.norms.try_allocate(index->rows) ||
-        !sp.roots.try_allocate(index->rows + 1) || !sp.centre.try_allocate(sp.pitch)) {
-        index->split = uha::SplitRows{};
-        index->split.ready = true;
-        return nullptr;
-    }
-    // the word past the roots receives the largest of them
-    unsigned int* largest = reinterpret_cast<unsigned int*>(sp.roots.get() + index->rows);
-    // the split writes every row's whole pitch; the vectors past the rows are zero
-    const uint64_t used = index->rows * sp.pitch * 4;
-    check_cuda(cudaMemsetAsync(sp.data.get() + used, 0, bytes - used, stream),
-               "cannot clear split rows");
-    auto split = [&] {
-        if (hierarchical) {
-            uha::launch_split_rows(index->rows64.get(), index->rows, index->scan_dim,
-                                   index->scan_dim, sp.data.get(), sp.pitch, sp.scale,
-                                   sp.centre.get(), sp.norms.get(), sp.roots.get(), largest,
-                                   stream);
-        } else {
-            uha::launch_split_rows(index->scan_rows.get(), index->rows, index->padded_dim,
-                                   index->scan_dim, sp.data.get(), sp.pitch, sp.scale,
-                                   sp.centre.get(), sp.norms.get(), sp.roots.get(), largest,
-                                   stream);
-        }
-        float root = 0.f;
-        check_cuda(cudaMemcpyAsync(&root, largest, sizeof(root), cudaMemcpyDeviceToHost, stream),
-                   "cannot copy the largest norm from the CUDA device");
-        check_cuda(cudaStreamSynchronize(stream), "cannot build split rows");
-        return root;
-    };
-    float root = split();
-    if (std::isfinite(root) && root > 0.f && (root < 0x1p-8f || root > 0x1p24f)) {
-        sp.scale = std::ldexp(1.f, -std::clamp(std::ilogb(root), -126, 126));
-        root = split();
-    }
-    sp.usable = root <= uha::split_largest_norm();
-    if (!sp.usable) {
-        sp.data.release();
-    }
-    index->split = std::move(sp);
-    return index->split.usable ? &index->split : nullptr;
-}
-
-// The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use on
-// `stream` and synchronised before they are published; null when the index
-// keeps the binary32 passes.
-const uha::RowBits* row_bits(const uha_index* index, cudaStream_t stream)
-{
-    std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    if (!index->bits.ready) {
-        const uint64_t p = index->projection_dimension;
-        uha::RowBits rb;  // published only once it is built
-        rb.ready = true;
-        rb.usable = rb.boundaries.try_allocate(uha::bits_boundaries(p)) &&
-                    rb.data.try_allocate(uha::bits_bytes(index->rows, p));
-        if (rb.usable) {
-            uha::launch_row_bits(index->scan_rows.get(), index->rows, index->padded_dim, p,
-                                 rb.boundaries.get(), rb.data.get(), stream);
-            check_cuda(cudaStreamSynchronize(stream), "cannot build row bitmaps");
-        } else {
-            rb.boundaries.release();
-        }
-        index->bits = std::move(rb);
-    }
-    return index->bits.usable ? &index->bits : nullptr;
+    return {n, std::max(n, c.upcoming), c.build_forms};
 }
 
 // The bitmap form of this batch's median scan (everything it needs allocated
 // here), or null when it takes the binary32 passes.
-const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
+const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuffers* buffers)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
@@ -1500,23 +1392,8 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
         !uha::bits_batch(index->projection_dimension, n)) {
         return nullptr;
     }
-    const uha::RowBits* bits = row_bits(index, ws->stream);
-    if (bits == nullptr) {
-        return nullptr;
-    }
-    auto grow = [&](auto& buffer, uint64_t count) {
-        if (buffer.size() >= count) {
-            return true;
-        }
-        check_cuda(cudaStreamSynchronize(ws->stream), "CUDA query failed");
-        return buffer.try_allocate(count);
-    };
-    const uint64_t b = ws->max_batch;
-    const uint64_t list = checked_mul(b, uha::bits_list(index->rows), "row lists");
-    if (!grow(ws->median_min, std::max(n, b)) || !grow(ws->split_words, 3 * b) ||
-        !grow(ws->projected64, checked_mul(b, index->projection_dimension, "queries")) ||
-        !grow(ws->bits_offsets, uha::bits_offsets(b, index->projection_dimension)) ||
-        !grow(ws->bits_listed, list) || !grow(ws->bits_medians, list)) {
+    const uha::RowBits* bits = row_bits(index, form_call(c, n), ws->stream);
+    if (bits != nullptr && !bits_buffers(ws, index, n, buffers)) {
         ws->split_disabled = true;
         return nullptr;
     }
@@ -1524,7 +1401,8 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n)
 }
 
 // One batch by the bitmap median scan.
-uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, const float* source,
+uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits,
+                            const BitsBuffers& buffers, const float* source,
                             uint64_t n, uha::Result* results, double* exact, bool time_scan,
                             cudaEvent_t scan_start, cudaEvent_t scan_stop)
 {
@@ -1535,7 +1413,7 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
     const uint64_t p = index->projection_dimension;
     uha::launch_gather_project64(source, n, query_dimension(c), query_columns(c),
                                  index->sample_size, index->projection64_t.get(), p,
-                                 ws->projected64.get(), ws->projected.get(), index->padded_dim,
+                                 buffers.projected, ws->projected.get(), index->padded_dim,
                                  ws->coord_err.get(), ws->query_err.get(), error_flag, stream);
     uha::BitsScan s{};
     s.rows = index->scan_rows.get();
@@ -1543,20 +1421,20 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
     s.padded_p = index->padded_dim;
     s.p = p;
     s.rows64 = index->rows64.get();
-    s.boundaries = bits.boundaries.get();
-    s.bits = bits.data.get();
+    s.boundaries = bits.boundaries;
+    s.bits = bits.data;
     s.queries = ws->projected.get();
-    s.y64 = ws->projected64.get();
+    s.y64 = buffers.projected;
     s.query_err = ws->query_err.get();
     s.coord_err = ws->coord_err.get();
     s.row_err_max = index->row_err_max;
     s.rel = kMedianRel;
     s.abs_err = kMedianAbs;
-    s.min_bits = ws->median_min.get();
-    s.counts = ws->split_words.get();
-    s.offsets = ws->bits_offsets.get();
-    s.listed = ws->bits_listed.get();
-    s.medians = ws->bits_medians.get();
+    s.min_bits = buffers.min_bits;
+    s.counts = buffers.counts;
+    s.offsets = buffers.offsets;
+    s.listed = buffers.listed;
+    s.medians = buffers.medians;
     if (time_scan) {
         check_cuda(cudaEventRecord(scan_start, stream), "event");
     }
@@ -1568,54 +1446,10 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits, con
     return 1 + launches;
 }
 
-// The fixed-point form of an exact or flat L1 index's rows, built on first use on
-// `stream` and synchronised before it is published; null when the index keeps
-// the binary32 scan.
-const uha::FixedRows* fixed_rows(const uha_index* index, cudaStream_t stream)
-{
-    std::lock_guard<std::mutex> lock(index->lowp_mutex);
-    if (index->fixed.ready) {
-        return index->fixed.usable ? &index->fixed : nullptr;
-    }
-    uha::FixedRows fx;  // published only once it is built
-    fx.ready = true;
-    fx.pitch = uha::fixed_pitch(index->scan_dim);
-    // in units of 16 bytes
-    const uint64_t head = index->rows + (fx.pitch + 4) / 4;
-    const uint64_t scratch = (uha::fixed_scratch_words(index->scan_dim) + 3) / 4;
-    const uint64_t values = checked_mul(index->rows, fx.pitch / 8, "fixed-point rows");
-    if (fx.store.try_allocate(head + scratch + values)) {
-        float* offsets = reinterpret_cast<float*>(fx.store.get() + index->rows);
-        unsigned int* words = reinterpret_cast<unsigned int*>(fx.store.get() + head);
-        uint16_t* data = reinterpret_cast<uint16_t*>(fx.store.get() + head + scratch);
-        fx.offsets = offsets;
-        fx.data = data;
-        uha::launch_fixed_rows(index->scan_rows.get(), index->rows, index->padded_dim,
-                               index->scan_dim, index->weights64.get(), data, fx.pitch, offsets,
-                               offsets + fx.pitch, fx.store.get(), words, stream);
-        fx.usable = uha::fixed_usable(words, index->scan_dim, fx.store.get(), index->rows,
-                                      offsets + fx.pitch, stream);
-        if (!fx.usable) {
-            fx.store.release();
-        }
-    }
-    index->fixed = std::move(fx);
-    return index->fixed.usable ? &index->fixed : nullptr;
-}
-
 // The fixed-point scan of this batch (everything it needs allocated here), or
 // null when it takes the binary32 scan: every direct L1 batch past the streaming
 // scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers the
-// queries it leaves open. An index's first such call also
-// builds the rows (7,028 x 60,660: 0.8 ms; 65,536 x 128: 0.1 ms and an allocation
-// of 0.35 ms), which the large calls win back at once.
-struct FixedBuffers {
-    uha::FixedParts* parts;
-    unsigned long long* upper;
-    unsigned long long* least;
-    uint16_t* queries;
-    uint32_t* sums;
-};
+// queries it leaves open.
 const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::FixedPlan* plan,
                                     FixedBuffers* buffers)
 {
@@ -1624,48 +1458,18 @@ const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::Fixe
     if (!c.estimates || ws->split_disabled ||
         ws->emulated_replay || index->kind == IndexKind::hierarchical ||
         index->metric != UHA_L1 || precision_strategy(c.strategy) || n <= 8 || n > 65535 ||
-        index->rows < 2 || index->rows > (1u << 24)) {
+        index->rows < 2 || index->rows > uha::kFixedRows) {
         return nullptr;
     }
-    const uha::FixedRows* fx = fixed_rows(index, ws->stream);
+    const uha::FixedRows* fx = fixed_rows(index, form_call(c, n), ws->stream);
     if (fx == nullptr) {
         return nullptr;
     }
     *plan = uha::plan_fixed(index->rows, fx->pitch, n, index->sm_count);
-    auto grow = [&](auto& buffer, uint64_t count) {
-        if (buffer.size() >= count) {
-            return true;
-        }
-        check_cuda(cudaStreamSynchronize(ws->stream), "CUDA query failed");
-        return buffer.try_allocate(count);
-    };
-    const uint64_t b = ws->max_batch;
-    // each part in 16-byte units; FixedParts is 24 bytes
-    const uint64_t parts = (24 * n * uha::kSplitSlices + 15) / 16;
-    const uint64_t upper = (n + 1) / 2;
-    const uint64_t least = (checked_mul(n, uha::fixed_tiles(index->rows), "partials") + 1) / 2;
-    const uint64_t queries = checked_mul(n, fx->pitch / 8, "query buffer");
-    const uint64_t sums =
-        (checked_mul(checked_mul(plan->splits, n, "partials"), index->rows, "partials") + 3) / 4;
-    const uint64_t total = parts + upper + least + queries + sums;
-    if (!grow(ws->fixed_store, (16 * total + 23) / 24) ||
-        !grow(ws->split_words, 3 * b) ||
-        !grow(ws->split_candidates, b * uha::kSplitCandidates) ||
-        !grow(ws->split_sums, uha::settle_sums(b))) {
+    if (!fixed_buffers(ws, index, fx->pitch, n, *plan, buffers)) {
         ws->split_disabled = true;
         return nullptr;
     }
-    unsigned char* at = reinterpret_cast<unsigned char*>(ws->fixed_store.get());
-    auto take = [&](uint64_t units) {
-        unsigned char* here = at;
-        at += 16 * units;
-        return here;
-    };
-    buffers->parts = reinterpret_cast<uha::FixedParts*>(take(parts));
-    buffers->upper = reinterpret_cast<unsigned long long*>(take(upper));
-    buffers->least = reinterpret_cast<unsigned long long*>(take(least));
-    buffers->queries = reinterpret_cast<uint16_t*>(take(queries));
-    buffers->sums = reinterpret_cast<uint32_t*>(take(sums));
     return fx;
 }
 
@@ -1680,7 +1484,6 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
     uha_workspace* ws = c.ws;
     cudaStream_t stream = ws->stream;
     int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
-    uint32_t* words = ws->split_words.get();
     uha::FixedVectors v{};
     v.source = source;
     v.source_pitch = query_dimension(c);
@@ -1694,12 +1497,12 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
     v.prepared = ws->prepared.get();
     v.prepared_pitch = index->padded_dim;
     v.query_parts = buffers.parts;
-    v.counts = words;
+    v.counts = buffers.counts;
     v.upper = buffers.upper;
-    v.done = words + 2 * ws->max_batch;
+    v.done = buffers.done;
     v.error_flag = error_flag;
     uha::launch_fixed_queries(v, n, stream);
-    const uha::FixedQuery f{rows.store.get(),
+    const uha::FixedQuery f{rows.terms,
                             v.query_parts,
                             uha::fixed_slices(rows.pitch, n),
                             v.upper,
@@ -1709,7 +1512,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
         check_cuda(cudaEventRecord(scan_start, stream), "event");
     }
     uha::launch_fixed_scan(plan, rows.data, index->rows, buffers.queries, n, rows.pitch,
-                           buffers.sums, buffers.least, f, ws->split_candidates.get(),
+                           buffers.sums, buffers.least, f, buffers.candidates,
                            error_flag, stream);
     if (time_scan) {
         check_cuda(cudaEventRecord(scan_stop, stream), "event");
@@ -1724,8 +1527,8 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
     in.weights64 = index->weights64.get();
     const uint32_t depth = uha::settle_depth(index->padded_dim);
     uha::launch_settle(uha::make_bound64(depth, index->scan_dim), in,
-                       ws->split_candidates.get(), v.counts, static_cast<uint32_t>(n),
-                       static_cast<uint32_t>(index->rows), ws->split_sums.get(), v.done,
+                       buffers.candidates, v.counts, static_cast<uint32_t>(n),
+                       static_cast<uint32_t>(index->rows), buffers.settled, v.done,
                        results, exact, ws->counters.get(), stream);
     return plan.splits > 1 ? 5 : 4;
 }
@@ -1736,7 +1539,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
 // settlement has to do without FP64 instructions (the norms, roots and sums of
 // the split scan are binary64). Everything the batch needs is allocated here.
 bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** rows,
-                   uha::SplitPlan* plan)
+                   uha::SplitPlan* plan, SplitBuffers* buffers)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
@@ -1745,19 +1548,19 @@ bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** row
         !split_shape(index, c.strategy, n)) {
         return false;
     }
-    const uha::SplitRows* sp = split_rows(index, ws->stream);
-    if (sp == nullptr) {
-        return false;
-    }
     const TunedPlan* tuned = ws->find_tuned(n, static_cast<int>(c.strategy));
     if (tuned != nullptr && !tuned->split) {
+        return false;
+    }
+    const uha::SplitRows* sp = split_rows(index, form_call(c, n), ws->stream);
+    if (sp == nullptr) {
         return false;
     }
     *plan = tuned != nullptr
                 ? tuned->split_plan
                 : uha::plan_split(index->rows, sp->pitch, n, index->sm_count);
     *rows = sp;
-    if (!ensure_split_workspace(ws, index, sp->pitch, n, *plan)) {
+    if (!split_buffers(ws, index, sp->pitch, n, *plan, buffers)) {
         ws->split_disabled = true;
         return false;
     }
@@ -1944,7 +1747,8 @@ void ensure_flat_scratch(const uha_index* index, uha_workspace* ws)
 // tensor-core estimates, every row that can be the minimum, and their
 // settlement from the original values.
 uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
-                             const uha::SplitPlan& plan, const float* source, uint64_t n,
+                             const uha::SplitPlan& plan, const SplitBuffers& buffers,
+                             const float* source, uint64_t n,
                              uha::Result* results, double* exact, bool time_scan,
                              cudaEvent_t scan_start, cudaEvent_t scan_stop)
 {
@@ -1954,38 +1758,37 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     int* error_flag = reinterpret_cast<int*>(ws->counters.get() + 1);
     const bool hierarchical = index->kind == IndexKind::hierarchical;
     const uint32_t b = static_cast<uint32_t>(n);
-    uint32_t* words = ws->split_words.get();
     uha::SplitVectors v{};
     v.source = source;
     v.source_pitch = query_dimension(c);
     v.dim = index->scan_dim;
     v.columns = query_columns(c);
     v.scales = index->scales.get();
-    v.centre = rows.centre.get();
+    v.centre = rows.centre;
     v.scale = rows.scale;
-    v.out = ws->split_queries.get();
+    v.out = buffers.queries;
     v.pitch = rows.pitch;
     v.prepared = ws->prepared.get();
     v.prepared_pitch = index->padded_dim;
-    v.squares = ws->split_squares.get();
-    v.counts = words;
-    v.upper = words + ws->max_batch;
-    v.done = words + 2 * ws->max_batch;
+    v.squares = buffers.squares;
+    v.counts = buffers.counts;
+    v.upper = buffers.upper;
+    v.done = buffers.done;
     v.error_flag = error_flag;
     uint64_t launches = 1;
     if (hierarchical) {
         const uint64_t p = index->projection_dimension;
         uha::launch_gather_project64(source, n, query_dimension(c), query_columns(c),
                                      index->sample_size, index->projection64_t.get(), p,
-                                     ws->projected64.get(), nullptr, index->padded_dim, nullptr,
+                                     buffers.projected, nullptr, index->padded_dim, nullptr,
                                      nullptr, error_flag, stream);
-        v.source = ws->projected64.get();
+        v.source = buffers.projected;
         v.source_pitch = p;
         ++launches;
     }
     uha::launch_split_queries(v, n, hierarchical, stream);
-    const uha::SplitQuery sq{rows.norms.get(),
-                             rows.roots.get(),
+    const uha::SplitQuery sq{rows.norms,
+                             rows.roots,
                              v.squares,
                              uha::split_slices(rows.pitch, n),
                              uha::split_error_rel(plan, index->rows),
@@ -1995,15 +1798,15 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
         check_cuda(cudaEventRecord(scan_start, stream), "event");
     }
     if (uha::split_filter_applies(plan, index->rows)) {
-        uha::launch_split_filter_scan(plan, rows.data.get(), index->rows,
-                                      ws->split_queries.get(), n, rows.pitch, sq,
-                                      ws->split_keys.get(), ws->split_candidates.get(),
+        uha::launch_split_filter_scan(plan, rows.data, index->rows,
+                                      buffers.queries, n, rows.pitch, sq,
+                                      buffers.keys, buffers.candidates,
                                       error_flag, index->sm_count, stream);
         launches += 3;
     } else {
-        uha::launch_split_scan(plan, rows.data.get(), index->rows, ws->split_queries.get(), n,
-                               rows.pitch, ws->split_partials.get(), sq,
-                               ws->split_candidates.get(), error_flag, index->sm_count, stream);
+        uha::launch_split_scan(plan, rows.data, index->rows, buffers.queries, n,
+                               rows.pitch, buffers.partials, sq,
+                               buffers.candidates, error_flag, index->sm_count, stream);
         launches += 3;
     }
     if (time_scan) {
@@ -2013,8 +1816,8 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
         // the reference's binary64 distance of every listed row, in the
         // projected space; the smallest (lowest row on ties) is the answer
         uha::launch_rescore_projected(
-            ws->split_candidates.get(), uha::kSplitCandidates, b, index->rows64.get(),
-            ws->projected64.get(), static_cast<uint32_t>(index->projection_dimension), results,
+            buffers.candidates, uha::kSplitCandidates, b, index->rows64.get(),
+            buffers.projected, static_cast<uint32_t>(index->projection_dimension), results,
             exact, stream, v.counts);
         return launches + 1;
     }
@@ -2026,7 +1829,7 @@ uint64_t enqueue_split_batch(const BatchContext& c, const uha::SplitRows& rows,
     in.padded_dim = index->padded_dim;
     const uint32_t depth = uha::settle_depth(index->padded_dim);
     uha::launch_settle(uha::make_bound64(depth, index->scan_dim), in,
-                       ws->split_candidates.get(), v.counts, b, static_cast<uint32_t>(index->rows), ws->split_sums.get(),
+                       buffers.candidates, v.counts, b, static_cast<uint32_t>(index->rows), buffers.sums,
                        v.done, results, exact, ws->counters.get(), stream);
     return launches + 1;
 }
@@ -2105,19 +1908,21 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     }
     const uha::SplitRows* split = nullptr;
     uha::SplitPlan split_plan{};
-    if (split_applies(c, n, &split, &split_plan)) {
-        return enqueue_split_batch(c, *split, split_plan, source, n, results, exact, time_scan,
+    SplitBuffers split_parts{};
+    if (split_applies(c, n, &split, &split_plan, &split_parts)) {
+        return enqueue_split_batch(c, *split, split_plan, split_parts, source, n, results, exact, time_scan,
                                    scan_start, scan_stop);
     }
     uha::FixedPlan fixed_plan{};
-    FixedBuffers fixed_buffers{};
-    if (const uha::FixedRows* fixed = fixed_applies(c, n, &fixed_plan, &fixed_buffers);
+    FixedBuffers fixed_parts{};
+    if (const uha::FixedRows* fixed = fixed_applies(c, n, &fixed_plan, &fixed_parts);
         fixed != nullptr) {
-        return enqueue_fixed_batch(c, *fixed, fixed_plan, fixed_buffers, source, n, results,
+        return enqueue_fixed_batch(c, *fixed, fixed_plan, fixed_parts, source, n, results,
                                    exact, time_scan, scan_start, scan_stop);
     }
-    if (const uha::RowBits* bits = bits_scan_applies(c, n); bits != nullptr) {
-        return enqueue_bits_batch(c, *bits, source, n, results, exact, time_scan, scan_start,
+    BitsBuffers bits_parts{};
+    if (const uha::RowBits* bits = bits_scan_applies(c, n, &bits_parts); bits != nullptr) {
+        return enqueue_bits_batch(c, *bits, bits_parts, source, n, results, exact, time_scan, scan_start,
                                   scan_stop);
     }
     float* prepared = c.prepared != nullptr ? c.prepared : ws->prepared.get();
@@ -2694,6 +2499,7 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
             const bool timed = ws->timing && b % ws->timing_stride == 0;
             bc.flat_lane = static_cast<int>(b % static_cast<uint64_t>(lanes));
             bc.flat_shared = lanes > 1;
+            bc.upcoming = n - start;
             launches += enqueue_batch(bc, source, count, ws->call_results.get() + start,
                                       ws->call_exact.get() + start, timed,
                                       timed ? ws->scan_events[2 * b] : nullptr,

@@ -22,14 +22,70 @@ const uha::LowpRows& lowp_rows(const uha_index* index, uha::LowpType type,
 void ensure_lowp_workspace(uha_workspace* ws, const uha_index* index,
                            cudaStream_t stream);
 
-// Batches of n queries that the certified split scan (split_scan.cu) can serve;
-// the split form of the index's rows (null: the index keeps the binary32 scan);
-// and the workspace buffers of a batch of n with this plan (false when the device
-// has no room).
+// Batches of n queries that the certified split scan (split_scan.cu) can serve.
 bool split_shape(const uha_index* index, uha_strategy strategy, uint64_t n);
-const uha::SplitRows* split_rows(const uha_index* index, cudaStream_t stream);
-bool ensure_split_workspace(uha_workspace* ws, const uha_index* index, uint64_t pitch,
-                            uint64_t n, const uha::SplitPlan& plan);
+
+// row_forms.cu: the rows' allocation (rows x padded_dim, with a small form's place),
+// and the forms, built on `stream` and synchronised before they are published; null
+// while the index keeps the binary32 scan (no room, out of the form's range, or not
+// worth its build yet).
+struct FormCall {
+    uint64_t batch;     // queries of this batch
+    uint64_t upcoming;  // of this and the call's later batches
+    bool now;           // built whatever it would save (captured and tuned batches)
+};
+void allocate_scan_rows(uha_index* index);
+const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
+                                 cudaStream_t stream);
+const uha::FixedRows* fixed_rows(const uha_index* index, const FormCall& call,
+                                 cudaStream_t stream);
+const uha::RowBits* row_bits(const uha_index* index, const FormCall& call, cudaStream_t stream);
+
+// The workspace's query buffer (max_batch x dimension), with the place of the scan
+// buffers of a largest batch where they are small and `scans` asks for it.
+void allocate_raw_queries(uha_workspace* ws, const uha_index* index, bool scans);
+// uha_workspace_create; without `scans` for a caller that never estimates.
+uha_status create_workspace(const uha_index* index, uint64_t maximum_batch_size, bool scans,
+                            uha_workspace** out);
+
+// The estimating scans' buffers of a batch of n, from the workspace's scan memory
+// (false when the device has no room). Only one scan's are in use at a time.
+struct SplitBuffers {
+    unsigned char* queries;
+    double* squares;
+    uint32_t* counts;
+    unsigned int* upper;
+    uint32_t* done;
+    uint32_t* candidates;
+    unsigned long long* keys;  // filter form
+    float* partials;           // else
+    double* sums;              // exact and flat: the settlement's
+    double* projected;         // hierarchies
+};
+struct FixedBuffers {
+    uha::FixedParts* parts;
+    uint32_t* counts;
+    unsigned long long* upper;
+    uint32_t* done;
+    uint32_t* candidates;
+    unsigned long long* least;
+    uint16_t* queries;
+    uint32_t* sums;
+    double* settled;  // the settlement's sums
+};
+struct BitsBuffers {
+    unsigned int* min_bits;
+    uint32_t* counts;
+    uint32_t* offsets;
+    uint32_t* listed;
+    float2* medians;
+    double* projected;
+};
+bool split_buffers(uha_workspace* ws, const uha_index* index, uint64_t pitch, uint64_t n,
+                   const uha::SplitPlan& plan, SplitBuffers* out);
+bool fixed_buffers(uha_workspace* ws, const uha_index* index, uint64_t pitch, uint64_t n,
+                   const uha::FixedPlan& plan, FixedBuffers* out);
+bool bits_buffers(uha_workspace* ws, const uha_index* index, uint64_t n, BitsBuffers* out);
 
 struct BatchContext {
     const uha_index* index;
@@ -55,6 +111,8 @@ struct BatchContext {
     // The direct strategy may take the estimating scans: the caller answers the
     // queries that they leave open (uha::kOpenQuery) by the binary32 scan.
     bool estimates = false;
+    uint64_t upcoming = 0;    // queries of the call from this batch on
+    bool build_forms = false;  // a row form is built whatever this call would save
     // Hierarchies: every reported distance in binary64, as the estimating scans
     // that this batch's scan stands in for report it.
     bool refine_every = false;

@@ -31,14 +31,15 @@ struct LowpRows {
 
 // The split form of an L2 index's scanned rows (split_scan.cu), built on first
 // use: lowp_padded_count(rows) vectors of 2 x pitch BF16 values, their centre,
-// squared norms and roots. `usable` is false when the memory for it was not
-// available or a norm is past the bound's range; such an index keeps the
-// binary32 scan.
+// squared norms and roots, in one allocation or the place beside the rows. `usable`
+// is false when the memory for it was not available or a norm is past the bound's
+// range; such an index keeps the binary32 scan.
 struct SplitRows {
-    DeviceBuffer<unsigned char> data;
-    DeviceBuffer<float> centre;
-    DeviceBuffer<float> norms;
-    DeviceBuffer<float> roots;
+    DeviceBuffer<unsigned char> own;
+    unsigned char* data = nullptr;
+    float* centre = nullptr;
+    float* norms = nullptr;
+    float* roots = nullptr;
     uint64_t pitch = 0;
     float scale = 1.f;
     bool ready = false;
@@ -46,11 +47,13 @@ struct SplitRows {
 };
 
 // The fixed-point form of an exact or flat L1 index's rows (fixed_scan.cu),
-// built on first use, in one allocation: each row's terms, the column offsets and
-// the step, the build's scratch, rows x pitch 16-bit values. `usable` is false when the memory was not
-// available or the step does not resolve the index's distances.
+// built on first use, in one allocation or the place beside the rows: each row's
+// terms, the column offsets and the step, the build's scratch, rows x pitch 16-bit
+// values. `usable` is false when the memory was not available or the step does not
+// resolve the index's distances.
 struct FixedRows {
-    DeviceBuffer<FixedTerms> store;
+    DeviceBuffer<unsigned char> own;
+    const FixedTerms* terms = nullptr;
     const float* offsets = nullptr;  // pitch values, then the step
     const uint16_t* data = nullptr;
     uint64_t pitch = 0;
@@ -61,8 +64,9 @@ struct FixedRows {
 // The row bitmaps of an L1 hierarchy (median_bits.cu), built on first use;
 // `usable` is false when the memory for them was not available.
 struct RowBits {
-    DeviceBuffer<unsigned char> data;
-    DeviceBuffer<float> boundaries;
+    DeviceBuffer<unsigned char> own;
+    unsigned char* data = nullptr;
+    float* boundaries = nullptr;
     bool ready = false;
     bool usable = false;
 };
@@ -87,7 +91,9 @@ struct uha_index {
     uint64_t padded_dim = 0;  // scan_dim rounded up to kColumnAlign
     uint64_t sample_size = 0;
     uint64_t sampled_multiplicity = 0;
-    uha::DeviceBuffer<float> scan_rows;   // rows x padded_dim
+    uha::DeviceBuffer<float> scan_rows;   // rows x padded_dim, the row form's place
+    unsigned char* form_space = nullptr;  // that place (small forms)
+    uint64_t form_space_bytes = 0;
     uha::DeviceBuffer<float> row_norms;   // rows (L2, norm-identity strategy)
     uha::DeviceBuffer<float> weights32;   // padded_dim (weighted L1 scan)
     uha::DeviceBuffer<double> weights64;  // scan_dim (weighted L1 replay)
@@ -114,9 +120,13 @@ struct uha_index {
     mutable std::mutex lowp_mutex;
     mutable uha::LowpRows lowp[2];
     mutable uha::LowpRows lowp_projection[2];  // L2 hierarchy: the p x k projection
+    // the row form of the estimating scans, and the time (us) that a form not built
+    // yet would have saved so far
+    mutable std::mutex forms_mutex;
     mutable uha::SplitRows split;
     mutable uha::RowBits bits;  // L1 hierarchy
     mutable uha::FixedRows fixed;  // exact and flat L1
+    mutable double form_saved = 0.0;
 };
 
 // A scan shape chosen by the autotuner for one (batch size, strategy) of a
@@ -141,7 +151,7 @@ struct uha_workspace {
     uint64_t max_batch = 0;
     uint64_t payload_bytes = 0;
     cudaStream_t stream = nullptr;
-    uha::DeviceBuffer<float> raw_queries;
+    uha::DeviceBuffer<float> raw_queries;  // max_batch x dimension, the scans' place
     uha::DeviceBuffer<float> prepared;
     uha::DeviceBuffer<float> projected;   // hierarchical: batch x padded p
     uha::DeviceBuffer<float> query_err;   // hierarchical: batch
@@ -178,27 +188,13 @@ struct uha_workspace {
     // calls on the binary32 scans, so such data costs little more than those.
     uint32_t estimates_skip = 0;
     uint32_t estimates_wait = 0;
-    // certified split scan (allocated on first use): split queries and their
-    // squared norms, partial estimates, per-query words (listed rows, smallest
-    // e + E, finished settlement blocks), candidate lists, the filter's
-    // keys, settlement sums. split_disabled: this workspace keeps the
-    // binary32 scans (persistent batches; no memory for these or the bitmaps').
-    uha::DeviceBuffer<unsigned char> split_queries;
-    uha::DeviceBuffer<double> split_squares;
-    uha::DeviceBuffer<float> split_partials;
-    uha::DeviceBuffer<uint32_t> split_words;
-    uha::DeviceBuffer<uint32_t> split_candidates;
-    uha::DeviceBuffer<unsigned long long> split_keys;
-    uha::DeviceBuffer<double> split_sums;
-    // fixed-point scan, one allocation: queries' parts, upper ends, tiles' least
-    // values, queries, sums (its other buffers are the split scan's)
-    uha::DeviceBuffer<uha::FixedParts> fixed_store;
+    // the estimating scans' buffers of a batch (row_forms.cu): their place behind the
+    // query buffer, or an allocation on first use. split_disabled: this workspace
+    // keeps the binary32 scans (persistent batches; no memory).
+    unsigned char* scan_space = nullptr;
+    uint64_t scan_space_bytes = 0;
+    uha::DeviceBuffer<unsigned char> scan_store;
     bool split_disabled = false;
-    // median scan by bitmaps (allocated on first use): intervals, listed rows
-    // and their medians; the per-query words are median_min and split_words
-    uha::DeviceBuffer<uint32_t> bits_offsets;
-    uha::DeviceBuffer<uint32_t> bits_listed;
-    uha::DeviceBuffer<float2> bits_medians;
     uha::DeviceBuffer<uint32_t> candidates;       // [batch][candidates_per_query]
     uha::DeviceBuffer<double> cand_dist;          // [batch][candidates_per_query]
     uha::DeviceBuffer<uint32_t> rescore_done;     // per query, zero between calls

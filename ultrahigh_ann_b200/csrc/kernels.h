@@ -507,6 +507,8 @@ struct FixedPlan {
     uint32_t columns_per_split;
 };
 uint64_t fixed_pitch(uint64_t dim);
+// The most rows the fixed-point scan takes.
+constexpr uint64_t kFixedRows = 1ull << 24;
 uint64_t fixed_scratch_words(uint64_t dim);
 // The rows (padded, weights nullable) in fixed point: row_count x pitch values,
 // offsets (pitch), the step and each row's terms; scratch:
@@ -530,9 +532,9 @@ void launch_fixed_scan(const FixedPlan& plan, const uint16_t* rows, uint64_t row
 
 // Certified argmin of each query over its listed candidates, from the original
 // binary32 rows (exact and flat ops; the bound of settle_depth()); kOpenQuery where
-// none or more than kSplitCandidates were listed. sums: settle_sums(batch) doubles; done: per query, zero.
+// none or more than kSplitCandidates were listed. sums: settle_sums() doubles; done: per query, zero.
 uint32_t settle_depth(uint64_t padded_dim);
-uint64_t settle_sums(uint64_t batch);
+uint64_t settle_sums(uint64_t batch, uint64_t padded_dim);
 void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
                    const uint32_t* counts, uint32_t batch, uint32_t rows, double* sums,
                    uint32_t* done, Result* results, double* exact_distances,

@@ -208,7 +208,7 @@ struct uha_server {
         Entry& e = *entries[id];
         Pooled* p = &pooled;
         p->index_id = id;
-        const uha_status st = uha_workspace_create(e.index, cfg.max_batch, &p->ws);
+        const uha_status st = create_workspace(e.index, cfg.max_batch, false, &p->ws);
         if (st != UHA_OK) {
             fail(st, uha_last_error());
         }
@@ -558,7 +558,7 @@ extern "C" uha_status uha_server_add_index(uha_server* server, const uha_index* 
         {
             // validate the strategy against the index as a query would
             uha_workspace* probe = nullptr;
-            const uha_status st = uha_workspace_create(index, 1, &probe);
+            const uha_status st = create_workspace(index, 1, false, &probe);
             if (st != UHA_OK) {
                 fail(st, uha_last_error());
             }
