@@ -346,6 +346,7 @@ struct uha_batch {
         // does again (0: never).
         bool estimates = true;
         uint32_t wait = 0;
+        uint32_t unpaid = 0;  // runs in a row whose estimates did not pay
         uha_tune_report tuning{};
     };
     int device = 0;
@@ -568,8 +569,8 @@ void capture_batch(uha_batch* batch)
     batch->launches = launches;
 }
 
-// Runs that a pair stays on the binary32 scans after one whose estimates left over
-// half of its queries open; both captures are paid back by then.
+// Runs that a pair stays on the binary32 scans after two in a row whose estimates
+// left so much open that they did not pay; both captures are paid back by then.
 constexpr uint32_t kPairWait = 64;
 
 // Answers the queries that a run left open (all of the pair's where a precision
@@ -757,8 +758,13 @@ extern "C" uha_status uha_batch_run(uha_batch* batch, const float* const* querie
                 fill_trivial(p.count, idx, dist);
                 continue;
             }
-            if ((p.ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u &&
-                2 * answer_pair(p) > p.count) {
+            const uint64_t left =
+                (p.ws->host_counters.get()[1] & uha::kCandidateOverflow) != 0u ? answer_pair(p)
+                                                                               : 0;
+            const bool paid = left == 0 || estimates_pay(p.index, p.count, left);
+            p.unpaid = paid ? 0 : p.unpaid + 1;
+            if (p.unpaid == 2) {
+                p.unpaid = 0;
                 p.estimates = false;
                 p.wait = kPairWait;
                 changed.push_back(&p);

@@ -2564,10 +2564,12 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
                 ws->host_counters.get()[0] =
                     replayed + static_cast<uint32_t>(more.replayed_queries);
                 ws->host_counters.get()[1] = flag;
+                // (a call of several batches: about its first one's share)
+                const uint64_t first = std::min(n, batch);
                 ws->estimates_wait =
-                    2 * open.size() > n
-                        ? std::clamp<uint32_t>(2 * ws->estimates_wait, 1, kLongestWait)
-                        : 0;
+                    estimates_pay(index, first, (open.size() * first + n - 1) / n)
+                        ? 0
+                        : std::clamp<uint32_t>(2 * ws->estimates_wait, 1, kLongestWait);
                 ws->estimates_skip = ws->estimates_wait;
                 finish_call(index, ws, n, results.data(), settled.data(), out_indices,
                             out_distances);

@@ -48,6 +48,10 @@ void allocate_raw_queries(uha_workspace* ws, const uha_index* index, bool scans)
 uha_status create_workspace(const uha_index* index, uint64_t maximum_batch_size, bool scans,
                             uha_workspace** out);
 
+// Whether estimates that leave `open` of n queries to the binary32 scan take less
+// time than the binary32 scan of them all.
+bool estimates_pay(const uha_index* index, uint64_t n, uint64_t open);
+
 // The estimating scans' buffers of a batch of n, from the workspace's scan memory
 // (false when the device has no room). Only one scan's are in use at a time.
 struct SplitBuffers {

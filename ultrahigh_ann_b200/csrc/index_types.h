@@ -183,9 +183,9 @@ struct uha_workspace {
     uha::DeviceBuffer<float> filter_norms;  // the sample rows' norms
     bool filter_disabled = false;  // answering again after an overflow
     // Calls that still skip the estimating scans, and how many the last such
-    // stretch was: a call that they left open for over half of its queries
-    // (equal rows, queries far outside the rows) is followed by 1, 2, 4 .. 64
-    // calls on the binary32 scans, so such data costs little more than those.
+    // stretch was: a call of which they left so much open (equal rows, queries far
+    // outside the rows) that they did not pay is followed by 1, 2, 4 .. 64 calls on
+    // the binary32 scans, so such data costs little more than those.
     uint32_t estimates_skip = 0;
     uint32_t estimates_wait = 0;
     // the estimating scans' buffers of a batch (row_forms.cu): their place behind the

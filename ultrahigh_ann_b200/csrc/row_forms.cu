@@ -119,24 +119,45 @@ struct Drain {
     ~Drain() { cudaStreamSynchronize(stream); }
 };
 
+// About the time (us) of a batch of n by the binary32 scan and by the estimating one:
+// a fixed part (launches, synchronisation, delivery) and the (query, row, column)
+// rates of each on a B200, within a third of what was measured from 1,000 x 300 to
+// 65,536 x 1,500 values and 9 to 4,096 queries. The binary32 tile takes 64 queries'
+// time at least.
+struct BatchTimes {
+    double binary32;
+    double estimates;
+};
+
+BatchTimes batch_times(const uha_index* index, uint64_t n)
+{
+    const double values = static_cast<double>(index->rows) * index->scan_dim;
+    const double all = values * n;
+    if (index->kind == IndexKind::hierarchical) {
+        return index->metric == UHA_L2 ? BatchTimes{230 + all / 4.5e6, 75 + all / 80e6}
+                                       : BatchTimes{290 + all / 3.2e6, 130 + all / 25e6};
+    }
+    const double binary32 = 60 + values * round_up(n, 64) / 12e6;
+    return index->metric == UHA_L2
+               ? BatchTimes{binary32, 45 + std::max(values * 4 / 5.5e6, 6 * all / 1.4e9)}
+               : BatchTimes{binary32, 45 + values * round_up(n, 32) / 24e6};
+}
+
 // Whether a form that is not there yet is built for this call. One with a place
-// beside the rows is at once (0.1 ms at most); a larger one, whose allocation and
-// two passes over the rows cost 0.45 ms and the bytes at about 5 TB/s, once the
-// batches so far and the rest of this call would have saved that: the binary32 scan
-// takes 64 queries' time at least, at 12e12 (query, row, column) a second, and the
-// forms' scans leave half of it (L1) or a seventh (split rows, bitmaps).
-// Called with forms_mutex held.
+// beside the rows is at once (50 us); a larger one, whose allocation and two passes
+// over the rows cost 0.45 ms and the bytes at about 5 TB/s, once the batches so far
+// and the rest of this call would have saved that. Called with forms_mutex held.
 bool form_due(const uha_index* index, const FormCall& call, uint64_t bytes)
 {
     if (call.now || bytes <= index->form_space_bytes) {
         return true;
     }
-    const double values = static_cast<double>(index->rows) * index->scan_dim;
-    const bool fixed = index->metric == UHA_L1 && index->kind != IndexKind::hierarchical;
-    auto saved = [&](uint64_t queries) {  // us
-        return (fixed ? 0.5 : 0.85) * values * std::max<uint64_t>(queries, 64) / 12e6;
+    auto saved = [&](uint64_t queries) {
+        const BatchTimes t = batch_times(index, queries);
+        return std::max(0.0, t.binary32 - t.estimates);
     };
-    const double cost = 450.0 + (2.0 * values * sizeof(float) + bytes) / 5e6;
+    const double rows = static_cast<double>(index->rows) * index->scan_dim * sizeof(float);
+    const double cost = 450.0 + (2.0 * rows + bytes) / 5e6;
     if (index->form_saved + saved(call.upcoming) >= cost) {
         return true;
     }
@@ -207,6 +228,12 @@ bool carve(uha_workspace* ws, uint64_t n, F&& layout)
 }
 
 }  // namespace
+
+bool estimates_pay(const uha_index* index, uint64_t n, uint64_t open)
+{
+    const BatchTimes all = batch_times(index, n);
+    return all.estimates + batch_times(index, open).binary32 <= all.binary32;
+}
 
 void allocate_scan_rows(uha_index* index)
 {
