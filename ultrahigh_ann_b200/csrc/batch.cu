@@ -102,6 +102,7 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
         return;
     }
     DeviceGuard guard(index->device);
+    const FormUse forms(index);
     cudaStream_t stream = ws->stream;
     ws->counters_clear = false;  // the timed launches may set the error word
     TunedPlan best{};
@@ -347,6 +348,7 @@ struct uha_batch {
         bool estimates = true;
         uint32_t wait = 0;
         uint32_t unpaid = 0;  // runs in a row whose estimates did not pay
+        std::unique_ptr<FormUse> forms;  // the graph reads them
         uha_tune_report tuning{};
     };
     int device = 0;
@@ -640,6 +642,7 @@ uha_status create_batch(const uha_index* const* indexes, const uint64_t* query_c
             p.strategy = strategies != nullptr ? strategies[i] : UHA_DIRECT;
             p.offset = batch->total;
             batch->total = uha::checked_add(batch->total, p.count, "batch queries");
+            p.forms = std::make_unique<FormUse>(p.index);
             const uha_status st = create_workspace(p.index, p.count, !persistent, &p.ws);
             if (st != UHA_OK) {
                 fail(st, uha_last_error());

@@ -59,6 +59,23 @@ inline uint64_t round_up(uint64_t value, uint64_t multiple)
     return (value + multiple - 1) / multiple * multiple;
 }
 
+// Gives back device memory of the current device that its owners can do without
+// (row forms that no call uses: row_forms.cu); false when there was none.
+bool reclaim_device_memory() noexcept;
+
+// cudaMalloc, once more after reclaim_device_memory() when there is no room.
+inline cudaError_t device_malloc(void** p, uint64_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (reclaim_device_memory()) {
+            e = cudaMalloc(p, bytes);
+        }
+    }
+    return e;
+}
+
 // Owner of one device allocation on the device that was current when it was
 // allocated.
 template <typename T>
@@ -92,11 +109,12 @@ public:
         }
         const uint64_t bytes = checked_mul(count, sizeof(T), "device buffer");
         void* p = nullptr;
-        check_cuda(cudaMalloc(&p, bytes), "cannot allocate device memory");
+        check_cuda(device_malloc(&p, bytes), "cannot allocate device memory");
         ptr_ = static_cast<T*>(p);
         count_ = count;
     }
-    // allocate(), but false (and empty) when the device has no room.
+    // allocate(), but false (and empty) when the device has no room; takes nothing
+    // from others.
     bool try_allocate(uint64_t count)
     {
         release();

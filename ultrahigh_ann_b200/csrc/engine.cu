@@ -2422,6 +2422,7 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
         const bool skipped = estimable && ws->estimates_skip > 0;
         ws->estimates_skip -= skipped ? 1 : 0;
         ctx.estimates = estimable && !skipped;
+        const FormUse forms(index);
         ctx.refine_every = ws->filter_disabled || skipped;
         ctx.gathered = !queries_on_device && gather_on_host(index, n);
         if (ctx.gathered) {
@@ -2762,6 +2763,9 @@ void importance_probabilities(int device, uha_metric metric, const float* host_r
     size_t free_bytes = 0;
     size_t total_bytes = 0;
     check_cuda(cudaMemGetInfo(&free_bytes, &total_bytes), "cannot query CUDA memory");
+    if (need > free_bytes && uha::reclaim_device_memory()) {
+        check_cuda(cudaMemGetInfo(&free_bytes, &total_bytes), "cannot query CUDA memory");
+    }
     if (need > free_bytes) {
         fail(UHA_RUNTIME_ERROR, "probability working set exceeds free device memory");
     }

@@ -34,6 +34,22 @@ struct FormCall {
     uint64_t upcoming;  // of this and the call's later batches
     bool now;           // built whatever it would save (captured and tuned batches)
 };
+// While one of these lives, the index's forms are not given back.
+class FormUse {
+public:
+    explicit FormUse(const uha_index* index) : users_(index->form_users) { ++*users_; }
+    FormUse(FormUse&& other) noexcept = default;
+    FormUse& operator=(FormUse&& other) = delete;
+    ~FormUse()
+    {
+        if (users_ != nullptr) {
+            --*users_;
+        }
+    }
+
+private:
+    std::shared_ptr<std::atomic<int>> users_;
+};
 void allocate_scan_rows(uha_index* index);
 const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
                                  cudaStream_t stream);

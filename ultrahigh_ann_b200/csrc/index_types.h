@@ -5,7 +5,9 @@
 #include "common.h"
 #include "kernels.h"
 
+#include <atomic>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -127,6 +129,10 @@ struct uha_index {
     mutable uha::RowBits bits;  // L1 hierarchy
     mutable uha::FixedRows fixed;  // exact and flat L1
     mutable double form_saved = 0.0;
+    // calls and captured batches that use the forms now: they are not given back
+    // meanwhile (shared with those batches, which may outlive the index)
+    std::shared_ptr<std::atomic<int>> form_users = std::make_shared<std::atomic<int>>(0);
+    ~uha_index();
 };
 
 // A scan shape chosen by the autotuner for one (batch size, strategy) of a

@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <functional>
+#include <set>
 
 namespace uha_engine {
 
@@ -102,14 +103,39 @@ uint64_t form_bytes(const uha_index* index)
                : 0;
 }
 
-// Memory for a form: its place beside the rows, or `own`; null without room.
+// Memory for a form: its place beside the rows, or `own`; null without room. One of
+// its own takes at most half of the free memory, so another index of that size, or
+// what else the program holds on the device, still finds room.
 unsigned char* form_store(const uha_index* index, uint64_t bytes,
                           uha::DeviceBuffer<unsigned char>& own)
 {
     if (bytes <= index->form_space_bytes) {
         return index->form_space;
     }
-    return own.try_allocate(bytes) ? own.get() : nullptr;
+    size_t free_bytes = 0;
+    size_t total = 0;
+    check_cuda(cudaMemGetInfo(&free_bytes, &total), "cannot query CUDA memory");
+    return bytes <= free_bytes / 2 && own.try_allocate(bytes) ? own.get() : nullptr;
+}
+
+// The indexes that hold a form of their own.
+struct Holders {
+    std::mutex mutex;
+    std::set<const uha_index*> indexes;
+};
+
+Holders& holders()
+{
+    static Holders* all = new Holders;  // indexes may be destroyed at exit
+    return *all;
+}
+
+// After a form of its own has been published (forms_mutex held).
+void note_holder(const uha_index* index)
+{
+    Holders& all = holders();
+    std::lock_guard<std::mutex> lock(all.mutex);
+    all.indexes.insert(index);
 }
 
 // A form's build has ended, one way or the other, before its memory is given back
@@ -229,6 +255,50 @@ bool carve(uha_workspace* ws, uint64_t n, F&& layout)
 
 }  // namespace
 
+}  // namespace uha_engine
+
+// A form goes only while no call uses it (its index's next batches build it again
+// when they pay for it and there is room). Locks are only tried, and those of the
+// indexes are never held while one of the set is waited for by a thread that holds
+// the set's, so a call that allocates while it holds its own cannot wait in a circle.
+bool uha::reclaim_device_memory() noexcept
+{
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        return false;
+    }
+    uha_engine::Holders& all = uha_engine::holders();
+    std::unique_lock<std::mutex> lock(all.mutex, std::try_to_lock);
+    if (!lock.owns_lock()) {
+        return false;
+    }
+    bool any = false;
+    for (auto it = all.indexes.begin(); it != all.indexes.end();) {
+        const uha_index* index = *it;
+        std::unique_lock<std::mutex> forms(index->forms_mutex, std::try_to_lock);
+        if (index->device != device || !forms.owns_lock() || index->form_users->load() != 0) {
+            ++it;
+            continue;
+        }
+        index->split = SplitRows{};
+        index->bits = RowBits{};
+        index->fixed = FixedRows{};
+        index->form_saved = 0.0;
+        it = all.indexes.erase(it);
+        any = true;
+    }
+    return any;
+}
+
+uha_index::~uha_index()
+{
+    uha_engine::Holders& all = uha_engine::holders();
+    std::lock_guard<std::mutex> lock(all.mutex);
+    all.indexes.erase(this);
+}
+
+namespace uha_engine {
+
 bool estimates_pay(const uha_index* index, uint64_t n, uint64_t open)
 {
     const BatchTimes all = batch_times(index, n);
@@ -305,6 +375,9 @@ const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
             }
         }
         index->split = std::move(sp);
+        if (index->split.own.size() != 0) {
+            note_holder(index);
+        }
     }
     return index->split.usable ? &index->split : nullptr;
 }
@@ -331,6 +404,9 @@ const uha::RowBits* row_bits(const uha_index* index, const FormCall& call, cudaS
             rb.usable = true;
         }
         index->bits = std::move(rb);
+        if (index->bits.own.size() != 0) {
+            note_holder(index);
+        }
     }
     return index->bits.usable ? &index->bits : nullptr;
 }
@@ -368,6 +444,9 @@ const uha::FixedRows* fixed_rows(const uha_index* index, const FormCall& call,
             }
         }
         index->fixed = std::move(fx);
+        if (index->fixed.own.size() != 0) {
+            note_holder(index);
+        }
     }
     return index->fixed.usable ? &index->fixed : nullptr;
 }
