@@ -127,7 +127,8 @@ typedef struct uha_query_stats {
  * importance_sampling.hpp:23-41, l1/importance_sampling.hpp:22-40). */
 typedef struct uha_probability_report {
     uint64_t pair_count;
-    uint64_t pair_chunks;     /* launches the pairs were split into */
+    uint64_t pair_chunks;     /* chunks in effect: min(pair_chunks, pairs); the
+                                 column launches are at most this many a pass */
     uint64_t device_working_set_bytes;
     double host_to_device_ms;
     double inverse_distance_ms;
@@ -566,8 +567,10 @@ typedef enum uha_pair_backend {
  * min(1, (a_j-b_j)^2 / ||a-b||^2); L1: p_j = max over pairs of
  * |a_j-b_j| / ||a-b||_1; pairs at distance zero are skipped. Pair distances
  * and the normalisation are binary64. The per-column maxima are folded in
- * min(pair_chunks, pairs) launches over consecutive pair ranges, which bounds
- * the duration of each kernel (pair_chunks must be positive). Replaces
+ * up to min(pair_chunks, pairs) launches a pass over consecutive row ranges,
+ * which bounds the duration of each kernel (pair_chunks must be positive): no
+ * more of them than hold 2^38 pairs times columns each (about 20 ms), so
+ * smaller builds are one launch a pass whatever is asked. Replaces
  * compute_l2_importance_probabilities_gpu (include/ultrahigh_ann/hnsvw25/l2/
  * importance_sampling.hpp:49-52) and compute_l1_importance_probabilities_gpu
  * (include/ultrahigh_ann/hnsvw25/l1/importance_sampling.hpp:45-48). */
