@@ -211,15 +211,12 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
         // the certified split scan: its tile widths and column splits
         std::vector<uha::SplitPlan> cands =
             uha::split_candidates(index->rows, sp->pitch, batch, index->sm_count);
-        if (uha::split_filter_applies(cands[0], index->rows)) {
-            // the filtered form has one shape
-            if (report != nullptr) {
-                *report = rep;
-            }
-            return;
+        const bool filter = uha::split_filter_applies(cands[0], index->rows);
+        if (filter) {
+            cands.resize(1);  // the filtered form has one shape
         }
-        // the scores of every candidate go to a slab here: first the memory for the
-        // largest
+        // the scores of every candidate go to a slab here, but for the filtered form's:
+        // first the memory for the largest
         SplitBuffers buffers{};
         for (const uha::SplitPlan& p : cands) {
             if (!split_buffers(ws, index, sp->pitch, batch, p, &buffers)) {
@@ -237,10 +234,33 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
                                            sp->pitch,
                                        stream),
                        "cannot clear the query buffer");
+            // queries at the rows' centre, empty lists
+            const uint32_t slices = uha::split_slices(sp->pitch, batch);
+            check_cuda(cudaMemsetAsync(buffers.squares, 0, batch * slices * sizeof(double),
+                                       stream),
+                       "cannot clear the query norms");
+            const uha::SplitQuery sq{sp->norms,
+                                     sp->roots,
+                                     buffers.squares,
+                                     slices,
+                                     uha::split_error_rel(p, index->rows),
+                                     buffers.upper,
+                                     buffers.counts};
             const double ms = time_launches(stream, reps, [&] {
-                uha::launch_split_scores(p, sp->data, index->rows, buffers.queries, batch,
-                                         sp->pitch, buffers.partials, flag, index->sm_count,
-                                         stream);
+                if (!filter) {
+                    uha::launch_split_scores(p, sp->data, index->rows, buffers.queries, batch,
+                                             sp->pitch, buffers.partials, flag,
+                                             index->sm_count, stream);
+                    return;
+                }
+                check_cuda(cudaMemsetAsync(buffers.upper, 0xff, batch * sizeof(uint32_t),
+                                           stream),
+                           "cannot clear the query words");
+                check_cuda(cudaMemsetAsync(buffers.counts, 0, batch * sizeof(uint32_t), stream),
+                           "cannot clear the query words");
+                uha::launch_split_filter_scan(p, sp->data, index->rows, buffers.queries, batch,
+                                              sp->pitch, sq, buffers.keys, buffers.candidates,
+                                              flag, index->sm_count, stream);
             });
             if (i == 0) {
                 rep.default_ms = ms;
