@@ -343,32 +343,49 @@ def cpu_baseline(ds, index, ws, batch):
     """The reference's own ExactL2Index (oracle/_ref) on all host cores, on a
     bounded sample of the same queries, at the engine's batch size (query_batch
     calls of `batch` queries with the reference's automatic strategy: split
-    over rows for one query). Also checks the engine's answers on that sample
-    against it (agreement with the binary64 exact scan)."""
+    over rows for one query); where that library is not built, the oracle's
+    restatement of the same scan, one query per core at a time. Also checks the
+    engine's answers on that sample against it (agreement with the binary64 exact
+    scan)."""
+    from concurrent.futures import ThreadPoolExecutor
+
     from oracle import oracle as O
 
     threads = os.cpu_count() or 1
-    ref = O.RefExactIndex("l2", ds.rows)
+    if O.ref_available():
+        ref = O.RefExactIndex("l2", ds.rows)
+        kind = "reference"
+        how = (f"ExactL2Index::query_batch in calls of {batch} (automatic strategy), "
+               f"{threads} OpenMP threads")
+
+        def answer(q):
+            return ref.query_in_batches(q, batch, threads)
+    else:
+        kind = "restatement"
+        how = f"the oracle's exact L2 scan, {threads} threads of one query each"
+
+        def answer(q):
+            with ThreadPoolExecutor(threads) as pool:
+                return np.concatenate(list(pool.map(
+                    lambda i: O.exact("l2", ds.rows, q[i:i + 1])[0], range(q.shape[0]))))
     probe = ds.queries[:max(threads, batch)]
     t = time.perf_counter()
-    ref.query_in_batches(probe, batch, threads)
+    answer(probe)
     per = (time.perf_counter() - t) / probe.shape[0]
     sample = int(min(ds.queries.shape[0], max(threads, 15.0 / per)))
     step = max(threads, batch)
-    sample = max(step, sample // step * step)
+    sample = min(ds.queries.shape[0], max(step, sample // step * step))
     q = ds.queries[:sample]
     t = time.perf_counter()
-    expected = ref.query_in_batches(q, batch, threads)
+    expected = answer(q)
     secs = time.perf_counter() - t
     got = np.zeros(sample, np.uint64)
     for s in range(sample):
         index.query_batch(q[s], 1, got[s:s + 1], ws)
     agree = float(np.mean(got == expected))
     return ({"value": round(sample / secs, 3), "unit": "queries/s", "cores": threads,
-             "kind": "reference",
-             "sample": f"{sample} of the {ds.queries.shape[0]} queries, "
-                       f"ExactL2Index::query_batch in calls of {batch} "
-                       f"(automatic strategy), {threads} OpenMP threads "
+             "kind": kind,
+             "sample": f"{sample} of the {ds.queries.shape[0]} queries, {how} "
                        f"({secs:.1f} s)"}, agree)
 
 
