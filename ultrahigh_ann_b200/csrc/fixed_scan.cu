@@ -2,7 +2,7 @@
 //
 // L1 has no contraction form, so its scan is bound by CUDA-core issue: the
 // binary32 tile scan spends two instructions per (query, row, column). As in
-// the split scan of L2 (split_scan.cu), an estimate with a proven error is
+// the split scan of L2 (split_scan.cu), an estimate with a bounded error is
 // enough to list the rows that can be a query's minimum. Per column, with its
 // smallest value o over the index's rows, its weight w (1 unless weighted) and
 // one step s for all columns, a value x becomes the integer

@@ -1,7 +1,7 @@
 // Certified L2 scan of larger batches on the tensor cores.
 //
 // The certified path needs the reference CPU's binary64 argmin, not binary32
-// distances of every row: any estimate with a proven error decides which rows
+// distances of every row: any estimate with a bounded error decides which rows
 // can be the minimum, and those few are settled from the original values in
 // binary64 (certify.cu). The binary32 tile scan spends two CUDA-core
 // instructions per (query, row, column) on that; here the estimate is a
@@ -21,7 +21,8 @@
 //     instruction aligns its products and the accumulator to the largest of
 //     them, keeps 2^-25 of it, adds and truncates to 24 bits: at most
 //     10.5 * 2^-24 of the magnitudes added (17 truncations and the last one);
-//     2^-19 is assumed                                4.1 * 2^-19 a b
+//     2^-19, three times that, is assumed (of all these terms the one that rests
+//     on a measurement)                               4.1 * 2^-19 a b
 //   binary32 sums of the chunks and splits           (chunks + splits) 2^-24 a b
 //   the centring's rounding, the norm's, the last
 //     roundings and the reference's own               2^-21 (a + b)^2
