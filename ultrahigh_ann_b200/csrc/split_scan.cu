@@ -416,7 +416,9 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                 // in flight behind the wait for the accumulator
                 const bool row_ok = scored < row_count;
                 const float b = row_ok ? sq.roots[row] : 0.f;
-                const float norm = row_ok ? sq.norms[row] : inf;
+                // a NaN: a row past the end passes no comparison (infinity would pass
+                // against an infinite side; the least pass takes whole tiles only)
+                const float norm = row_ok ? sq.norms[row] : __int_as_float(0x7fffffff);
                 if (query_tile(unit) != loaded_tile) {
                     loaded_tile = query_tile(unit);
                     __syncwarp();
@@ -441,8 +443,7 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                 if (!accumulated()) {
                     break;
                 }
-                // the row's side. A row past the end has none: it is masked out
-                // below (the least pass takes whole tiles only)
+                // the row's side
                 const float square = __fmul_ru(0x1p-21f, __fmul_ru(b, b));
                 const float low = MODE == Score::filter ? __fsub_rd(norm, square)
                                                         : __fadd_ru(norm, square);
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                             most = fmaxf(most, fmaxf(filter_side(l.x, l.y, b, v[j]),
                                                      filter_side(l.z, l.w, b, v[j + 1])));
                         }
-                        if (!__any_sync(0xffffffffu, row_ok && most >= low)) {
+                        if (!__any_sync(0xffffffffu, most >= low)) {
                             continue;
                         }
                         // the lane's passing columns, taken one per turn
@@ -486,7 +487,6 @@ __global__ void __launch_bounds__(Epilogue<BN, MODE>::threads, 1)
                             bits |= filter_side(l.x, l.y, b, v[j]) >= low ? 1u << j : 0u;
                             bits |= filter_side(l.z, l.w, b, v[j + 1]) >= low ? 2u << j : 0u;
                         }
-                        bits = row_ok ? bits : 0u;
                         for (uint32_t mask = __ballot_sync(0xffffffffu, bits != 0u); mask != 0u;
                              mask = __ballot_sync(0xffffffffu, bits != 0u)) {
                             if (bits != 0u) {
