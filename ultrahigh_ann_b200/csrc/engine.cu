@@ -1491,7 +1491,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
     v.columns = query_columns(c);
     v.weights = index->weights64.get();
     v.offsets = rows.offsets;
-    v.step = rows.offsets + rows.pitch;
+    v.step = rows.step;
     v.out = buffers.queries;
     v.pitch = rows.pitch;
     v.prepared = ws->prepared.get();

@@ -33,7 +33,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
-#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -67,7 +66,6 @@ __host__ __device__ constexpr double largest_error(uint64_t dim)
 constexpr uint64_t kNarrowColumns = 32000;
 static_assert(65535.0 * kNarrowColumns + largest_error(kNarrowColumns) < 2147483647.0,
               "the narrow epilogue's differences fit 32 bits");
-constexpr uint32_t kPairs = 64;          // row pairs of the quality estimate
 constexpr float kLevels = 65535.f;
 
 __device__ __forceinline__ unsigned int ordered(float f)
@@ -100,7 +98,8 @@ __device__ __forceinline__ double block_total(double v, double* scratch)
 
 // ---------------------------------------------------------------- index side
 
-// Ordered bits of each column's smallest and largest value. grid (columns, slices
+// Ordered bits (the smallest's inverted, so both grow from 0) of each column's
+// smallest and largest value. grid (columns, slices
 // of kRangeRows rows); a grid of kRangeSlices takes every so many-th slice.
 __global__ void __launch_bounds__(kThreads)
     column_range_kernel(const float* __restrict__ rows, uint32_t row_count, uint64_t padded,
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(kThreads)
             b = fmaxf(b, x);
         }
     }
-    atomicMin(low + j, ordered(a));
+    atomicMax(low + j, ~ordered(a));
     atomicMax(high + j, ordered(b));
 }
 
@@ -139,7 +138,7 @@ __global__ void __launch_bounds__(kThreads)
     const uint64_t j = blockIdx.x * static_cast<uint64_t>(kThreads) + threadIdx.x;
     float s = 0.f;
     if (j < pitch) {
-        const float o = j < dim ? from_ordered(low[j]) : 0.f;
+        const float o = j < dim ? from_ordered(~low[j]) : 0.f;
         offsets[j] = o;
         if (j < dim) {
             const double range =
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-// L1 distances of kPairs spread pairs of rows, for the host's estimate of
+// L1 distances of kFixedPairs spread pairs of rows, for the host's estimate of
 // whether the step is fine enough for this index.
 __global__ void __launch_bounds__(kThreads)
     pair_sample_kernel(const float* __restrict__ rows, uint32_t row_count, uint64_t padded,
@@ -603,27 +602,15 @@ uint64_t fixed_pitch(uint64_t dim)
     return round_up(dim == 0 ? 1 : dim, kStageColumns);
 }
 
-uint64_t fixed_scratch_words(uint64_t dim)
-{
-    // column ranges, the sampled pairs' distances, the coarse-row flag
-    return round_up(2 * dim, 2) + 2 * kPairs + 2;
-}
-
 void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, uint64_t dim,
                        const double* weights, uint16_t* out, uint64_t pitch, float* offsets,
-                       float* step, FixedTerms* terms, unsigned int* scratch, cudaStream_t stream)
+                       FixedSummary* summary, FixedTerms* terms, unsigned int* ranges,
+                       cudaStream_t stream)
 {
     const uint32_t rc = static_cast<uint32_t>(row_count);
-    unsigned int* low = scratch;
-    unsigned int* high = scratch + dim;
-    double* pairs = reinterpret_cast<double*>(scratch + round_up(2 * dim, 2));
-    check_cuda(cudaMemsetAsync(low, 0xff, dim * sizeof(unsigned int), stream),
-               "cannot clear column ranges");
-    check_cuda(cudaMemsetAsync(high, 0, dim * sizeof(unsigned int), stream),
-               "cannot clear column ranges");
-    check_cuda(cudaMemsetAsync(step, 0, sizeof(float), stream), "cannot clear the step");
-    check_cuda(cudaMemsetAsync(pairs + kPairs, 0, sizeof(double), stream),
-               "cannot clear the row error flag");
+    unsigned int* low = ranges;
+    unsigned int* high = ranges + dim;
+    float* step = &summary->step;
     const uint32_t column_blocks = static_cast<uint32_t>((dim + kThreads - 1) / kThreads);
     const uint32_t slices = std::min((rc + kRangeRows - 1) / kRangeRows, kRangeSlices);
     column_range_kernel<<<dim3(column_blocks, slices), kThreads, 0, stream>>>(rows, rc, padded,
@@ -632,7 +619,8 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     column_offset_kernel<<<static_cast<uint32_t>((pitch + kThreads - 1) / kThreads), kThreads, 0,
                            stream>>>(low, high, dim, pitch, weights, offsets,
                                      reinterpret_cast<unsigned int*>(step));
-    pair_sample_kernel<<<kPairs, kThreads, 0, stream>>>(rows, rc, padded, dim, weights, pairs);
+    pair_sample_kernel<<<kFixedPairs, kThreads, 0, stream>>>(rows, rc, padded, dim, weights,
+                                                             summary->pairs);
     FixedVectors v{};
     v.source_pitch = padded;
     v.dim = dim;
@@ -642,7 +630,7 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     v.pitch = pitch;
     v.slice = pitch;
     v.vector_loads = true;  // rows are padded to 16-byte boundaries
-    v.error_flag = reinterpret_cast<int*>(pairs + kPairs);
+    v.error_flag = &summary->coarse;
     for (uint64_t at = 0; at < row_count; at += 65535) {
         const uint64_t count = std::min<uint64_t>(65535, row_count - at);
         v.source = rows + at * padded;
@@ -654,36 +642,32 @@ void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, u
     check_cuda(cudaGetLastError(), "cannot launch the fixed-point row kernels");
 }
 
-bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* terms,
-                  uint64_t row_count, const float* device_step, cudaStream_t stream)
+bool fixed_usable(const FixedSummary* summary, uint64_t row_count, cudaStream_t stream)
 {
-    double pairs[kPairs + 1];  // the last: the flag
-    FixedTerms errors[kPairs];
-    float step = 0.f;
-    const uint64_t count = std::min<uint64_t>(row_count, kPairs);
-    check_cuda(cudaMemcpyAsync(pairs, scratch + round_up(2 * dim, 2), sizeof(pairs),
+    // the summary and the first rows' terms behind it, in one copy
+    struct {
+        FixedSummary sum;
+        FixedTerms terms[kFixedPairs];
+    } host;
+    static_assert(sizeof(FixedSummary) % alignof(FixedTerms) == 0, "terms follow the summary");
+    const uint64_t count = std::min<uint64_t>(row_count, kFixedPairs);
+    check_cuda(cudaMemcpyAsync(&host, summary, sizeof(FixedSummary) + count * sizeof(FixedTerms),
                                cudaMemcpyDeviceToHost, stream),
-               "cannot copy sampled distances from the CUDA device");
-    check_cuda(cudaMemcpyAsync(errors, terms, count * sizeof(FixedTerms),
-                               cudaMemcpyDeviceToHost, stream),
-               "cannot copy row errors from the CUDA device");
-    check_cuda(cudaMemcpyAsync(&step, device_step, sizeof(step), cudaMemcpyDeviceToHost, stream),
-               "cannot copy the step from the CUDA device");
+               "cannot copy the rows' errors from the CUDA device");
     check_cuda(cudaStreamSynchronize(stream), "cannot build fixed-point rows");
-    int coarse = 0;
-    std::memcpy(&coarse, pairs + kPairs, sizeof(coarse));
     double distance = 0.0;
-    for (uint32_t i = 0; i < kPairs; ++i) {
-        distance += pairs[i] / kPairs;
+    for (double d : host.sum.pairs) {
+        distance += d / kFixedPairs;
     }
     double error = 0.0;
     for (uint64_t i = 0; i < count; ++i) {
-        error += static_cast<double>(errors[i].error) / static_cast<double>(count);
+        error += static_cast<double>(host.terms[i].error) / static_cast<double>(count);
     }
+    const float step = host.sum.step;
     // two vectors' errors within 1/512 of a typical distance: rows closer together
     // than that are rare enough for the candidate lists
-    return coarse == 0 && std::isfinite(step) && std::isfinite(distance) && step >= 0x1p-100f &&
-           1024.0 * error * static_cast<double>(step) <= distance;
+    return host.sum.coarse == 0 && std::isfinite(step) && std::isfinite(distance) &&
+           step >= 0x1p-100f && 1024.0 * error * static_cast<double>(step) <= distance;
 }
 
 uint32_t fixed_slices(uint64_t pitch, uint64_t batch)

@@ -50,13 +50,14 @@ struct SplitRows {
 
 // The fixed-point form of an exact or flat L1 index's rows (fixed_scan.cu),
 // built on first use, in one allocation or the place beside the rows: each row's
-// terms, the column offsets and the step, the build's scratch, rows x pitch 16-bit
+// terms, the column offsets and the step, the build's ranges, rows x pitch 16-bit
 // values. `usable` is false when the memory was not available or the step does not
 // resolve the index's distances.
 struct FixedRows {
     DeviceBuffer<unsigned char> own;
     const FixedTerms* terms = nullptr;
-    const float* offsets = nullptr;  // pitch values, then the step
+    const float* offsets = nullptr;  // pitch values
+    const float* step = nullptr;
     const uint16_t* data = nullptr;
     uint64_t pitch = 0;
     bool ready = false;

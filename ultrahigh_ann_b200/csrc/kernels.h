@@ -368,7 +368,8 @@ uint64_t split_pitch(uint64_t dim);
 // The largest vector norm the estimates' bound covers.
 float split_largest_norm();
 // The centre (pitch floats) of the rows, and of the centred rows times `scale`
-// (a power of two) the split parts, squared norms and roots; *largest: bits of the largest root (infinity when one is not finite).
+// (a power of two) the split parts, squared norms and roots; *largest (0 before):
+// bits of the largest root (infinity when one is not finite).
 // `out` is zero where no value is stored.
 void launch_split_rows(const float* rows, uint64_t row_count, uint64_t src_pitch, uint64_t dim,
                        void* out, uint64_t pitch, float scale, float* centre, float* norms,
@@ -507,18 +508,26 @@ struct FixedPlan {
     uint32_t columns_per_split;
 };
 uint64_t fixed_pitch(uint64_t dim);
+// What the host reads of a build: L1 distances of spread pairs of rows, the step,
+// whether some row's error is past what the arithmetic allows. The rows' terms lie
+// behind it.
+constexpr uint32_t kFixedPairs = 64;
+struct alignas(16) FixedSummary {
+    double pairs[kFixedPairs];
+    float step;
+    int coarse;
+};
 // The most rows the fixed-point scan takes.
 constexpr uint64_t kFixedRows = 1ull << 24;
-uint64_t fixed_scratch_words(uint64_t dim);
 // The rows (padded, weights nullable) in fixed point: row_count x pitch values,
-// offsets (pitch), the step and each row's terms; scratch:
-// fixed_scratch_words(dim).
+// offsets (pitch), the summary and each row's terms; ranges: 2 x dim words. The
+// ranges and the summary are zero before.
 void launch_fixed_rows(const float* rows, uint64_t row_count, uint64_t padded, uint64_t dim,
                        const double* weights, uint16_t* out, uint64_t pitch, float* offsets,
-                       float* step, FixedTerms* terms, unsigned int* scratch, cudaStream_t stream);
+                       FixedSummary* summary, FixedTerms* terms, unsigned int* ranges,
+                       cudaStream_t stream);
 // Whether the step resolves this index's distances (synchronises `stream`).
-bool fixed_usable(const unsigned int* scratch, uint64_t dim, const FixedTerms* terms,
-                  uint64_t row_count, const float* step, cudaStream_t stream);
+bool fixed_usable(const FixedSummary* summary, uint64_t row_count, cudaStream_t stream);
 uint32_t fixed_slices(uint64_t pitch, uint64_t batch);
 void launch_fixed_queries(FixedVectors v, uint64_t batch, cudaStream_t stream);
 FixedPlan plan_fixed(uint64_t rows, uint64_t pitch, uint64_t batch, int sm_count);

@@ -45,11 +45,12 @@ struct Parts {
 
 struct SplitLayout {
     Parts parts;
-    uint64_t data, norms, roots, centre;
+    uint64_t data, largest, norms, roots, centre;
     SplitLayout(uint64_t rows, uint64_t pitch)
         : data(parts.take(checked_mul(uha::lowp_padded_count(rows), pitch, "split rows"), 4)),
+          largest(parts.take(1, sizeof(uint32_t))),  // of the roots; cleared with the data's end
           norms(parts.take(rows, sizeof(float))),
-          roots(parts.take(rows + 1, sizeof(float))),  // and the largest of them
+          roots(parts.take(rows, sizeof(float))),
           centre(parts.take(pitch, sizeof(float)))
     {
     }
@@ -57,11 +58,15 @@ struct SplitLayout {
 
 struct FixedLayout {
     Parts parts;
-    uint64_t terms, offsets, scratch, data;
+    uint64_t ranges, summary, offsets, data;
     FixedLayout(uint64_t rows, uint64_t dim, uint64_t pitch)
-        : terms(parts.take(rows, sizeof(uha::FixedTerms))),
-          offsets(parts.take(pitch + 1, sizeof(float))),  // and the step
-          scratch(parts.take(uha::fixed_scratch_words(dim), sizeof(uint32_t))),
+        : ranges(parts.take(2 * dim, sizeof(uint32_t))),  // cleared with the summary
+          // the summary, and the rows' terms right behind it
+          summary(parts.take(uha::checked_add(
+                                 sizeof(uha::FixedSummary) / sizeof(uha::FixedTerms), rows,
+                                 "fixed-point rows"),
+                             sizeof(uha::FixedTerms))),
+          offsets(parts.take(pitch, sizeof(float))),
           data(parts.take(checked_mul(rows, pitch, "fixed-point rows"), sizeof(uint16_t)))
     {
     }
@@ -340,13 +345,13 @@ const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
             sp.norms = part<float>(base, at.norms);
             sp.roots = part<float>(base, at.roots);
             sp.centre = part<float>(base, at.centre);
-            unsigned int* largest = reinterpret_cast<unsigned int*>(sp.roots + index->rows);
-            // the split writes every row's whole pitch; the vectors past the rows are
-            // zero
+            unsigned int* largest = part<unsigned int>(base, at.largest);
             const uint64_t used = index->rows * pitch * 4;
-            check_cuda(cudaMemsetAsync(sp.data + used, 0, at.norms - used, stream),
-                       "cannot clear split rows");
             auto split = [&] {
+                // the split writes every row's whole pitch; the vectors past the rows
+                // are zero
+                check_cuda(cudaMemsetAsync(sp.data + used, 0, at.norms - used, stream),
+                           "cannot clear split rows");
                 if (index->kind == IndexKind::hierarchical) {
                     uha::launch_split_rows(index->rows64.get(), index->rows, index->scan_dim,
                                            index->scan_dim, sp.data, pitch, sp.scale, sp.centre,
@@ -427,18 +432,22 @@ const uha::FixedRows* fixed_rows(const uha_index* index, const FormCall& call,
         fx.pitch = pitch;
         unsigned char* base = form_store(index, at.parts.bytes, fx.own);
         if (base != nullptr) {
-            uha::FixedTerms* terms = part<uha::FixedTerms>(base, at.terms);
+            uha::FixedSummary* summary = part<uha::FixedSummary>(base, at.summary);
+            uha::FixedTerms* terms = reinterpret_cast<uha::FixedTerms*>(summary + 1);
             float* offsets = part<float>(base, at.offsets);
-            unsigned int* words = part<unsigned int>(base, at.scratch);
             uint16_t* data = part<uint16_t>(base, at.data);
             fx.terms = terms;
             fx.offsets = offsets;
+            fx.step = &summary->step;
             fx.data = data;
+            check_cuda(cudaMemsetAsync(base + at.ranges, 0,
+                                       at.summary + sizeof(uha::FixedSummary) - at.ranges,
+                                       stream),
+                       "cannot clear column ranges");
             uha::launch_fixed_rows(index->scan_rows.get(), index->rows, index->padded_dim,
                                    index->scan_dim, index->weights64.get(), data, pitch, offsets,
-                                   offsets + pitch, terms, words, stream);
-            fx.usable = uha::fixed_usable(words, index->scan_dim, terms, index->rows,
-                                          offsets + pitch, stream);
+                                   summary, terms, part<unsigned int>(base, at.ranges), stream);
+            fx.usable = uha::fixed_usable(summary, index->rows, stream);
             if (!fx.usable) {
                 fx.own.release();
             }

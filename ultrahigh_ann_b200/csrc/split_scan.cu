@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kPrepThreads)
     double acc = 0.0;
     int bad = 0;
     // four columns per thread and step; slices and pitch are multiples of 64
-    for (uint64_t j = begin + 4ull * threadIdx.x; j < end; j += 4ull * kPrepThreads) {
+    for (uint64_t j = begin + 4ull * threadIdx.x; j < end; j += 4ull * blockDim.x) {
         alignas(8) __nv_bfloat16 hi[4];
         alignas(8) __nv_bfloat16 lo[4];
         T x[4];
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(kPrepThreads)
         return;
     }
     double total = 0.0;
-    for (int w = 0; w < kPrepThreads / 32; ++w) {
+    for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
         total += scratch[w];
     }
     if constexpr (kRows) {
@@ -955,6 +955,13 @@ void launch_split_tiles(const SplitPlan& plan, const void* rows, uint64_t row_co
     }
 }
 
+// Threads of a slice's block: four columns each, at most kPrepThreads.
+uint32_t prep_threads(uint64_t slice)
+{
+    return static_cast<uint32_t>(
+        std::min<uint64_t>(kPrepThreads, round_up((slice + 3) / 4, 32)));
+}
+
 template <typename T, SplitSource SRC>
 void split_rows_typed(const T* rows, uint64_t row_count, uint64_t src_pitch, uint64_t dim,
                       void* out, uint64_t pitch, float scale, float* centre, float* norms,
@@ -980,11 +987,9 @@ void split_rows_typed(const T* rows, uint64_t row_count, uint64_t src_pitch, uin
         v.out = static_cast<__nv_bfloat16*>(out) + at * 2 * pitch;
         v.norms = norms + at;
         v.roots = roots + at;
-        split_vectors_kernel<SRC><<<dim3(1, static_cast<uint32_t>(count)), kPrepThreads, 0,
-                                    stream>>>(v);
+        split_vectors_kernel<SRC><<<dim3(1, static_cast<uint32_t>(count)),
+                                    prep_threads(v.slice), 0, stream>>>(v);
     }
-    check_cuda(cudaMemsetAsync(largest, 0, sizeof(unsigned int), stream),
-               "cannot clear the largest norm");
     largest_root_kernel<<<64, 256, 0, stream>>>(roots, row_count, largest);
     check_cuda(cudaGetLastError(), "cannot launch the row splitting kernels");
 }
@@ -1036,14 +1041,15 @@ void launch_split_queries(SplitVectors v, uint64_t batch, bool projected, cudaSt
     const uint32_t slices = split_slices(v.pitch, batch);
     v.slice = round_up((v.pitch + slices - 1) / slices, kStageColumns);
     const dim3 grid(slices, static_cast<uint32_t>(batch));
+    const uint32_t threads = prep_threads(v.slice);
     if (projected) {
-        split_vectors_kernel<SplitSource::projected><<<grid, kPrepThreads, 0, stream>>>(v);
+        split_vectors_kernel<SplitSource::projected><<<grid, threads, 0, stream>>>(v);
     } else if (v.columns != nullptr) {
-        split_vectors_kernel<SplitSource::sampled><<<grid, kPrepThreads, 0, stream>>>(v);
+        split_vectors_kernel<SplitSource::sampled><<<grid, threads, 0, stream>>>(v);
     } else {
         v.vector_loads = v.source_pitch % 4 == 0 &&
                          reinterpret_cast<uintptr_t>(v.source) % 16 == 0;
-        split_vectors_kernel<SplitSource::dense><<<grid, kPrepThreads, 0, stream>>>(v);
+        split_vectors_kernel<SplitSource::dense><<<grid, threads, 0, stream>>>(v);
     }
     check_cuda(cudaGetLastError(), "cannot launch the query splitting kernel");
 }
