@@ -8,7 +8,7 @@
 // would have saved its cost, and a call's scan buffers are parts of one: the
 // workspace's query buffer where its largest batch needs up to kReservedScan, else
 // one of their own. First batch of a new index and workspace, 65,536 x 128 (L1), 256
-// queries: 0.81 ms by the binary32 scan (one allocation), 1.29 ms with five, 0.29 ms
+// queries: 0.81 ms by the binary32 scan (one allocation), 1.33 ms with five, 0.27 ms
 // with none.
 #include "engine_internal.h"
 
