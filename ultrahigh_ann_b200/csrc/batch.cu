@@ -608,20 +608,25 @@ uint64_t answer_pair(uha_batch::Pair& p)
             open.push_back(q);
         }
     }
-    if (p.again == nullptr || p.again->max_batch < open.size()) {
+    uint64_t most = std::min<uint64_t>(open.size(), kOpenBatch);
+    if (p.again == nullptr || p.again->max_batch < most) {
         if (p.again != nullptr) {
             uha_workspace_destroy(p.again);
             p.again = nullptr;
         }
-        const uha_status status =
-            create_workspace(p.index, open.size(), false, &p.again);
+        // fewer queries at a time where there is little room
+        uha_status status = create_workspace(p.index, most, false, &p.again);
+        while (no_device_memory(status) && most > 64) {
+            most /= 2;
+            status = create_workspace(p.index, most, false, &p.again);
+        }
         if (status != UHA_OK) {
             fail(status, uha_last_error());
         }
         p.again->candidates_per_query = ws->candidates_per_query;
     }
     const uha_query_stats more =
-        answer_open(p.index, p.again, ws->raw_queries.get(), open, open.size(), p.strategy, true,
+        answer_open(p.index, p.again, ws->raw_queries.get(), open, most, p.strategy, true,
                     ws->host_results.get(), ws->host_exact.get());
     uint32_t* words = ws->host_counters.get();
     words[0] = (left != 0 ? words[0] : 0u) + static_cast<uint32_t>(more.replayed_queries);

@@ -59,6 +59,8 @@ inline uint64_t round_up(uint64_t value, uint64_t multiple)
     return (value + multiple - 1) / multiple * multiple;
 }
 
+constexpr char kNoDeviceMemory[] = "cannot allocate device memory";
+
 // Gives back device memory of the current device that its owners can do without
 // (row forms that no call uses: row_forms.cu); false when there was none.
 bool reclaim_device_memory() noexcept;
@@ -109,7 +111,7 @@ public:
         }
         const uint64_t bytes = checked_mul(count, sizeof(T), "device buffer");
         void* p = nullptr;
-        check_cuda(device_malloc(&p, bytes), "cannot allocate device memory");
+        check_cuda(device_malloc(&p, bytes), kNoDeviceMemory);
         ptr_ = static_cast<T*>(p);
         count_ = count;
     }
@@ -125,7 +127,7 @@ public:
             cudaGetLastError();
             return false;
         }
-        check_cuda(e, "cannot allocate device memory");
+        check_cuda(e, kNoDeviceMemory);
         ptr_ = static_cast<T*>(p);
         count_ = count;
         return true;

@@ -1380,6 +1380,15 @@ FormCall form_call(const BatchContext& c, uint64_t n)
     return {n, std::max(n, c.upcoming), c.build_forms};
 }
 
+// No room for a batch's scan buffers: the workspace keeps the binary32 scans, and the
+// memory that the estimates took is theirs.
+void give_up_estimates(const BatchContext& c)
+{
+    c.ws->split_disabled = true;
+    c.ws->scan_store.release();
+    drop_form(c.index);
+}
+
 // The bitmap form of this batch's median scan (everything it needs allocated
 // here), or null when it takes the binary32 passes.
 const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuffers* buffers)
@@ -1394,7 +1403,7 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuf
     }
     const uha::RowBits* bits = row_bits(index, form_call(c, n), ws->stream);
     if (bits != nullptr && !bits_buffers(ws, index, n, buffers)) {
-        ws->split_disabled = true;
+        give_up_estimates(c);
         return nullptr;
     }
     return bits;
@@ -1467,7 +1476,7 @@ const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::Fixe
     }
     *plan = uha::plan_fixed(index->rows, fx->pitch, n, index->sm_count);
     if (!fixed_buffers(ws, index, fx->pitch, n, *plan, buffers)) {
-        ws->split_disabled = true;
+        give_up_estimates(c);
         return nullptr;
     }
     return fx;
@@ -1561,7 +1570,7 @@ bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** row
                 : uha::plan_split(index->rows, sp->pitch, n, index->sm_count);
     *rows = sp;
     if (!split_buffers(ws, index, sp->pitch, n, *plan, buffers)) {
-        ws->split_disabled = true;
+        give_up_estimates(c);
         return false;
     }
     return true;
@@ -2153,6 +2162,12 @@ void finish_call(const uha_index* index, uha_workspace* ws, uint64_t n,
     ws->last.certified_queries = n - std::min<uint64_t>(n, replayed);
 }
 
+bool no_device_memory(uha_status status)
+{
+    return status == UHA_RUNTIME_ERROR &&
+           std::strstr(uha_last_error(), uha::kNoDeviceMemory) != nullptr;
+}
+
 std::vector<uint64_t> open_queries(const uha::Result* results, uint64_t n)
 {
     std::vector<uint64_t> open;
@@ -2170,12 +2185,13 @@ uha_query_stats answer_open(const uha_index* index, uha_workspace* ws, const flo
                             double* exact)
 {
     const uint64_t d = index->dimension;
-    const uint64_t most = std::min<uint64_t>({batch, ws->max_batch, open.size()});
+    uint64_t most = std::min<uint64_t>({batch, ws->max_batch, open.size(), kOpenBatch});
     std::vector<uint64_t> rows(most);
     std::vector<double> distances(want_distances ? most : 0);
     uha_query_stats total{};
-    for (uint64_t at = 0; at < open.size(); at += most) {
-        const uint64_t count = std::min<uint64_t>(most, open.size() - at);
+    uint64_t count = 0;
+    for (uint64_t at = 0; at < open.size(); at += count) {
+        count = std::min<uint64_t>(most, open.size() - at);
         // runs of consecutive queries, one copy each
         for (uint64_t i = 0, run = 0; i < count; i += run) {
             run = 1;
@@ -2192,6 +2208,11 @@ uha_query_stats answer_open(const uha_index* index, uha_workspace* ws, const flo
             uha_query_many(index, ws, ws->raw_queries.get(), count, count, 1, strategy,
                            rows.data(), want_distances ? distances.data() : nullptr);
         ws->filter_disabled = false;
+        if (no_device_memory(status) && count > 64) {
+            most = count / 2;
+            count = 0;
+            continue;
+        }
         if (status != UHA_OK) {
             fail(status, uha_last_error());
         }
@@ -2368,11 +2389,42 @@ extern "C" uha_status uha_query(const uha_index* index, uha_workspace* ws,
                           queries_on_device, strategy, out_indices, out_distances);
 }
 
+namespace {
+
+uha_status query_once(const uha_index* index, uha_workspace* ws, const float* queries,
+                      uint64_t query_count, uint64_t batch, int queries_on_device,
+                      uha_strategy strategy, uint64_t* out_indices, double* out_distances);
+
+}  // namespace
+
 extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
                                      const float* queries, uint64_t query_count,
                                      uint64_t batch, int queries_on_device,
                                      uha_strategy strategy, uint64_t* out_indices,
                                      double* out_distances)
+{
+    const uha_status status = query_once(index, ws, queries, query_count, batch,
+                                         queries_on_device, strategy, out_indices,
+                                         out_distances);
+    if (no_device_memory(status) && ws->scan_store.size() != 0) {
+        // no room beside the buffers that estimating calls left
+        const uha_status released = guarded([&] {
+            DeviceGuard guard(ws->device);
+            ws->scan_store.release();
+        });
+        return released != UHA_OK
+                   ? released
+                   : query_once(index, ws, queries, query_count, batch, queries_on_device,
+                                strategy, out_indices, out_distances);
+    }
+    return status;
+}
+
+namespace {
+
+uha_status query_once(const uha_index* index, uha_workspace* ws, const float* queries,
+                      uint64_t query_count, uint64_t batch, int queries_on_device,
+                      uha_strategy strategy, uint64_t* out_indices, double* out_distances)
 {
     return guarded([&] {
         require(batch != 0, UHA_INVALID_ARGUMENT, "batch size must be positive");
@@ -2595,6 +2647,8 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
                     out_indices, out_distances);
     });
 }
+
+}  // namespace
 
 extern "C" uha_status uha_workspace_set_replay(uha_workspace* workspace,
                                                uha_replay_arithmetic arithmetic)

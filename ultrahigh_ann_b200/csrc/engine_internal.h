@@ -51,6 +51,10 @@ private:
     std::shared_ptr<std::atomic<int>> users_;
 };
 void allocate_scan_rows(uha_index* index);
+// Gives the index's form back when only the calling thread uses it (it is built again
+// when it pays): a call that finds no room for its scan buffers needs the memory for
+// the binary32 scan's.
+void drop_form(const uha_index* index);
 const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
                                  cudaStream_t stream);
 const uha::FixedRows* fixed_rows(const uha_index* index, const FormCall& call,
@@ -182,10 +186,17 @@ void finish_call(const uha_index* index, uha_workspace* ws, uint64_t n,
                  const uha::Result* results, const double* exact,
                  uint64_t* out_indices, double* out_distances);
 
+// Open queries answered at a time: enough for the binary32 scan to fill the chip, and
+// its sums (of each query and row) stay small beside the estimates' that are held.
+constexpr uint64_t kOpenBatch = 1024;
+
+// A call's status and message say that an allocation found no room.
+bool no_device_memory(uha_status status);
+
 // The queries of a call that the estimating scans left open.
 std::vector<uint64_t> open_queries(const uha::Result* results, uint64_t n);
 // Answers them by the binary32 scans into results and exact, in batches of at most
-// `batch` on ws (whose query buffer, status words and last stats it overwrites);
+// `batch` (and kOpenBatch) on ws (whose query buffer, status words and last stats it overwrites);
 // queries: host or device, n x dimension. Returns the stats of these calls, added
 // up.
 uha_query_stats answer_open(const uha_index* index, uha_workspace* ws, const float* queries,

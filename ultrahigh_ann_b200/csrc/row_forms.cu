@@ -304,6 +304,18 @@ uha_index::~uha_index()
 
 namespace uha_engine {
 
+void drop_form(const uha_index* index)
+{
+    std::lock_guard<std::mutex> lock(index->forms_mutex);
+    if (index->form_users->load() <= 1) {
+        // (cudaFree waits for the batches of this call that still read it)
+        index->split = uha::SplitRows{};
+        index->bits = uha::RowBits{};
+        index->fixed = uha::FixedRows{};
+        index->form_saved = 0.0;
+    }
+}
+
 bool estimates_pay(const uha_index* index, uint64_t n, uint64_t open)
 {
     const BatchTimes all = batch_times(index, n);
