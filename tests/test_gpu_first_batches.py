@@ -67,18 +67,20 @@ def test_a_large_form_is_built_when_it_pays(metric):
     d = (rows[at].double() - queries.double())
     exact = (d.square() if metric == "l2" else d.abs()).sum(1).cpu().numpy()
     ws = index.make_query_workspace(64)
-    launches = []
+    launches, first = [], None
     for n in [9] * 12 + [64]:
         out, dist = np.zeros(n, np.uint64), np.zeros(n)
         index.query_device_batch(queries.data_ptr(), n, out, ws, distances=dist)
         assert np.array_equal(out, at[:n].cpu().numpy().astype(np.uint64))
-        np.testing.assert_allclose(dist, exact[:n], rtol=1e-5)
+        np.testing.assert_allclose(dist, exact[:n], rtol=1e-10)
         launches.append(ws.last_stats()["kernel_launches"])
-    # preparation, scan and argmin; then the estimating scan, for good
-    assert launches[0] == 3 and launches[-2] > 3
+        first = dist if first is None else first
+    # preparation, scan, argmin and the winners' distances; then the estimating scan,
+    # for good, with the same bits
+    assert launches[0] == 4 and launches[-2] > 4
+    assert np.array_equal(first, dist[:9])
     changes = [a != b for a, b in zip(launches[:-1], launches[1:-1])]
     assert sum(changes) == 1
-    np.testing.assert_allclose(dist, exact, rtol=1e-10)
 
 
 @pytest.mark.parametrize("kind", KINDS)

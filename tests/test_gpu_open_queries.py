@@ -152,3 +152,21 @@ def test_projections_past_the_bound(oracle_module, kind):
     dist = np.zeros(60)
     out = index.query_batch(queries, 60, None, ws, distances=dist)
     _compare(out, dist, expected, edist, [11])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_skipped_calls_report_binary64_distances(oracle_module, kind):
+    index, queries, (expected, edist) = _case(oracle_module, kind, 7, 40, slice(0, 36))
+    _, plain, (pexpected, pedist) = _case(oracle_module, kind, 7, 40, [])
+    ws = index.make_query_workspace(40)
+    estimated = np.zeros(40)
+    index.query_batch(plain, 40, None, ws, distances=estimated)
+    for _ in range(2):                  # left open; the next call skips the estimates
+        dist = np.zeros(40)
+        assert np.array_equal(index.query_batch(queries, 40, None, ws, distances=dist), expected)
+        np.testing.assert_allclose(dist, edist, rtol=1e-10, atol=1e-30)
+    index.query_batch(queries, 40, None, ws)
+    dist = np.zeros(40)                 # skipped
+    assert np.array_equal(index.query_batch(plain, 40, None, ws, distances=dist), pexpected)
+    np.testing.assert_allclose(dist, pedist, rtol=1e-10)
+    np.testing.assert_allclose(dist, estimated, rtol=1e-13)

@@ -205,7 +205,7 @@ void autotune(const uha_index* index, uha_workspace* ws, uint64_t batch,
     } else if (const uha::SplitRows* sp =
                    !ws->split_disabled && split_shape(index, strategy, batch) &&
                            (!ws->emulated_replay || index->kind == IndexKind::hierarchical)
-                       ? split_rows(index, FormCall{batch, batch, true}, stream)
+                       ? split_rows(index, FormCall{batch, batch, true, nullptr}, stream)
                        : nullptr;
                sp != nullptr) {
         // the certified split scan: its tile widths and column splits

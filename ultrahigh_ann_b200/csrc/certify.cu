@@ -2196,6 +2196,57 @@ __global__ void __launch_bounds__(kFinalizeThreads)
              replay_count);
 }
 
+// Columns of each of a settled distance's parts.
+__device__ __forceinline__ uint64_t part_width(uint64_t padded_dim, uint32_t parts)
+{
+    return (padded_dim / 4 + parts - 1) / parts * 4;
+}
+
+// Block-wide: the binary64 distance of a row and a query over the columns
+// begin .. end - 1.
+__device__ double block_part_64(const ReplayInputs& in, const float* qrow, uint32_t row,
+                                uint64_t begin, uint64_t end, double* scratch)
+{
+    const float* rrow = in.rows + static_cast<uint64_t>(row) * in.padded_dim;
+    if (in.op == ReplayOp::l2_sequential) {
+        return block_l2_64(qrow + begin, rrow + begin, end - begin, scratch);
+    }
+    const bool weighted = in.op == ReplayOp::l1_weighted_sequential;
+    return block_l1_64(qrow + begin, rrow + begin, weighted ? in.weights64 + begin : nullptr,
+                       in.dim > begin ? in.dim - begin : 0, end - begin, scratch);
+}
+
+// The binary64 distance of each query's answer, where the argmin did not replay it:
+// settle_kernel's sum of one candidate, part for part, for batches that the binary32
+// scan answers in an estimating scan's place. One block per query (64 queries x
+// 60,660 columns: 58 us, beside a scan of 2.4 ms).
+__global__ void __launch_bounds__(kFinalizeThreads)
+    settle_winners_kernel(ReplayInputs in, uint32_t parts, uint32_t row_count,
+                          Result* results, double* exact_distances)
+{
+    __shared__ double scratch[kFinalizeThreads / 32];
+    const uint32_t q = blockIdx.x;
+    const double known = exact_distances[q];
+    const uint32_t row = results[q].row;
+    if (known == known || row >= row_count) {
+        return;
+    }
+    const float* qrow = in.queries + static_cast<uint64_t>(q) * in.padded_dim;
+    const uint64_t width = part_width(in.padded_dim, parts);
+    double d = 0.0;
+    for (uint32_t p = 0; p < parts; ++p) {
+        const uint64_t begin = min(in.padded_dim, p * width);
+        const uint64_t end = min(in.padded_dim, begin + width);
+        const double part = block_part_64(in, qrow, row, begin, end, scratch);
+        d = p == 0 ? part : d + part;
+        __syncthreads();  // scratch is free again
+    }
+    if (threadIdx.x == 0) {
+        results[q].distance = static_cast<float>(d);
+        exact_distances[q] = d;
+    }
+}
+
 // The candidate lists of the split and fixed-point scans. grid = (parts, batch):
 // each block sums its part of the columns for every candidate of the query
 // (usually one or two), from the original binary32 rows; the query's last block
@@ -2226,23 +2277,14 @@ __global__ void __launch_bounds__(kFinalizeThreads)
         return;
     }
     const float* qrow = in.queries + static_cast<uint64_t>(q) * in.padded_dim;
-    const uint64_t width = (in.padded_dim / 4 + parts - 1) / parts * 4;
+    const uint64_t width = part_width(in.padded_dim, parts);
     const uint64_t begin = min(in.padded_dim, blockIdx.x * width);
     const uint64_t end = min(in.padded_dim, begin + width);
     // parts[q][candidate][part]
     double* mine = sums + static_cast<uint64_t>(q) * kSplitCandidates * parts;
     for (uint32_t i = 0; i < k; ++i) {
         const uint32_t row = candidates[static_cast<uint64_t>(q) * kSplitCandidates + i];
-        const float* rrow = in.rows + static_cast<uint64_t>(row) * in.padded_dim;
-        double d;
-        if (in.op == ReplayOp::l2_sequential) {
-            d = block_l2_64(qrow + begin, rrow + begin, end - begin, scratch);
-        } else {
-            const bool weighted = in.op == ReplayOp::l1_weighted_sequential;
-            d = block_l1_64(qrow + begin, rrow + begin,
-                            weighted ? in.weights64 + begin : nullptr,
-                            in.dim > begin ? in.dim - begin : 0, end - begin, scratch);
-        }
+        const double d = block_part_64(in, qrow, row, begin, end, scratch);
         __syncthreads();  // scratch is free again
         if (threadIdx.x == 0) {
             mine[i * parts + blockIdx.x] = d;
@@ -2776,6 +2818,14 @@ void launch_settle(Bound64 bound, ReplayInputs in, const uint32_t* candidates,
     settle_kernel<<<dim3(parts, batch), kFinalizeThreads, 0, stream>>>(
         bound, in, candidates, counts, rows, sums, done, results, exact_distances, replay_count);
     check_cuda(cudaGetLastError(), "cannot launch the settlement kernel");
+}
+
+void launch_settle_winners(ReplayInputs in, uint32_t batch, uint32_t rows, Result* results,
+                           double* exact_distances, cudaStream_t stream)
+{
+    settle_winners_kernel<<<batch, kFinalizeThreads, 0, stream>>>(
+        in, settle_parts(batch, in.padded_dim), rows, results, exact_distances);
+    check_cuda(cudaGetLastError(), "cannot launch the winners' settlement kernel");
 }
 
 void emulated_replay_bound(uint64_t dim, float* rel, float* abs)

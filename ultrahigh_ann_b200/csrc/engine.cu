@@ -1375,9 +1375,9 @@ uint64_t enqueue_lowp_candidates(const BatchContext& c, uint64_t n, const uha::L
 }
 
 // What the row forms are asked for a batch of n.
-FormCall form_call(const BatchContext& c, uint64_t n)
+FormCall form_call(const BatchContext& c, uint64_t n, bool* deferred)
 {
-    return {n, std::max(n, c.upcoming), c.build_forms};
+    return {n, std::max(n, c.upcoming), c.build_forms, deferred};
 }
 
 // No room for a batch's scan buffers: the workspace keeps the binary32 scans, and the
@@ -1391,7 +1391,8 @@ void give_up_estimates(const BatchContext& c)
 
 // The bitmap form of this batch's median scan (everything it needs allocated
 // here), or null when it takes the binary32 passes.
-const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuffers* buffers)
+const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuffers* buffers,
+                                      bool* deferred)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
@@ -1401,7 +1402,7 @@ const uha::RowBits* bits_scan_applies(const BatchContext& c, uint64_t n, BitsBuf
         !uha::bits_batch(index->projection_dimension, n)) {
         return nullptr;
     }
-    const uha::RowBits* bits = row_bits(index, form_call(c, n), ws->stream);
+    const uha::RowBits* bits = row_bits(index, form_call(c, n, deferred), ws->stream);
     if (bits != nullptr && !bits_buffers(ws, index, n, buffers)) {
         give_up_estimates(c);
         return nullptr;
@@ -1460,7 +1461,7 @@ uint64_t enqueue_bits_batch(const BatchContext& c, const uha::RowBits& bits,
 // scan's 8 queries (fixed_scan.cu has both sides' times) whose caller answers the
 // queries it leaves open.
 const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::FixedPlan* plan,
-                                    FixedBuffers* buffers)
+                                    FixedBuffers* buffers, bool* deferred)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
@@ -1470,7 +1471,7 @@ const uha::FixedRows* fixed_applies(const BatchContext& c, uint64_t n, uha::Fixe
         index->rows < 2 || index->rows > uha::kFixedRows) {
         return nullptr;
     }
-    const uha::FixedRows* fx = fixed_rows(index, form_call(c, n), ws->stream);
+    const uha::FixedRows* fx = fixed_rows(index, form_call(c, n, deferred), ws->stream);
     if (fx == nullptr) {
         return nullptr;
     }
@@ -1548,7 +1549,7 @@ uint64_t enqueue_fixed_batch(const BatchContext& c, const uha::FixedRows& rows,
 // settlement has to do without FP64 instructions (the norms, roots and sums of
 // the split scan are binary64). Everything the batch needs is allocated here.
 bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** rows,
-                   uha::SplitPlan* plan, SplitBuffers* buffers)
+                   uha::SplitPlan* plan, SplitBuffers* buffers, bool* deferred)
 {
     const uha_index* index = c.index;
     uha_workspace* ws = c.ws;
@@ -1561,7 +1562,7 @@ bool split_applies(const BatchContext& c, uint64_t n, const uha::SplitRows** row
     if (tuned != nullptr && !tuned->split) {
         return false;
     }
-    const uha::SplitRows* sp = split_rows(index, form_call(c, n), ws->stream);
+    const uha::SplitRows* sp = split_rows(index, form_call(c, n, deferred), ws->stream);
     if (sp == nullptr) {
         return false;
     }
@@ -1915,22 +1916,23 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
         }
         return 1;
     }
+    bool deferred = false;
     const uha::SplitRows* split = nullptr;
     uha::SplitPlan split_plan{};
     SplitBuffers split_parts{};
-    if (split_applies(c, n, &split, &split_plan, &split_parts)) {
+    if (split_applies(c, n, &split, &split_plan, &split_parts, &deferred)) {
         return enqueue_split_batch(c, *split, split_plan, split_parts, source, n, results, exact, time_scan,
                                    scan_start, scan_stop);
     }
     uha::FixedPlan fixed_plan{};
     FixedBuffers fixed_parts{};
-    if (const uha::FixedRows* fixed = fixed_applies(c, n, &fixed_plan, &fixed_parts);
+    if (const uha::FixedRows* fixed = fixed_applies(c, n, &fixed_plan, &fixed_parts, &deferred);
         fixed != nullptr) {
         return enqueue_fixed_batch(c, *fixed, fixed_plan, fixed_parts, source, n, results,
                                    exact, time_scan, scan_start, scan_stop);
     }
     BitsBuffers bits_parts{};
-    if (const uha::RowBits* bits = bits_scan_applies(c, n, &bits_parts); bits != nullptr) {
+    if (const uha::RowBits* bits = bits_scan_applies(c, n, &bits_parts, &deferred); bits != nullptr) {
         return enqueue_bits_batch(c, *bits, bits_parts, source, n, results, exact, time_scan, scan_start,
                                   scan_stop);
     }
@@ -2100,11 +2102,17 @@ uint64_t enqueue_batch(const BatchContext& c, const float* source, uint64_t n,
     uha::launch_argmin(view, bound, in, results, exact, ws->finalize_scratch.get(),
                        ws->max_batch, replay_count, stream);
     ++launches;
+    const bool refine_every = c.refine_every || deferred;
     if (hierarchical && c.want_distances) {
         // reported distances of a hierarchy: the reference's binary64 value of
         // each selected row
         uha::launch_refine_winners(in, bound, results, static_cast<uint32_t>(n), exact,
-                                   stream, c.refine_every);
+                                   stream, refine_every);
+        ++launches;
+    } else if (!hierarchical && c.want_distances && refine_every && c.prepared == nullptr &&
+               !in.emulated) {
+        uha::launch_settle_winners(in, static_cast<uint32_t>(n),
+                                   static_cast<uint32_t>(index->rows), results, exact, stream);
         ++launches;
     }
     return launches;

@@ -33,6 +33,7 @@ struct FormCall {
     uint64_t batch;     // queries of this batch
     uint64_t upcoming;  // of this and the call's later batches
     bool now;           // built whatever it would save (captured and tuned batches)
+    bool* deferred;     // set when the form is not built yet
 };
 // While one of these lives, the index's forms are not given back.
 class FormUse {
@@ -137,8 +138,8 @@ struct BatchContext {
     bool estimates = false;
     uint64_t upcoming = 0;    // queries of the call from this batch on
     bool build_forms = false;  // a row form is built whatever this call would save
-    // Hierarchies: every reported distance in binary64, as the estimating scans
-    // that this batch's scan stands in for report it.
+    // Every reported distance in binary64, as the estimating scans that this batch's
+    // binary32 scan stands in for report it.
     bool refine_every = false;
     // The batch's queries hold the sampled values alone (gathered on the host).
     bool gathered = false;

@@ -612,6 +612,11 @@ void launch_median_tuning_queries(const float* rows, uint64_t row_count, uint64_
 void launch_transpose_rows(const float* rows, uint64_t row_count, uint64_t padded_p,
                            float* out, uint64_t r_pitch, cudaStream_t stream);
 
+// The binary64 distance of each answer that the argmin did not replay, as
+// launch_settle sums it (exact and flat ops).
+void launch_settle_winners(ReplayInputs in, uint32_t batch, uint32_t rows, Result* results,
+                           double* exact_distances, cudaStream_t stream);
+
 // ---- the median scan by row bitmaps (median_bits.cu)
 // Gathers a batch's sampled coordinates (error_flag |= 1 for a non-finite one)
 // and projects them in the reference's binary64 order: y64, batch x p

@@ -193,6 +193,7 @@ bool form_due(const uha_index* index, const FormCall& call, uint64_t bytes)
         return true;
     }
     index->form_saved += saved(call.batch);
+    *call.deferred = true;
     return false;
 }
 
