@@ -398,6 +398,9 @@ struct uha_batch {
         int previous = 0;
         const bool ok = cudaGetDevice(&previous) == cudaSuccess;
         cudaSetDevice(device);
+        if (stream != nullptr) {
+            cudaStreamSynchronize(stream);  // a run that failed after its launch
+        }
         if (exec != nullptr) {
             cudaGraphExecDestroy(exec);
         }

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <limits>
 #include <memory>
 #include <string>
@@ -1385,6 +1386,8 @@ FormCall form_call(const BatchContext& c, uint64_t n, bool* deferred)
 void give_up_estimates(const BatchContext& c)
 {
     c.ws->split_disabled = true;
+    // earlier batches of the call may still read both
+    check_cuda(cudaStreamSynchronize(c.ws->stream), "CUDA query failed");
     c.ws->scan_store.release();
     drop_form(c.index);
 }
@@ -2430,6 +2433,26 @@ extern "C" uha_status uha_query_many(const uha_index* index, uha_workspace* ws,
 
 namespace {
 
+// A call that fails leaves nothing in flight: what it read may be given back next.
+struct DrainOnError {
+    const uha_workspace* ws;
+    int uncaught = std::uncaught_exceptions();
+    ~DrainOnError()
+    {
+        if (std::uncaught_exceptions() > uncaught) {
+            cudaStreamSynchronize(ws->stream);
+            if (ws->finish_stream != nullptr) {
+                cudaStreamSynchronize(ws->finish_stream);
+            }
+            for (int i = 1; i < uha::kFlatLanes; ++i) {
+                if (ws->flat_streams[i] != nullptr) {
+                    cudaStreamSynchronize(ws->flat_streams[i]);
+                }
+            }
+        }
+    }
+};
+
 uha_status query_once(const uha_index* index, uha_workspace* ws, const float* queries,
                       uint64_t query_count, uint64_t batch, int queries_on_device,
                       uha_strategy strategy, uint64_t* out_indices, double* out_distances)
@@ -2483,6 +2506,7 @@ uha_status query_once(const uha_index* index, uha_workspace* ws, const float* qu
         ws->estimates_skip -= skipped ? 1 : 0;
         ctx.estimates = estimable && !skipped;
         const FormUse forms(index);
+        const DrainOnError drain{ws};
         ctx.refine_every = ws->filter_disabled || skipped;
         ctx.gathered = !queries_on_device && gather_on_host(index, n);
         if (ctx.gathered) {

@@ -52,9 +52,9 @@ private:
     std::shared_ptr<std::atomic<int>> users_;
 };
 void allocate_scan_rows(uha_index* index);
-// Gives the index's form back when only the calling thread uses it (it is built again
-// when it pays): a call that finds no room for its scan buffers needs the memory for
-// the binary32 scan's.
+// Gives the index's own form back when only the calling thread uses it and has
+// nothing in flight that reads it (it is built again when it pays): a call that finds
+// no room for its scan buffers needs the memory for the binary32 scan's.
 void drop_form(const uha_index* index);
 const uha::SplitRows* split_rows(const uha_index* index, const FormCall& call,
                                  cudaStream_t stream);

@@ -264,9 +264,8 @@ bool carve(uha_workspace* ws, uint64_t n, F&& layout)
 }  // namespace uha_engine
 
 // A form goes only while no call uses it (its index's next batches build it again
-// when they pay for it and there is room). Locks are only tried, and those of the
-// indexes are never held while one of the set is waited for by a thread that holds
-// the set's, so a call that allocates while it holds its own cannot wait in a circle.
+// when they pay for it and there is room). An index's lock is only tried here: the
+// builder of a form holds its own while it waits for the set's.
 bool uha::reclaim_device_memory() noexcept
 {
     int device = 0;
@@ -274,10 +273,7 @@ bool uha::reclaim_device_memory() noexcept
         return false;
     }
     uha_engine::Holders& all = uha_engine::holders();
-    std::unique_lock<std::mutex> lock(all.mutex, std::try_to_lock);
-    if (!lock.owns_lock()) {
-        return false;
-    }
+    std::lock_guard<std::mutex> lock(all.mutex);
     bool any = false;
     for (auto it = all.indexes.begin(); it != all.indexes.end();) {
         const uha_index* index = *it;
@@ -308,8 +304,9 @@ namespace uha_engine {
 void drop_form(const uha_index* index)
 {
     std::lock_guard<std::mutex> lock(index->forms_mutex);
-    if (index->form_users->load() <= 1) {
-        // (cudaFree waits for the batches of this call that still read it)
+    const uint64_t own =
+        index->split.own.size() + index->bits.own.size() + index->fixed.own.size();
+    if (own != 0 && index->form_users->load() <= 1) {
         index->split = uha::SplitRows{};
         index->bits = uha::RowBits{};
         index->fixed = uha::FixedRows{};
